@@ -1393,6 +1393,9 @@ private:
                            ? reinterpret_cast<const void*>(&pcg_resident_kernel<16, kResidentMaxWidth, 0, 1>)
                            : reinterpret_cast<const void*>(&pcg_resident_kernel<8, kResidentMaxWidth, 0, 1>);
             }
+            if (cluster_ && SYNC == 0)
+                return topo_.max_width <= 6 ? reinterpret_cast<const void*>(&pcg_resident_kernel<16, 6, 2>)
+                                            : reinterpret_cast<const void*>(&pcg_resident_kernel<16, kResidentMaxWidth, 2>);
             if (topo_.max_width <= 6)
                 return resident_warps_ == 16 ? reinterpret_cast<const void*>(&pcg_resident_kernel<16, 6, SYNC>)
                                              : reinterpret_cast<const void*>(&pcg_resident_kernel<8, 6, SYNC>);
@@ -1456,6 +1459,7 @@ private:
     // co-resident.  Returns false when the system does not fit.
     bool plan_resident(int sms) {
         resident_ = false;  // a previous plan's choice must not leak into this one
+        cluster_ = false;
         // the register-resident rows hold symmetric blocks only
         // (and have no contact-operator gather)
         if (solver_path_ != kPathPersistent || topo_.max_width > kResidentMaxWidth || use_bending_ || co_active_)
@@ -1466,6 +1470,7 @@ private:
             resident_warps_ = W;
             const int grid = (n_slices + W - 1) / W;
             build_plan(topo_.inst_slice, grid, plan_);
+            if (W == 16 && plan_cluster()) return true;
             plan_coarse();
             pers_smem_ = (size_t)W * kSlotW * sizeof(double) + (size_t)plan_.max_inst_per_cta * sizeof(LocalInst);
             if (coarse_on_)  // the coarse block's rows of A_c^-1, a phase's block values and its staged slots
@@ -1481,6 +1486,46 @@ private:
         }
         resident_ = false;
         return false;
+    }
+
+    // The cluster build of the resident kernel, for plans whose CTAs (16 warps
+    // each) form one cluster: a single CTA, with any number of instances, or
+    // up to kClusterMax CTAs of one instance (8192 rows; a cluster stops as a
+    // whole; the grid barrier takes 1.5 times as long at 90 x 90 particles,
+    // 2.2 times at 10 x 10).  Block-Jacobi in synchronisation mode 0 only.
+    bool plan_cluster() {
+        cluster_ = false;
+        const int ctas = plan_.grid;
+        if (pc_kind_ != 0 || sync_mode_ != 0 || ctas > kClusterMax || (ctas > 1 && plan_.n_inst > 1) ||
+            plan_.max_slices_per_cta > 16)
+            return false;
+        coarse_on_ = false;
+        coarse_batched_ = false;
+        cluster_ = true;
+        pers_smem_ = (size_t)16 * kSlotW * sizeof(double) + (size_t)plan_.max_inst_per_cta * sizeof(LocalInst);
+        const void* fn = persistent_fn();
+        ck(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pers_smem_),
+           "cudaFuncSetAttribute(cluster smem)");
+        if (ctas > 8)
+            ck(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
+               "cudaFuncSetAttribute(cluster size)");
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(ctas);
+        cfg.blockDim = dim3(512);
+        cfg.dynamicSmemBytes = pers_smem_;
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = ctas;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int fit = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveClusters(&fit, fn, &cfg);
+        if (e != cudaSuccess || fit < 1) {
+            cudaGetLastError();  // no room for the cluster on this device: the grid-barrier build
+            cluster_ = false;
+        }
+        return cluster_;
     }
 
     // Coarse level of the two-level preconditioner (kind 2) of a
@@ -2042,10 +2087,17 @@ private:
             p.sharedMemBytes = (unsigned)pers_smem_;
             p.kernelParams = pargs;
             ck(cudaGraphAddKernelNode(&pcg_node_, graph_, &reset, 1, &p), "add persistent PCG node");
-            cudaLaunchAttributeValue coop{};
-            coop.cooperative = 1;
-            ck(cudaGraphKernelNodeSetAttribute(pcg_node_, cudaLaunchAttributeCooperative, &coop),
-               "cooperative attribute");
+            cudaLaunchAttributeValue av{};
+            if (cluster_) {
+                av.clusterDim.x = plan_.grid;
+                av.clusterDim.y = av.clusterDim.z = 1;
+                ck(cudaGraphKernelNodeSetAttribute(pcg_node_, cudaLaunchAttributeClusterDimension, &av),
+                   "cluster attribute");
+            } else {
+                av.cooperative = 1;
+                ck(cudaGraphKernelNodeSetAttribute(pcg_node_, cudaLaunchAttributeCooperative, &av),
+                   "cooperative attribute");
+            }
         }
         {
             const int vgrid = std::max(1, grid_for(topo_.n, kVecBlock));
@@ -2296,6 +2348,7 @@ private:
     int row_order_ = 0;
     std::vector<int> order_;  // particles in row order (row_order_ 1)
     bool resident_ = false;
+    bool cluster_ = false;  // the resident plan runs as one thread-block cluster
     int resident_warps_ = 16;
     std::vector<TuneResult> tune_;
     int sync_mode_ = 0;    // 0 grid counter barrier, 1 polled per-instance slots

@@ -266,6 +266,25 @@ __device__ __forceinline__ double dot3d(float3 a, float3 b) {
 }
 
 // ---------------------------------------------------------------------------
+// Cluster synchronisation (the resident kernel instantiated with SYNC = 2):
+// the whole grid is one thread-block cluster (or a single CTA), so a phase
+// needs no trip through L2: each CTA writes its partial sums into every
+// CTA's shared memory and the cluster's hardware barrier is the wait.
+// ---------------------------------------------------------------------------
+constexpr int kClusterMax = 16;  // CTAs per cluster (above 8: non-portable, opted in by the host)
+
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// *p (this CTA's shared memory) of the cluster's CTA `rank` = v
+__device__ __forceinline__ void cluster_store(double* p, int rank, double v) {
+    const uint32_t local = static_cast<uint32_t>(__cvta_generic_to_shared(p));
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(remote), "d"(v) : "memory");
+}
+
+// ---------------------------------------------------------------------------
 // Per-instance bookkeeping
 // ---------------------------------------------------------------------------
 // Where this CTA's instances live (all threads of the CTA, once per solve;
@@ -318,6 +337,59 @@ __device__ __forceinline__ void warp0_publish(const BatchPlan& bp, const double*
 #pragma unroll
                 for (int q = 0; q < NV; ++q) bp.slots[((size_t)set * bp.n_slots + L.own_slot) * kSlotW + q] = acc[q];
             }
+        }
+    }
+}
+
+// One reduction phase of the cluster mode (SYNC = 2), called by every thread
+// after the __syncthreads that follows the partials: warp 0 adds the CTA's
+// slices (as warp0_publish) and writes the sums to its slot in every CTA's
+// cslot[set], all threads meet at the cluster barrier, and warp 0 adds the
+// CTAs' slots as warp0_read_totals does (lane l takes slot l, then the xor
+// tree: identical totals) and applies `step`.  A single CTA needs neither
+// slots nor barrier, and may hold several instances.
+template <int NV, class Step>
+__device__ __forceinline__ void cluster_phase(const double* spart, LocalInst* li, int nloc,
+                                              double (*cslot)[kClusterMax][kSlotW], int set, Step&& step) {
+    const int lane = threadIdx.x & 31, ctas = (int)gridDim.x;
+    if (ctas > 1) {
+        if (threadIdx.x < 32 && !li[0].done) {
+            const LocalInst& L = li[0];
+            double acc[NV];
+#pragma unroll
+            for (int q = 0; q < NV; ++q) acc[q] = 0.0;
+            for (int sl = L.seg_lo + lane; sl < L.seg_hi; sl += 32) {
+#pragma unroll
+                for (int q = 0; q < NV; ++q) acc[q] += spart[sl * kSlotW + q];
+            }
+#pragma unroll
+            for (int q = 0; q < NV; ++q) {
+                acc[q] = warp_sum(acc[q]);
+                if (lane < ctas) cluster_store(&cslot[set][blockIdx.x][q], lane, acc[q]);
+            }
+        }
+        cluster_sync_all();
+    }
+    if (threadIdx.x < 32) {
+        for (int t = 0; t < nloc; ++t) {
+            LocalInst& L = li[t];
+            if (L.done) continue;
+            double tot[NV];
+#pragma unroll
+            for (int q = 0; q < NV; ++q) tot[q] = 0.0;
+            if (ctas > 1) {
+#pragma unroll
+                for (int q = 0; q < NV; ++q) tot[q] = lane < ctas ? cslot[set][lane][q] : 0.0;
+            } else {
+                for (int sl = L.seg_lo + lane; sl < L.seg_hi; sl += 32) {
+#pragma unroll
+                    for (int q = 0; q < NV; ++q) tot[q] += spart[sl * kSlotW + q];
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < NV; ++q) tot[q] = warp_sum(tot[q]);
+            if (lane == 0) step(L, tot);
+            __syncwarp();
         }
     }
 }
@@ -809,16 +881,18 @@ __device__ __forceinline__ void instances_fail(const BatchPlan& bp, const LocalI
 // still be reading from the phase before (it can only publish phase ph + 2
 // into that set after the barrier of phase ph + 1, which every reader of
 // phase ph must have reached).
-#define slot_set(ph) (SYNC ? (ph) % 3 : (ph) & 1)
+#define slot_set(ph) (SYNC == 1 ? (ph) % 3 : (ph) & 1)
 
-// The phase protocol shared by both kernels.  After the CTA's slice
-// partials are in spart and a __syncthreads, this runs the warp-0 phase and
-// leaves, after a closing __syncthreads, s_flag = 1 on a failed wait and
-// (counter mode, with `exit_test`) s_exit = 1 when every instance of the
-// batch is done.
+// The phase protocol of the resident kernel.  After the CTA's slice
+// partials are in spart and a __syncthreads, this runs the warp-0 phase (or
+// the cluster phase) and leaves, after a closing __syncthreads, s_flag = 1 on
+// a failed wait and (counter mode, with `exit_test`) s_exit = 1 when every
+// instance of the batch is done.
 #define CHYSX_REDUCE_PHASE(NV, KP, exit_test, STEP)                                                  \
     do {                                                                                             \
-        if (warp == 0) {                                                                             \
+        if constexpr (SYNC == 2) {                                                                   \
+            cluster_phase<NV>(spart, li, nloc, s_cslot, slot_set(ph), STEP);                         \
+        } else if (warp == 0) {                                                                             \
             const bool w0ok = warp0_phase<NV, SYNC, KP>(bp, spart, li, nloc, slot_set(ph), target, STEP); \
             if (lane == 0) {                                                                         \
                 if (!w0ok) s_flag = 1;                                                               \
@@ -1493,6 +1567,14 @@ namespace chysx_b200 {
 // the same CTA are read from there, the others from L2, a batch of gathers
 // in flight at once.  Same phases, reductions, barrier and per-instance
 // logic as pcg_persistent_kernel.
+//
+// SYNC = 2 is the build for plans of one cluster: at this size an iteration
+// is two reductions' latency and little else, and the counter barrier costs
+// an L2 round trip to arrive, one to see the count and one to read the slots
+// even when a single CTA waits for itself.  Measured on B200, the whole step
+// at 50 iterations, grid barrier against cluster: 10 x 10 grid (1 CTA) 300
+// against 137 us, 32 x 32 (2) 328 / 230, 64 x 64 (8) 371 / 239, 90 x 90 (16)
+// 376 / 256.
 // ---------------------------------------------------------------------------
 template <int W, int MAXW, int SYNC = 0, int PC = 0>
 __global__ void __launch_bounds__(W * 32, 512 / (W * 32))  // 512 threads of rows per SM
@@ -1523,6 +1605,8 @@ pcg_resident_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, ZP
         s_flag = 0;
         s_exit = 0;
     }
+    // a CTA of the cluster writes into another's shared memory only once that one runs
+    if (SYNC == 2 && gridDim.x > 1) cluster_sync_all();
     init_local(bp, li, s0, s1, il0, il1);
     bool ok = true;
     auto no_step = [](LocalInst&, const double*) {};
@@ -1540,9 +1624,13 @@ pcg_resident_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, ZP
     S6 B[MAXW];
     // column indices: registers, or shared memory in the slot-polling build
     // (its waits need the registers)
-    int cols_r[SYNC ? 1 : MAXW];
-    __shared__ int s_cols[SYNC ? MAXW * W * 32 : 1];
-    auto col_at = [&](int k) -> int & { return SYNC ? s_cols[k * W * 32 + threadIdx.x] : cols_r[SYNC ? 0 : k]; };
+    int cols_r[SYNC == 1 ? 1 : MAXW];
+    __shared__ int s_cols[SYNC == 1 ? MAXW * W * 32 : 1];
+    auto col_at = [&](int k) -> int & {
+        return SYNC == 1 ? s_cols[k * W * 32 + threadIdx.x] : cols_r[SYNC == 1 ? 0 : k];
+    };
+    // cluster mode: every CTA's partial sums of a phase, two sets by parity
+    __shared__ double s_cslot[SYNC == 2 ? 2 : 1][kClusterMax][SYNC == 2 ? kSlotW : 1];
     int w = 0;
     float3 b = f3(0.f, 0.f, 0.f), x = b, r = b, z = b, p = b;
 #pragma unroll
