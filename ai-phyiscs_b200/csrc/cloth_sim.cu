@@ -119,13 +119,22 @@ void ensure_train_smem() {
     if (!g_train_smem_set[dev]) {
         ck(cudaFuncSetAttribute(mlp_train_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem),
            "cudaFuncSetAttribute(mlp_train_tile_kernel)");
+        ck(cudaFuncSetAttribute(mlp_dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDwSmem),
+           "cudaFuncSetAttribute(mlp_dw_kernel)");
         g_train_smem_set[dev] = true;
     }
 }
 
-// the weight-gradient kernel's per-chunk partials: a 64 x 64 block and 64 biases per kDwRows rows
+// the weight-gradient kernel's partials: a flat gradient vector (kDwFlat
+// floats) per chunk of kDwRows rows in space for a 64 x 64 block and 64 biases
+// per 64 rows, which it fits from two chunks on; a single chunk writes the
+// gradient itself
+constexpr int kDwSpaceRows = 64;
+constexpr size_t kDwSpace = 64 * 64 + 64;
+static_assert(2 * kDwFlat <= (kDwRows / kDwSpaceRows + 1) * kDwSpace && kDwFlat <= kDwRows / kDwSpaceRows * kDwSpace,
+              "the chunks' gradient vectors fit the partials' space");
 size_t dw_partial_bytes(int rows) {
-    return (size_t)((std::max(rows, 1) + kDwRows - 1) / kDwRows) * (64 * 64 + 64) * sizeof(float);
+    return (size_t)((std::max(rows, 1) + kDwSpaceRows - 1) / kDwSpaceRows) * kDwSpace * sizeof(float);
 }
 
 size_t mlp_workspace_bytes(int rows) {
@@ -136,9 +145,12 @@ size_t mlp_workspace_bytes(int rows) {
 
 // Forward + backward (when targets != 0) of rows feature vectors; grads in
 // the flat parameter layout (normalisation entries zero); optional predicted
-// dv output.  Loss = mean squared error of the standardised outputs.
+// dv output.  Loss = mean squared error of the standardised outputs.  With
+// `adam` the weights take their Adam step behind the gradient, ahead of the
+// wait for the loss.
 void mlp_gradients(uintptr_t params, uintptr_t features, uintptr_t targets, int rows, uintptr_t grad, double* loss,
-                   uintptr_t dv_out, uintptr_t workspace, uint64_t ws_bytes, uintptr_t stream_u) {
+                   uintptr_t dv_out, uintptr_t workspace, uint64_t ws_bytes, uintptr_t stream_u,
+                   const AdamArgs* adam = nullptr) {
     if (rows <= 0) throw std::invalid_argument("mlp: rows must be positive");
     if (!params || !features || !workspace) throw std::invalid_argument("mlp: null device pointer");
     if (ws_bytes < mlp_workspace_bytes(rows)) throw std::invalid_argument("mlp: workspace too small");
@@ -160,61 +172,49 @@ void mlp_gradients(uintptr_t params, uintptr_t features, uintptr_t targets, int 
     bufs.sse = reinterpret_cast<double*>(ws + off);
     off += align_up((size_t)train_blocks(rows) * kTrainWarps * sizeof(double));
     const int chunks = (rows + kDwRows - 1) / kDwRows;
-    float* part_w = reinterpret_cast<float*>(ws + off);
-    float* part_b = part_w + (size_t)chunks * 64 * 64;
+    float* part = chunks == 1 && targets ? reinterpret_cast<float*>(grad) + MlpOffsets::w1
+                                         : reinterpret_cast<float*>(ws + off);
     bufs.out = reinterpret_cast<float*>(dv_out);
-    mlp_pack_kernel<<<8, 256, 0, stream>>>(reinterpret_cast<const float*>(params), packed);
+    mlp_pack_kernel<<<74, 128, 0, stream>>>(reinterpret_cast<const float*>(params), packed);
     ck(cudaGetLastError(), "mlp_pack_kernel launch");
     ensure_train_smem();
     const int blocks = train_blocks(rows);
-    // with no targets the kernel still runs the backward on zero residuals;
-    // a zero-target buffer is not needed because target rows are only read
-    // when targets != 0
     mlp_train_tile_kernel<<<blocks, kTrainWarps * 32, kTrainSmem, stream>>>(
         packed, reinterpret_cast<const float*>(features), reinterpret_cast<const float*>(targets), rows,
         2.0f / (3.0f * (float)rows), bufs);
     ck(cudaGetLastError(), "mlp_train_tile_kernel launch");
     if (targets) {
-        using O = MlpOffsets;
-        float* g = reinterpret_cast<float*>(grad);
-        ck(cudaMemsetAsync(g, 0, sizeof(float) * O::w1, stream), "cudaMemsetAsync(grad)");
-        struct L { int in, out, w, b; } layers[4] = {
-            {kMlpIn, kMlpHid, O::w1, O::b1}, {kMlpHid, kMlpHid, O::w2, O::b2},
-            {kMlpHid, kMlpHid, O::w3, O::b3}, {kMlpHid, kMlpOut, O::w4, O::b4}};
-        for (int l = 0; l < 4; ++l) {
-            // kDwPadSmem bytes of unused dynamic shared memory hold an SM to
-            // at most 6 of these CTAs (6 x 64 TMEM columns of 512), so no CTA
-            // waits in tcgen05.alloc
-            mlp_dw_kernel<<<chunks, kDwThreads, kDwPadSmem, stream>>>(bufs.act[l], bufs.dz[l], rows, layers[l].in,
-                                                                      layers[l].out, part_w, part_b);
-            ck(cudaGetLastError(), "mlp_dw_kernel launch");
-            const int outs = layers[l].in * layers[l].out + layers[l].out;
-            mlp_dw_reduce_kernel<<<(outs + 255) / 256, 256, 0, stream>>>(part_w, part_b, chunks, layers[l].in,
-                                                                        layers[l].out, g + layers[l].w,
-                                                                        g + layers[l].b);
-            ck(cudaGetLastError(), "mlp_dw_reduce_kernel launch");
-        }
+        mlp_dw_kernel<<<dim3(chunks, 4), kDwThreads, kDwSmem, stream>>>(bufs, rows, part);
+        ck(cudaGetLastError(), "mlp_dw_kernel launch");
+        mlp_dw_reduce_kernel<<<grid_for(MlpOffsets::total, 128), 128, 0, stream>>>(
+            part, chunks, reinterpret_cast<float*>(grad), 1, adam ? *adam : AdamArgs{});
+        ck(cudaGetLastError(), "mlp_dw_reduce_kernel launch");
         if (loss) {
-            std::vector<double> part((size_t)blocks * kTrainWarps);
-            ck(cudaMemcpyAsync(part.data(), bufs.sse, part.size() * sizeof(double), cudaMemcpyDeviceToHost, stream),
+            std::vector<double> sse((size_t)blocks * kTrainWarps);
+            ck(cudaMemcpyAsync(sse.data(), bufs.sse, sse.size() * sizeof(double), cudaMemcpyDeviceToHost, stream),
                "cudaMemcpyAsync(loss)");
             ck(cudaStreamSynchronize(stream), "cudaStreamSynchronize(loss)");
             double s = 0.0;
-            for (double v : part) s += v;
+            for (double v : sse) s += v;
             *loss = s / (3.0 * rows);
         }
     }
 }
 
-void mlp_adam(uintptr_t params, uintptr_t grad, uintptr_t m1, uintptr_t m2, float lr, int t, uintptr_t stream_u) {
+AdamArgs adam_args(uintptr_t params, uintptr_t grad, uintptr_t m1, uintptr_t m2, float lr, int t) {
     if (!params || !grad || !m1 || !m2) throw std::invalid_argument("mlp_adam: null device pointer");
     if (t < 1) throw std::invalid_argument("mlp_adam: step must be >= 1");
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.0f / (1.0f - std::pow(b1, (float)t)), c2 = 1.0f / (1.0f - std::pow(b2, (float)t));
-    mlp_adam_kernel<<<16, 256, 0, reinterpret_cast<cudaStream_t>(stream_u)>>>(
-        reinterpret_cast<float*>(params), reinterpret_cast<const float*>(grad), reinterpret_cast<float*>(m1),
-        reinterpret_cast<float*>(m2), MlpOffsets::w1, MlpOffsets::total, lr, b1, b2, 1e-8f, c1, c2);
-    ck(cudaGetLastError(), "mlp_adam_kernel launch");
+    return AdamArgs{reinterpret_cast<float*>(params), reinterpret_cast<float*>(m1), reinterpret_cast<float*>(m2),
+                    lr, b1, b2, 1e-8f, c1, c2};
+}
+
+void mlp_adam(uintptr_t grad, const AdamArgs& ad, uintptr_t stream_u) {
+    float* g = reinterpret_cast<float*>(grad);
+    mlp_dw_reduce_kernel<<<grid_for(MlpOffsets::total, 128), 128, 0, reinterpret_cast<cudaStream_t>(stream_u)>>>(
+        g + MlpOffsets::w1, 1, g, 0, ad);
+    ck(cudaGetLastError(), "mlp_dw_reduce_kernel launch");
 }
 
 // ---------------------------------------------------------------------------
@@ -230,7 +230,7 @@ constexpr int kNoAllocPartials = (kNoAllocMaxRows + 16 * kTrainWarps - 1) / (16 
 constexpr size_t kNoAllocScratchBytes =
     align_up_c(sizeof(MlpPacked)) + 8 * align_up_c((size_t)kNoAllocMaxRows * 64 * sizeof(__nv_bfloat16)) +
     align_up_c((size_t)kNoAllocPartials * sizeof(double)) +
-    align_up_c((size_t)((kNoAllocMaxRows + kDwRows - 1) / kDwRows) * (64 * 64 + 64) * sizeof(float));
+    align_up_c((size_t)((kNoAllocMaxRows + kDwSpaceRows - 1) / kDwSpaceRows) * kDwSpace * sizeof(float));
 static_assert(kNoAllocPartials <= 1184 * kTrainWarps, "partials follow train_blocks()");
 
 static __device__ __align__(256) unsigned char g_mlp_noalloc_scratch[kNoAllocScratchBytes];
@@ -739,7 +739,7 @@ public:
             if (!std::isfinite(params[q])) throw std::invalid_argument("set_network: non-finite parameter");
         d_net_params_.upload(params, n);
         d_net_.resize(1);
-        mlp_pack_kernel<<<8, 256>>>(d_net_params_.get(), d_net_.get());
+        mlp_pack_kernel<<<74, 128>>>(d_net_params_.get(), d_net_.get());
         ck(cudaGetLastError(), "mlp_pack_kernel launch");
         ck(cudaDeviceSynchronize(), "cudaDeviceSynchronize(set_network)");
         warm_guess_ = true;
@@ -2703,9 +2703,10 @@ int chysx_mlp_train_step(uintptr_t params, uintptr_t grad, uintptr_t m1, uintptr
                          uintptr_t targets, int rows, float lr, int adam_step, uintptr_t workspace,
                          uint64_t workspace_bytes, double* loss, uintptr_t stream) {
     return guard([&] {
-        chysx_b200::mlp_gradients(params, features, targets, rows, grad, loss, 0, workspace, workspace_bytes,
-                                  stream);
-        chysx_b200::mlp_adam(params, grad, m1, m2, lr, adam_step, stream);
+        const chysx_b200::AdamArgs ad = chysx_b200::adam_args(params, grad, m1, m2, lr, adam_step);
+        chysx_b200::mlp_gradients(params, features, targets, rows, grad, loss, 0, workspace, workspace_bytes, stream,
+                                  &ad);
+        if (!targets) chysx_b200::mlp_adam(grad, ad, stream);  // a step along the gradient given
     });
 }
 int chysx_mlp_noalloc_max_rows(void) { return CHYSX_MLP_NOALLOC_MAX_ROWS; }

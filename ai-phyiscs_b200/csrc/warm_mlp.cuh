@@ -102,8 +102,11 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 __device__ __forceinline__ uint32_t ld_u32(const __nv_bfloat16* p) { return *reinterpret_cast<const uint32_t*>(p); }
 
 __device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
-__device__ __forceinline__ float gelu_grad(float x) {
-    return 0.5f * (1.0f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
+// GELU and its derivative from one error function.
+__device__ __forceinline__ float gelu_both(float x, float& grad) {
+    const float e = 1.0f + erff(x * 0.70710678118654752f);
+    grad = 0.5f * e + x * 0.39894228040143268f * expf(-0.5f * x * x);
+    return 0.5f * x * e;
 }
 
 // One dense layer for a 16-row tile: acc[nt][4] = A(16 x 16*KT) * Wt^T,
@@ -135,16 +138,20 @@ __device__ __forceinline__ void acc_to_a(const float (&h)[8][4], uint32_t (&a)[4
 }
 
 // bias + GELU in place; column of element (n, e) is 8n + 2t + (e & 1)
-__device__ __forceinline__ void bias_gelu(float (&h)[8][4], const float* bias, int lane, float (*pre)[4] = nullptr) {
+__device__ __forceinline__ void bias_gelu(float (&h)[8][4], const float* bias, int lane) {
     const int t = lane & 3;
 #pragma unroll
     for (int n = 0; n < 8; ++n)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float z = h[n][e] + bias[8 * n + 2 * t + (e & 1)];
-            if (pre) pre[n][e] = z;
-            h[n][e] = gelu(z);
-        }
+        for (int e = 0; e < 4; ++e) h[n][e] = gelu(h[n][e] + bias[8 * n + 2 * t + (e & 1)]);
+}
+// the same, with GELU's derivative at every element
+__device__ __forceinline__ void bias_gelu_grad(float (&h)[8][4], const float* bias, int lane, float (&grad)[8][4]) {
+    const int t = lane & 3;
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) h[n][e] = gelu_both(h[n][e] + bias[8 * n + 2 * t + (e & 1)], grad[n][e]);
 }
 
 // Loads the A fragments of a 16 x 32 feature tile stored [row][kT1] in smem.
@@ -527,7 +534,11 @@ __global__ void mlp_pack_kernel(const float* __restrict__ p, MlpPacked* __restri
     }
 }
 
-// Forward + backward of one minibatch, one warp per 16 rows.  Writes the
+// Forward + backward of one minibatch, one warp per 16 rows (prediction
+// alone without targets).  Bound by a warp's chain of dependent steps, so the
+// tile's features come in as 10 coalesced loads per lane (one lane per row
+// walked 20 dependent load-store pairs), the packed weights in 16-byte pieces,
+// and GELU's derivative is formed beside GELU from one error function.  Writes the
 // BF16 layer inputs A0..A3 ([rows][64], A0 padded to 32 in a 64-wide row)
 // and BF16 pre-activation gradients dZ1..dZ4 ([rows][64], dZ4 uses 8
 // columns) for the weight-gradient GEMM, the FP32 output (optional) and the
@@ -550,12 +561,15 @@ mlp_train_tile_kernel(const MlpPacked* __restrict__ net, const float* __restrict
     extern __shared__ __align__(16) unsigned char s_raw[];
     MlpPacked& Wp = *reinterpret_cast<MlpPacked*>(s_raw);
     auto s_feat = reinterpret_cast<__nv_bfloat16(*)[16 * kT1]>(s_raw + sizeof(MlpPacked));
+    // GELU's derivative at the first two hidden layers, 16-byte columns per lane
     auto s_z = reinterpret_cast<float(*)[2][16 * 64]>(s_raw + sizeof(MlpPacked) +
                                                      sizeof(__nv_bfloat16) * kTrainWarps * 16 * kT1);
     {
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(net);
-        uint32_t* dst = reinterpret_cast<uint32_t*>(&Wp);
-        for (int q = threadIdx.x; q < (int)(sizeof(MlpPacked) / 4); q += blockDim.x) dst[q] = src[q];
+        static_assert(sizeof(MlpPacked) % 16 == 0, "copied in 16-byte pieces");
+        const uint4* __restrict__ src = reinterpret_cast<const uint4*>(net);
+        uint4* __restrict__ dst = reinterpret_cast<uint4*>(&Wp);
+#pragma unroll 8
+        for (int q = threadIdx.x; q < (int)(sizeof(MlpPacked) / 16); q += kTrainWarps * 32) dst[q] = __ldg(src + q);
     }
     __syncthreads();
     const MlpFwd& W = Wp.f;
@@ -566,18 +580,32 @@ mlp_train_tile_kernel(const MlpPacked* __restrict__ net, const float* __restrict
     double sse = 0.0;
     for (int tile = blockIdx.x * kTrainWarps + warp; tile < tiles; tile += gridDim.x * kTrainWarps) {
         const int r0 = tile * 16;
-        // standardised features -> smem (lanes 0..15: one row each)
-        if (lane < 16) {
-            const int r = r0 + lane;
-            __nv_bfloat16* fr = s_feat[warp] + lane * kT1;
-            for (int q = 0; q < kMlpInPad; ++q) {
-                float z = 0.f;
-                if (r < rows && q < kMlpIn) z = (feat[(size_t)r * kMlpIn + q] - W.mu_in[q]) * W.inv_sd_in[q];
-                fr[q] = __float2bfloat16_rn(z);
-                if (r < rows) bufs.act[0][(size_t)r * 64 + q] = fr[q];
+        // standardised features -> smem: the tile's 320 floats are consecutive
+        {
+            const float* __restrict__ fsrc = feat + (size_t)r0 * kMlpIn;
+            const int left = (rows - r0) * kMlpIn;
+            float fv[10];
+#pragma unroll
+            for (int u = 0; u < 10; ++u) fv[u] = u * 32 + lane < left ? __ldg(fsrc + u * 32 + lane) : 0.f;
+#pragma unroll
+            for (int u = 0; u < 10; ++u) {
+                const int x = u * 32 + lane, q = x % kMlpIn;
+                s_feat[warp][(x / kMlpIn) * kT1 + q] =
+                    __float2bfloat16_rn(x < left ? (fv[u] - W.mu_in[q]) * W.inv_sd_in[q] : 0.f);
             }
+            for (int x = lane; x < 16 * (kMlpInPad - kMlpIn); x += 32)
+                s_feat[warp][(x / (kMlpInPad - kMlpIn)) * kT1 + kMlpIn + x % (kMlpInPad - kMlpIn)] =
+                    __float2bfloat16_rn(0.f);
         }
         __syncwarp();
+        if (target) {
+            for (int x = lane; x < 16 * 4; x += 32) {
+                const int r = x >> 2, c = (x & 3) * 8;
+                if (r0 + r < rows)
+                    *reinterpret_cast<uint4*>(bufs.act[0] + (size_t)(r0 + r) * 64 + c) =
+                        *reinterpret_cast<const uint4*>(s_feat[warp] + r * kT1 + c);
+            }
+        }
         auto store_rows = [&](__nv_bfloat16* dst, const float (&h)[8][4]) {
 #pragma unroll
             for (int n = 0; n < 8; ++n) {
@@ -591,28 +619,50 @@ mlp_train_tile_kernel(const MlpPacked* __restrict__ net, const float* __restrict
         // ---- forward
         uint32_t a0[2][4];
         load_a_features(a0, s_feat[warp], lane);
-        float h[8][4], z3[8][4];
-        float pre[8][4];
+        float h[8][4], gr[8][4];
         uint32_t a[4][4];
+        // a lane's own values come back to it: 16-byte pieces, lanes side by side
+        auto keep = [&](int l) {
+#pragma unroll
+            for (int n = 0; n < 8; ++n)
+                *reinterpret_cast<float4*>(&s_z[warp][l][n * 128 + lane * 4]) =
+                    make_float4(gr[n][0], gr[n][1], gr[n][2], gr[n][3]);
+        };
+        auto kept = [&](int l, float (&q)[8][4]) {
+#pragma unroll
+            for (int n = 0; n < 8; ++n) {
+                const float4 f4v = *reinterpret_cast<const float4*>(&s_z[warp][l][n * 128 + lane * 4]);
+                q[n][0] = f4v.x;
+                q[n][1] = f4v.y;
+                q[n][2] = f4v.z;
+                q[n][3] = f4v.w;
+            }
+        };
         layer_mma<2, 8>(h, a0, W.wt1, kT1, lane);
-        bias_gelu(h, W.b1, lane, pre);
-#pragma unroll
-        for (int n = 0; n < 8; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) s_z[warp][0][(g + 8 * (e >> 1)) * 64 + 8 * n + 2 * t + (e & 1)] = pre[n][e];
-        store_rows(bufs.act[1], h);
+        if (target) {
+            bias_gelu_grad(h, W.b1, lane, gr);
+            keep(0);
+            store_rows(bufs.act[1], h);
+        } else {
+            bias_gelu(h, W.b1, lane);
+        }
         acc_to_a(h, a);
         layer_mma<4, 8>(h, a, W.wt2, kTH, lane);
-        bias_gelu(h, W.b2, lane, pre);
-#pragma unroll
-        for (int n = 0; n < 8; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) s_z[warp][1][(g + 8 * (e >> 1)) * 64 + 8 * n + 2 * t + (e & 1)] = pre[n][e];
-        store_rows(bufs.act[2], h);
+        if (target) {
+            bias_gelu_grad(h, W.b2, lane, gr);
+            keep(1);
+            store_rows(bufs.act[2], h);
+        } else {
+            bias_gelu(h, W.b2, lane);
+        }
         acc_to_a(h, a);
         layer_mma<4, 8>(h, a, W.wt3, kTH, lane);
-        bias_gelu(h, W.b3, lane, z3);
-        store_rows(bufs.act[3], h);
+        if (target) {
+            bias_gelu_grad(h, W.b3, lane, gr);
+            store_rows(bufs.act[3], h);
+        } else {
+            bias_gelu(h, W.b3, lane);
+        }
         acc_to_a(h, a);
         float o[1][4];
         layer_mma<4, 1>(o, a, W.wt4, kTH, lane);
@@ -633,6 +683,10 @@ mlp_train_tile_kernel(const MlpPacked* __restrict__ net, const float* __restrict
             }
             d4[e] = d * grad_scale;  // dL/dy for L = grad_scale/2 * sum d^2
         }
+        if (!target) {  // prediction only
+            __syncwarp();
+            continue;
+        }
         // dZ4 (16 x 8) -> global, and as A fragment of one k-tile (cols 8..15 zero)
         if (r0 + g < rows)
             *reinterpret_cast<uint32_t*>(bufs.dz[3] + (size_t)(r0 + g) * 64 + 2 * t) = pack_bf16(d4[0], d4[1]);
@@ -650,23 +704,23 @@ mlp_train_tile_kernel(const MlpPacked* __restrict__ net, const float* __restrict
 #pragma unroll
         for (int n = 0; n < 8; ++n)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) dz[n][e] = dA[n][e] * gelu_grad(z3[n][e]);
+            for (int e = 0; e < 4; ++e) dz[n][e] = dA[n][e] * gr[n][e];
         store_rows(bufs.dz[2], dz);
         acc_to_a(dz, a);
         layer_mma<4, 8>(dA, a, WB.w3, kTH, lane);  // dA2 = dZ3 W3^T
+        kept(1, gr);
 #pragma unroll
         for (int n = 0; n < 8; ++n)
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-                dz[n][e] = dA[n][e] * gelu_grad(s_z[warp][1][(g + 8 * (e >> 1)) * 64 + 8 * n + 2 * t + (e & 1)]);
+            for (int e = 0; e < 4; ++e) dz[n][e] = dA[n][e] * gr[n][e];
         store_rows(bufs.dz[1], dz);
         acc_to_a(dz, a);
         layer_mma<4, 8>(dA, a, WB.w2, kTH, lane);  // dA1 = dZ2 W2^T
+        kept(0, gr);
 #pragma unroll
         for (int n = 0; n < 8; ++n)
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-                dz[n][e] = dA[n][e] * gelu_grad(s_z[warp][0][(g + 8 * (e >> 1)) * 64 + 8 * n + 2 * t + (e & 1)]);
+            for (int e = 0; e < 4; ++e) dz[n][e] = dA[n][e] * gr[n][e];
         store_rows(bufs.dz[0], dz);
         __syncwarp();
     }
@@ -674,28 +728,41 @@ mlp_train_tile_kernel(const MlpPacked* __restrict__ net, const float* __restrict
     if (lane == 0) bufs.sse[(size_t)blockIdx.x * kTrainWarps + warp] = sse;
 }
 
-// Weight gradients on the fifth-generation tensor cores, split over the
-// rows (the GEMM's K): CTA c forms the partial dW = act^T dz of rows
-// [c kDwRows, (c + 1) kDwRows) as one M = 128 (in features, padded with
-// zero rows) x N = 64 (out features, zero-padded) MMA chain from shared
-// memory -- both operands MN-major (features contiguous, as act and dz are
-// stored [row][64]) in the no-swizzle layout -- into TMEM, and its partial
-// bias gradient; mlp_dw_reduce_kernel adds the partials in chunk order.
-constexpr int kDwRows = 64;
+// Weight gradients on the fifth-generation tensor cores, all four layers in
+// one launch (blockIdx.y), split over the rows (the GEMM's K): CTA c forms the
+// partial dW = act^T dz of rows [c kDwRows, (c + 1) kDwRows) as one M = 128
+// (in features, padded with zero rows) x N = 64 (out features, zero-padded)
+// MMA chain from shared memory -- both operands MN-major (features
+// contiguous, as act and dz are stored [row][64]) in the no-swizzle layout --
+// into TMEM, and its partial bias gradient, at the layer's place in a flat
+// gradient vector (w1, b1, ... b4); mlp_dw_reduce_kernel adds the chunks'
+// vectors in order.  Four launches of 64-row chunks, each with its own
+// reduction, took 80 us of the 8,192-row step's kernels; the work is 0.2
+// GFLOP and 8 MB, so launches and tails were all of it.  With the tile
+// kernel's wide loads (below) the whole step went from 133 to 66 us.
+constexpr int kDwRows = 256;
 constexpr int kDwThreads = 128;
-constexpr int kDwPadSmem = 12 * 1024;
+constexpr int kDwFlat = MlpOffsets::total - MlpOffsets::w1;  // floats per chunk
+constexpr uint32_t kDwSbo = (kDwRows / 8) * 128;             // bytes between 8-feature groups
+// both operands; two such CTAs fit an SM, so no CTA waits in tcgen05.alloc
+constexpr size_t kDwSmem = (16 + 8) * (size_t)kDwSbo + 1024;
 __host__ __device__ constexpr uint32_t umma_idesc_bf16_mn(int n) {
     return umma_idesc_bf16(n) | (1u << 15) | (1u << 16);  // A and B MN-major
 }
 __global__ void __launch_bounds__(kDwThreads)
-mlp_dw_kernel(const __nv_bfloat16* __restrict__ act, const __nv_bfloat16* __restrict__ dz, int rows, int in_dim,
-              int out_dim, float* __restrict__ part_w, float* __restrict__ part_b) {
-    constexpr uint32_t kSbo = (kDwRows / 8) * 128;  // bytes between 8-feature groups
-    __shared__ __align__(1024) uint8_t s_a[128 * kDwRows * 2];
-    __shared__ __align__(1024) uint8_t s_b[64 * kDwRows * 2];
+mlp_dw_kernel(MlpTrainBufs bufs, int rows, float* __restrict__ part) {
+    constexpr uint32_t kSbo = kDwSbo;
+    extern __shared__ __align__(16) uint8_t s_dyn[];
+    uint8_t* s_a = s_dyn + ((1024u - (smem_addr(s_dyn) & 1023u)) & 1023u);
+    uint8_t* s_b = s_a + 16 * kSbo;
     __shared__ __align__(8) uint64_t s_bar;
     __shared__ uint32_t s_tmem;
-    const int tid = threadIdx.x, warp = tid >> 5, c = blockIdx.x;
+    const int tid = threadIdx.x, warp = tid >> 5, c = blockIdx.x, layer = blockIdx.y;
+    const int in_dim = layer == 0 ? kMlpIn : kMlpHid, out_dim = layer == 3 ? kMlpOut : kMlpHid;
+    using O = MlpOffsets;
+    const int w_off = (layer == 0 ? O::w1 : (layer == 1 ? O::w2 : (layer == 2 ? O::w3 : O::w4))) - O::w1;
+    const __nv_bfloat16* __restrict__ act = bufs.act[layer];
+    const __nv_bfloat16* __restrict__ dz = bufs.dz[layer];
     const int r0 = c * kDwRows, nr = min(kDwRows, rows - r0);
     // element (f, k) of a feature-major operand: feature group f / 8 at
     // kSbo, row group k / 8 at 128 bytes, row k % 8 at 16, feature f % 8 at 2
@@ -708,12 +775,15 @@ mlp_dw_kernel(const __nv_bfloat16* __restrict__ act, const __nv_bfloat16* __rest
         }
         return make_uint4(w[0], w[1], w[2], w[3]);
     };
+#pragma unroll 4
     for (int x = tid; x < kDwRows * 8; x += kDwThreads) {
         const int k = x >> 3, g = x & 7;
         uint4 va = make_uint4(0u, 0u, 0u, 0u), vb = va;
         if (k < nr) {
-            va = keep8(*reinterpret_cast<const uint4*>(act + (size_t)(r0 + k) * 64 + g * 8), g * 8, in_dim);
-            vb = keep8(*reinterpret_cast<const uint4*>(dz + (size_t)(r0 + k) * 64 + g * 8), g * 8, out_dim);
+            if (g * 8 < in_dim)
+                va = keep8(__ldg(reinterpret_cast<const uint4*>(act + (size_t)(r0 + k) * 64 + g * 8)), g * 8, in_dim);
+            if (g * 8 < out_dim)
+                vb = keep8(__ldg(reinterpret_cast<const uint4*>(dz + (size_t)(r0 + k) * 64 + g * 8)), g * 8, out_dim);
         }
         const uint32_t off = (uint32_t)g * kSbo + (uint32_t)(k >> 3) * 128u + (uint32_t)(k & 7) * 16u;
         *reinterpret_cast<uint4*>(s_a + off) = va;
@@ -743,9 +813,23 @@ mlp_dw_kernel(const __nv_bfloat16* __restrict__ act, const __nv_bfloat16* __rest
                       s > 0);
         umma_commit(&s_bar);
     }
+    // beside the MMAs: the bias gradient, two threads per output, 128 rows each
+    __shared__ float s_bias[kDwThreads];
+    {
+        const int f = tid & 63, k0 = (tid >> 6) * (kDwRows / 2);
+        const uint8_t* col = s_b + (uint32_t)(f >> 3) * kSbo + (uint32_t)(f & 7) * 2u;
+        float b4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+        for (int k = k0; k < k0 + kDwRows / 2; k += 4)
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                b4[u] += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(
+                    col + (uint32_t)((k + u) >> 3) * 128u + (uint32_t)((k + u) & 7) * 16u));
+        s_bias[tid] = (b4[0] + b4[1]) + (b4[2] + b4[3]);
+    }
     const bool ok = __syncthreads_and(mbar_wait(&s_bar, 0)) != 0;
     tc_fence_after();
-    float* pw = part_w + (size_t)c * 64 * 64;
+    float* pw = part + (size_t)c * kDwFlat + w_off;
     if (warp < 2) {  // TMEM lanes 0..63: the in features
         const int m = tid;
 #pragma unroll
@@ -753,15 +837,12 @@ mlp_dw_kernel(const __nv_bfloat16* __restrict__ act, const __nv_bfloat16* __rest
             float h[16];
             tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + c16, h);
 #pragma unroll
-            for (int q = 0; q < 16; ++q) pw[m * 64 + c16 + q] = ok ? h[q] : __int_as_float(0x7fc00000);
+            for (int q = 0; q < 16; ++q)
+                if (m < in_dim && c16 + q < out_dim)
+                    pw[m * out_dim + c16 + q] = ok ? h[q] : __int_as_float(0x7fc00000);
         }
     }
-    if (tid < 64) {  // partial bias gradient of output tid
-        float bacc = 0.f;
-        if (tid < out_dim)
-            for (int k = 0; k < nr; ++k) bacc += __bfloat162float(dz[(size_t)(r0 + k) * 64 + tid]);
-        part_b[(size_t)c * 64 + tid] = bacc;
-    }
+    if (tid < out_dim) pw[in_dim * out_dim + tid] = s_bias[tid] + s_bias[tid + 64];
     if (!ok) (void)mbar_wait(&s_bar, 0);  // the MMAs must be done before the columns go
     tc_fence_before();
     __syncthreads();
@@ -770,34 +851,42 @@ mlp_dw_kernel(const __nv_bfloat16* __restrict__ act, const __nv_bfloat16* __rest
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(64) : "memory");
 }
 
-// gw[in][out] and gb[out]: the chunks' partials added in chunk order.
-__global__ void mlp_dw_reduce_kernel(const float* __restrict__ part_w, const float* __restrict__ part_b, int chunks,
-                                     int in_dim, int out_dim, float* __restrict__ gw, float* __restrict__ gb) {
+// The gradient in the flat parameter layout (normalisation entries zero):
+// the chunks' vectors added in chunk order (a single chunk is the gradient
+// itself, part == grad + w1), and with `p` the Adam step on the FP32 master
+// weights (only the trainable slice, from w1).
+struct AdamArgs {
+    float* p;
+    float* m1;
+    float* m2;
+    float lr, b1, b2, eps, c1, c2;
+};
+__global__ void __launch_bounds__(128) mlp_dw_reduce_kernel(const float* part, int chunks, float* grad, int zero_norm,
+                                                             AdamArgs ad) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < in_dim * out_dim) {
-        const int m = q / out_dim, n = q % out_dim;
-        float acc = 0.f;
-        for (int c = 0; c < chunks; ++c) acc += part_w[(size_t)c * 64 * 64 + m * 64 + n];
-        gw[q] = acc;
-    } else if (q < in_dim * out_dim + out_dim) {
-        const int n = q - in_dim * out_dim;
-        float acc = 0.f;
-        for (int c = 0; c < chunks; ++c) acc += part_b[(size_t)c * 64 + n];
-        gb[n] = acc;
+    if (q >= MlpOffsets::total) return;
+    if (q < MlpOffsets::w1) {
+        if (zero_norm) grad[q] = 0.f;
+        return;
     }
-}
-
-// Adam on the FP32 master weights (only the trainable slice, from w1).
-__global__ void mlp_adam_kernel(float* __restrict__ p, const float* __restrict__ grad, float* __restrict__ m1,
-                                float* __restrict__ m2, int begin, int end, float lr, float b1, float b2,
-                                float eps, float c1, float c2) {
-    for (int q = begin + blockIdx.x * blockDim.x + threadIdx.x; q < end; q += gridDim.x * blockDim.x) {
-        const float gq = grad[q];
-        const float a = b1 * m1[q] + (1.f - b1) * gq;
-        const float b = b2 * m2[q] + (1.f - b2) * gq * gq;
-        m1[q] = a;
-        m2[q] = b;
-        p[q] -= lr * (a * c1) / (sqrtf(b * c2) + eps);
+    const float* src = part + (q - MlpOffsets::w1);
+    float gq = src[0];
+    int c = 1;
+    for (; c + 8 <= chunks; c += 8) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = src[(size_t)(c + u) * kDwFlat];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) gq += v[u];
+    }
+    for (; c < chunks; ++c) gq += src[(size_t)c * kDwFlat];
+    grad[q] = gq;
+    if (ad.p) {
+        const float a = ad.b1 * ad.m1[q] + (1.f - ad.b1) * gq;
+        const float b = ad.b2 * ad.m2[q] + (1.f - ad.b2) * gq * gq;
+        ad.m1[q] = a;
+        ad.m2[q] = b;
+        ad.p[q] -= ad.lr * (a * ad.c1) / (sqrtf(b * ad.c2) + ad.eps);
     }
 }
 
