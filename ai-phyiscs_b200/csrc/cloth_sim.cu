@@ -870,9 +870,9 @@ public:
     bool pc_active() const { return pc_kind_ >= 1 && resident_ && graph_path_ == kPathPersistent && sync_mode_ == 0; }
 
     // kernel actually used by the last graph build: 0 resident, 1 loop,
-    // 2 streamed
+    // 2 streamed (a contact operator's lists are, whichever kernel holds the rows)
     void solver_info(int* path, int* grid, int* block) const {
-        const int used = graph_path_ == kPathLoop ? 1 : (resident_ ? 0 : 2);
+        const int used = graph_path_ == kPathLoop ? 1 : (resident_ && !co_active_ ? 0 : 2);
         if (path) *path = used;
         if (grid) *grid = used == 1 ? 0 : plan_.grid;
         if (block) *block = used == 1 ? kVecBlock : (resident_ ? resident_warps_ * 32 : pcg_block_);
@@ -1393,6 +1393,15 @@ private:
                            ? reinterpret_cast<const void*>(&pcg_resident_kernel<16, kResidentMaxWidth, 0, 1>)
                            : reinterpret_cast<const void*>(&pcg_resident_kernel<8, kResidentMaxWidth, 0, 1>);
             }
+            if (co_active_ && SYNC == 0) {  // 16 warps, block-Jacobi (plan_resident)
+                if (cluster_)
+                    return topo_.max_width <= 6
+                               ? reinterpret_cast<const void*>(&pcg_resident_kernel<16, 6, 2, 0, 1>)
+                               : reinterpret_cast<const void*>(&pcg_resident_kernel<16, kResidentMaxWidth, 2, 0, 1>);
+                return topo_.max_width <= 6
+                           ? reinterpret_cast<const void*>(&pcg_resident_kernel<16, 6, 0, 0, 1>)
+                           : reinterpret_cast<const void*>(&pcg_resident_kernel<16, kResidentMaxWidth, 0, 0, 1>);
+            }
             if (cluster_ && SYNC == 0)
                 return topo_.max_width <= 6 ? reinterpret_cast<const void*>(&pcg_resident_kernel<16, 6, 2>)
                                             : reinterpret_cast<const void*>(&pcg_resident_kernel<16, kResidentMaxWidth, 2>);
@@ -1460,12 +1469,14 @@ private:
     bool plan_resident(int sms) {
         resident_ = false;  // a previous plan's choice must not leak into this one
         cluster_ = false;
-        // the register-resident rows hold symmetric blocks only
-        // (and have no contact-operator gather)
-        if (solver_path_ != kPathPersistent || topo_.max_width > kResidentMaxWidth || use_bending_ || co_active_)
+        // the register-resident rows hold symmetric blocks only; the contact
+        // operator's build is block-Jacobi in synchronisation mode 0
+        if (solver_path_ != kPathPersistent || topo_.max_width > kResidentMaxWidth || use_bending_ ||
+            (co_active_ && (pc_kind_ != 0 || sync_mode_ != 0)))
             return false;
         const int n_slices = std::max(1, topo_.n_slices);
         for (int W : {16, 8}) {
+            if (W == 8 && co_active_) break;
             resident_ = true;
             resident_warps_ = W;
             const int grid = (n_slices + W - 1) / W;

@@ -172,8 +172,8 @@ int chysx_cloth_get_static_contact(const chysx_cloth* h, float* thickness, float
  * and slips are given.  A contact whose stiffness is not finite and
  * positive is skipped; one with a weighted particle index outside the
  * particle range is dropped and counted (contact_stats).  Needs the
- * single-instance layout; a step with a contact operator uses the streamed
- * or graph-loop PCG kernel. */
+ * single-instance layout; the contact terms are streamed in every solver
+ * iteration, whichever kernel holds the rows (chysx_cloth_solver_info). */
 typedef struct chysx_contact_op {
     uintptr_t pairs;       /* int32 x 4 per contact, 16-byte aligned */
     uintptr_t weights;     /* float x 8 per contact: w0..w3, nx, ny, nz, depth; 16-byte aligned */
@@ -445,7 +445,9 @@ int chysx_cloth_row_of_particles(const chysx_cloth* h, int n, int32_t* rows);
 int chysx_cloth_set_preconditioner(chysx_cloth* h, int kind, int degree, float ratio);
 int chysx_cloth_preconditioner(const chysx_cloth* h, int* kind, int* degree, float* ratio, int* in_use);
 /* Kernel used at the last graph build: path 0 register-resident persistent,
- * 1 graph loop, 2 streamed persistent; with its grid and block size. */
+ * 1 graph loop, 2 streamed persistent (every kernel that reads part of the
+ * system again in each iteration: with a contact operator the register-
+ * resident rows too); with its grid and block size. */
 int chysx_cloth_solver_info(const chysx_cloth* h, int* path, int* grid, int* block);
 
 /* Measurement hooks (no counterpart in the reference): when enabled, the
