@@ -31,6 +31,7 @@
 #include "../../include/chysx_vbd.h"
 #include "cloth_kernels.cuh"
 #include "pcg_persistent.cuh"
+#include "pcg_tiled.cuh"
 #include "topology.h"
 #include "warm_mlp.cuh"
 
@@ -875,8 +876,9 @@ public:
         const int used = graph_path_ == kPathLoop ? 1 : (resident_ && !co_active_ ? 0 : 2);
         if (path) *path = used;
         if (grid) *grid = used == 1 ? 0 : plan_.grid;
-        if (block) *block = used == 1 ? kVecBlock : (resident_ ? resident_warps_ * 32 : pcg_block_);
+        if (block) *block = used == 1 ? kVecBlock : solver_block();
     }
+    int solver_block() const { return resident_ ? resident_warps_ * 32 : (tiled_ ? kTileThreads : pcg_block_); }
 
     // ---- autotuner (no counterpart in the reference) -------------------
     // Times the solver configurations that apply to the current system on
@@ -938,7 +940,7 @@ public:
         for (const Cand& c : cands) {
             solver_path_ = c.path;
             pcg_block_ = c.block;
-            pcg_block_req_ = c.block;
+            pcg_block_req_ = c.path == kPathPersistent ? 0 : c.block;  // path 0: the planner's own choice
             pcg_grid_req_ = 0;
             sync_mode_ = c.sync;
             graph_dirty_ = true;
@@ -967,7 +969,7 @@ public:
         if (!best) throw std::runtime_error("autotune: no configuration solved the system");
         solver_path_ = best->path;
         pcg_block_ = best->block;
-        pcg_block_req_ = best->block;
+        pcg_block_req_ = best->path == kPathPersistent ? 0 : best->block;
         pcg_grid_req_ = 0;
         sync_mode_ = best->sync;
         graph_dirty_ = true;
@@ -1412,6 +1414,13 @@ private:
                        ? reinterpret_cast<const void*>(&pcg_resident_kernel<16, kResidentMaxWidth, SYNC>)
                        : reinterpret_cast<const void*>(&pcg_resident_kernel<8, kResidentMaxWidth, SYNC>);
         }
+        if (tiled_) {
+            if (plan_.n_inst == 1)
+                return coarse_on_ ? reinterpret_cast<const void*>(&pcg_tiled_kernel<true, 1>)
+                                  : reinterpret_cast<const void*>(&pcg_tiled_kernel<true, 0>);
+            return coarse_on_ ? reinterpret_cast<const void*>(&pcg_tiled_kernel<false, 2>)
+                              : reinterpret_cast<const void*>(&pcg_tiled_kernel<false, 0>);
+        }
         if (pcg_block_ == 64) {
             // the planner's choice for batches with the coarse level only (synchronisation mode 0)
             if (SYNC != 0) throw std::logic_error("64-thread streamed kernel without synchronisation mode 0");
@@ -1438,6 +1447,7 @@ private:
     void* exchange_buffer(int k) const {
         const size_t np = (size_t)std::max(1, topo_.n_pad);
         if (resident_) return d_zp_.get() + k * np;
+        if (tiled_ && k == 0) return d_tile_.get();
         return nullptr;
     }
 
@@ -1782,7 +1792,86 @@ private:
         return c;
     }
 
+    // The tiled kernel's plan: one CTA per SM, every solver vector of its rows
+    // on the SM.  Chosen for every system that is too large for the
+    // register-resident kernel and fits: at most kTileMaxSlices slices per CTA
+    // (tensor memory), own and halo rows of p in shared memory.  A caller's
+    // block or grid request, synchronisation mode 1, general 3x3 blocks
+    // (bending) and the contact operator keep the streamed kernel.
+    bool plan_tiled(int sms) {
+        tiled_ = false;
+        if (solver_path_ != kPathPersistent || pcg_block_req_ != 0 || pcg_grid_req_ != 0 || sync_mode_ != 0 ||
+            use_bending_ || co_active_)
+            return false;
+        build_plan(topo_.inst_slice, std::min(sms, std::max(1, topo_.n_slices)), plan_);
+        if (plan_.max_slices_per_cta > kTileMaxSlices) return false;
+        // 16-bit columns: the CTA's own rows, then its halo in order of first use
+        const int grid = plan_.grid;
+        std::vector<unsigned short> lcol(std::max<size_t>(1, topo_.col.size())), halo_li;
+        std::vector<int> halo_off(grid + 1, 0), halo_row, stamp(std::max(1, topo_.n_pad), -1), index(stamp.size());
+        std::vector<unsigned> bmask(std::max(1, topo_.n_slices), 0u);
+        int max_halo = 0;
+        for (int c = 0; c < grid; ++c) {
+            const int r0 = plan_.cta_slice[c] * 32, own = plan_.cta_slice[c + 1] * 32 - r0;
+            const int first = (int)halo_row.size();
+            for (int e = topo_.slice_off[plan_.cta_slice[c]]; e < topo_.slice_off[plan_.cta_slice[c + 1]]; ++e) {
+                const int j = topo_.col[e];
+                if (j >= r0 && j < r0 + own) {
+                    lcol[e] = (unsigned short)(j - r0);
+                    continue;
+                }
+                if (stamp[j] != c) {
+                    stamp[j] = c;
+                    index[j] = own + (int)halo_row.size() - first;
+                    if (index[j] > 65535) return false;
+                    halo_row.push_back(j);
+                    halo_li.push_back((unsigned short)(plan_.slice_inst[j >> 5] - plan_.cta_inst_lo[c]));
+                    bmask[j >> 5] |= 1u << (j & 31);
+                }
+                lcol[e] = (unsigned short)index[j];
+            }
+            halo_off[c + 1] = (int)halo_row.size();
+            max_halo = std::max(max_halo, halo_off[c + 1] - halo_off[c]);
+        }
+        tiled_ = true;
+        int cols = 32;
+        while (cols < kTileCols * ((plan_.max_slices_per_cta + 3) / 4)) cols *= 2;
+        int dev = 0, limit = 0;
+        ck(cudaGetDevice(&dev), "cudaGetDevice");
+        ck(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "cudaDeviceGetAttribute");
+        plan_coarse();
+        pers_smem_ = tile_smem(plan_.n_inst == 1 ? kTileWarps : plan_.max_slices_per_cta, plan_.max_inst_per_cta,
+                               coarse_stream_smem(), plan_.max_slices_per_cta, max_halo).bytes;
+        cudaFuncAttributes fa{};
+        ck(cudaFuncGetAttributes(&fa, persistent_fn()), "cudaFuncGetAttributes(tiled)");
+        if (pers_smem_ + fa.sharedSizeBytes > (size_t)limit) {
+            tiled_ = false;
+            coarse_on_ = false;
+            coarse_batched_ = false;
+            return false;
+        }
+        ck(cudaFuncSetAttribute(persistent_fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pers_smem_),
+           "cudaFuncSetAttribute(tiled smem)");
+        d_tile_lcol_.upload(lcol);
+        d_tile_hoff_.upload(halo_off);
+        d_tile_hrow_.upload(halo_row.empty() ? std::vector<int>{0} : halo_row);
+        d_tile_hli_.upload(halo_li.empty() ? std::vector<unsigned short>{0} : halo_li);
+        d_tile_mask_.upload(bmask);
+        TileArgs ta{};
+        ta.lcol = d_tile_lcol_.get();
+        ta.halo_off = d_tile_hoff_.get();
+        ta.halo_row = d_tile_hrow_.get();
+        ta.halo_li = d_tile_hli_.get();
+        ta.bmask = d_tile_mask_.get();
+        ta.tmem_cols = cols;
+        ta.max_slices = plan_.max_slices_per_cta;
+        ta.max_halo = max_halo;
+        d_tile_.upload(&ta, 1);
+        return true;
+    }
+
     void plan_persistent() {
+        tiled_ = false;
         int dev = 0, sms = 0;
         ck(cudaGetDevice(&dev), "cudaGetDevice");
         ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
@@ -1790,6 +1879,10 @@ private:
             upload_plan();
             d_zp_.resize(2 * (size_t)std::max(1, topo_.n_pad));
             d_zp_.zero();
+            return;
+        }
+        if (plan_tiled(sms)) {
+            upload_plan();
             return;
         }
         if (pcg_block_req_ == 0) {
@@ -1843,6 +1936,10 @@ private:
     // launch: the kernel's shared-memory layout fits the bytes requested and
     // the resident kernel owns at most one slice per warp.
     void check_plan() const {
+        if (tiled_) {  // plan_tiled sized it
+            if (plan_.max_slices_per_cta > kTileMaxSlices) throw std::logic_error("tiled PCG plan exceeds tensor memory");
+            return;
+        }
         const size_t li_bytes = (size_t)plan_.max_inst_per_cta * sizeof(LocalInst);
         size_t need = resident_ ? (size_t)resident_warps_ * kSlotW * sizeof(double) + li_bytes
                                 : (size_t)plan_.max_slices_per_cta * kSlotW * sizeof(double) + li_bytes;
@@ -2094,7 +2191,7 @@ private:
             cudaKernelNodeParams p{};
             p.func = const_cast<void*>(persistent_fn());
             p.gridDim = dim3(plan_.grid);
-            p.blockDim = dim3(resident_ ? resident_warps_ * 32 : pcg_block_);
+            p.blockDim = dim3(solver_block());
             p.sharedMemBytes = (unsigned)pers_smem_;
             p.kernelParams = pargs;
             ck(cudaGraphAddKernelNode(&pcg_node_, graph_, &reset, 1, &p), "add persistent PCG node");
@@ -2246,7 +2343,7 @@ private:
             cudaKernelNodeParams pp{};
             pp.func = const_cast<void*>(persistent_fn());
             pp.gridDim = dim3(plan_.grid);
-            pp.blockDim = dim3(resident_ ? resident_warps_ * 32 : pcg_block_);
+            pp.blockDim = dim3(solver_block());
             pp.sharedMemBytes = (unsigned)pers_smem_;
             pp.kernelParams = pargs;
             ck(cudaGraphExecKernelNodeSetParams(exec_, pcg_node_, &pp), "update persistent PCG node");
@@ -2359,6 +2456,11 @@ private:
     int row_order_ = 0;
     std::vector<int> order_;  // particles in row order (row_order_ 1)
     bool resident_ = false;
+    bool tiled_ = false;    // the tiled kernel (streamed matrix, vectors on the SM)
+    DevBuf<unsigned short> d_tile_lcol_, d_tile_hli_;
+    DevBuf<int> d_tile_hoff_, d_tile_hrow_;
+    DevBuf<unsigned> d_tile_mask_;
+    DevBuf<TileArgs> d_tile_;
     bool cluster_ = false;  // the resident plan runs as one thread-block cluster
     int resident_warps_ = 16;
     std::vector<TuneResult> tune_;

@@ -1,0 +1,685 @@
+// Tiled persistent PCG: one CTA per SM keeps every solver vector of its rows
+// on the SM for the whole solve and streams nothing but the matrix.
+//
+// The streamed kernel (pcg_persistent.cuh) re-reads z, p, x, r, A p of every
+// row each iteration and gathers each neighbour's z and old p from L2: 32 B
+// per entry on top of the entry's own 28, so its 96 us iteration at 1024 x
+// 1024 rows is bound by L2 traffic (~0.7 GB), not by the 0.4 GB that must come
+// from HBM.  Here
+//   * p of the CTA's rows and of its halo (the other CTAs' rows that its
+//     entries reach) lies in shared memory, and entries carry 16-bit indices
+//     into it, so a gather is a shared-memory read;
+//   * x, r and A p (then z in the same place) lie in tensor memory, used as
+//     plain storage: 9 columns of one warp's 32 lanes per 32-row slice, 512
+//     columns, i.e. up to 224 slices (7,168 rows) per SM;
+//   * x takes alpha p one iteration later, when p is at hand anyway;
+//   * only z of rows in another CTA's halo goes through global memory: the
+//     owner writes it with the update, every CTA forms the halo's p = z +
+//     beta p itself, with the arithmetic of the owner (identical values).
+// Per iteration a row costs its blocks and 16-bit columns (26 B each), D'
+// and M^-1 (48 B), and 32 B of coarse weights with the coarse level.
+// Measured on B200, streamed against tiled: 801 x 643 rows, 50 iterations,
+// 2.88 against 1.48 ms (53 against 25 us per iteration); 1024 x 1024 with the
+// coarse level 118 against 56 us per iteration; a batch of 128 grids of 16 to
+// 128 a side 105 against 47.
+//
+// Phases, per-instance logic, preconditioner (block-Jacobi, or with a coarse
+// level: CO = 1 dense, CO = 2 batched) and stopping rules are those of
+// pcg_persistent_kernel; symmetric blocks only, synchronisation by the
+// counter barrier.  ONE: a single instance, whose per-row sums are kept per
+// thread and added once per phase.
+#pragma once
+
+#include "pcg_persistent.cuh"
+
+namespace chysx_b200 {
+
+constexpr int kTileThreads = 1024;
+constexpr int kTileWarps = kTileThreads / 32;
+constexpr int kTileCols = 9;          // TMEM columns per slice: x, r, A p / z
+constexpr int kTileMaxSlices = 224;   // 4 lane quarters x 56 slices x 9 columns <= 512
+
+struct TileArgs {
+    const unsigned short* lcol;       // [ELL entries] own row (< the CTA's rows) or rows + halo index
+    const int* halo_off;              // [grid + 1]
+    const int* halo_row;              // internal row of every halo entry
+    const unsigned short* halo_li;    // its instance, relative to the CTA's first
+    const unsigned* bmask;            // [n_slices] rows in some halo, one bit per lane
+    int tmem_cols;                    // columns allocated (power of two >= 32)
+    int max_slices;                   // per CTA
+    int max_halo;
+};
+
+// Dynamic shared memory: slice partials, instance records, coarse values,
+// slice offsets / masks / instances, halo rows and instances, p.
+__host__ __device__ inline size_t tile_align(size_t v) { return (v + 15) & ~static_cast<size_t>(15); }
+struct TileSmem {
+    size_t li, vbuf, soff, mask, sli, hrow, hli, p, bytes;
+};
+__host__ __device__ inline TileSmem tile_smem(int parts, int max_inst, size_t coarse_bytes, int max_slices,
+                                              int max_halo) {
+    TileSmem s;
+    s.li = (size_t)parts * kSlotW * sizeof(double);
+    s.vbuf = tile_align(s.li + (size_t)max_inst * sizeof(LocalInst));
+    s.soff = tile_align(s.vbuf + coarse_bytes);
+    s.mask = s.soff + (size_t)(max_slices + 1) * sizeof(int);
+    s.sli = s.mask + (size_t)max_slices * sizeof(unsigned);
+    s.hrow = tile_align(s.sli + (size_t)max_slices * sizeof(unsigned short));
+    s.hli = s.hrow + (size_t)max_halo * sizeof(int);
+    s.p = tile_align(s.hli + (size_t)max_halo * sizeof(unsigned short));
+    s.bytes = s.p + (size_t)3 * (32 * (size_t)max_slices + max_halo) * sizeof(float);
+    return s;
+}
+
+// ---- tensor memory as storage: this warp's 32 lanes, consecutive columns ----
+__device__ __forceinline__ void tm_ld1(uint32_t a, float& x) {
+    uint32_t u;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(u) : "r"(a) : "memory");
+    x = __uint_as_float(u);
+}
+__device__ __forceinline__ void tm_ld2(uint32_t a, float& x, float& y) {
+    uint32_t u, v;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(u), "=r"(v) : "r"(a) : "memory");
+    x = __uint_as_float(u);
+    y = __uint_as_float(v);
+}
+__device__ __forceinline__ void tm_ld4(uint32_t a, float& x, float& y, float& z, float& w) {
+    uint32_t u, v, s, t;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(u), "=r"(v), "=r"(s), "=r"(t)
+                 : "r"(a)
+                 : "memory");
+    x = __uint_as_float(u);
+    y = __uint_as_float(v);
+    z = __uint_as_float(s);
+    w = __uint_as_float(t);
+}
+// the loads above have arrived in a and b (which pass through, so no use moves ahead of the wait)
+__device__ __forceinline__ void tm_wait_ld(float3& a, float3& b) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+f"(a.x), "+f"(a.y), "+f"(a.z), "+f"(b.x), "+f"(b.y), "+f"(b.z)
+                 :
+                 : "memory");
+}
+__device__ __forceinline__ void tm_st1(uint32_t a, float x) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(a), "r"(__float_as_uint(x)) : "memory");
+}
+__device__ __forceinline__ void tm_st2(uint32_t a, float x, float y) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(a), "r"(__float_as_uint(x)),
+                 "r"(__float_as_uint(y))
+                 : "memory");
+}
+__device__ __forceinline__ void tm_st4(uint32_t a, float x, float y, float z, float w) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(__float_as_uint(x)),
+                 "r"(__float_as_uint(y)), "r"(__float_as_uint(z)), "r"(__float_as_uint(w))
+                 : "memory");
+}
+__device__ __forceinline__ void tm_wait_st() {
+    __syncwarp();
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tm_ld3(uint32_t a, float3& v) {
+    __syncwarp();  // .sync.aligned: the warp must have reconverged
+    tm_ld2(a, v.x, v.y);
+    tm_ld1(a + 2, v.z);
+}
+__device__ __forceinline__ void tm_st3(uint32_t a, float3 v) {
+    __syncwarp();
+    tm_st2(a, v.x, v.y);
+    tm_st1(a + 2, v.z);
+}
+// columns of a slice
+constexpr uint32_t kTmX = 0, kTmR = 3, kTmQ = 6;
+
+// streaming loads: read once per phase, not worth an L1 line
+__device__ __forceinline__ float ld_na(const float* p) {
+    float v;
+    asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ S6 ld6_na(const float* p) {
+    return S6{ld_na(p), ld_na(p + 32), ld_na(p + 64), ld_na(p + 96), ld_na(p + 128), ld_na(p + 160)};
+}
+__device__ __forceinline__ int ld_na(const unsigned short* p) {
+    unsigned short v;
+    asm volatile("ld.global.L1::no_allocate.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    return v;
+}
+
+template <bool ONE, int CO>
+__global__ void __launch_bounds__(kTileThreads, 1)
+pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const TileArgs* ta, void*) {
+    constexpr int SYNC = 0;  // slot_set: two sets by parity
+    constexpr int BLOCK = kTileThreads;
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    __shared__ int s_flag, s_exit;
+    __shared__ uint32_t s_tmem;
+    __shared__ float s_tmp[CO ? BLOCK : 1];
+    __shared__ float s_cb[12], s_c0[12], s_cw[12], s_cu[12], s_cn[12];
+    __shared__ CoarseRegs creg;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int s0 = bp.cta_slice[blockIdx.x], s1 = bp.cta_slice[blockIdx.x + 1], ns = s1 - s0;
+    const int il0 = bp.cta_inst_lo[blockIdx.x], il1 = bp.cta_inst_hi[blockIdx.x];
+    const int nloc = il1 - il0 + 1;
+    const TileArgs T = *ta;
+    const int h0 = T.halo_off[blockIdx.x], nh = T.halo_off[blockIdx.x + 1] - h0;
+    const int nown = ns * 32;
+    const bool coarse = CO == 1 && bp.cg != nullptr && bp.cg->on && bp.cg->dense && *(volatile int*)bp.cg->fail == 0;
+    const bool coarse_b =
+        CO == 2 && !warm && bp.cg != nullptr && bp.cg->on && bp.cg->batched && *(volatile int*)bp.cg->fail == 0;
+    const bool any_c = coarse || coarse_b;
+    const size_t cbytes = CO == 1 ? (bp.cg ? (size_t)bp.cg->m * sizeof(float) + 16 : 0)
+                                  : (CO == 2 ? (size_t)bp.max_inst_per_cta * kInstCoarseW * sizeof(float) + 16 : 0);
+    const TileSmem lay = tile_smem(ONE ? kTileWarps : T.max_slices, bp.max_inst_per_cta, cbytes, T.max_slices,
+                                   T.max_halo);
+    double* spart = reinterpret_cast<double*>(s_raw);
+    LocalInst* li = reinterpret_cast<LocalInst*>(s_raw + lay.li);
+    float* c_vbuf = reinterpret_cast<float*>(s_raw + lay.vbuf);
+    float* c_inst = c_vbuf;
+    int* s_off = reinterpret_cast<int*>(s_raw + lay.soff);
+    unsigned* s_mask = reinterpret_cast<unsigned*>(s_raw + lay.mask);
+    unsigned short* s_sli = reinterpret_cast<unsigned short*>(s_raw + lay.sli);
+    int* s_hrow = reinterpret_cast<int*>(s_raw + lay.hrow);
+    unsigned short* s_hli = reinterpret_cast<unsigned short*>(s_raw + lay.hli);
+    float* s_p = reinterpret_cast<float*>(s_raw + lay.p);
+    unsigned target = 0;
+    int ph = 0;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         static_cast<uint32_t>(__cvta_generic_to_shared(&s_tmem))),
+                     "r"(T.tmem_cols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        s_flag = 0;
+        s_exit = 0;
+        creg = coarse_regs(bp, any_c);
+    }
+    init_local(bp, li, s0, s1, il0, il1);
+    for (int k = tid; k <= ns; k += BLOCK) s_off[k] = t.slice_off[s0 + k];
+    for (int k = tid; k < ns; k += BLOCK) {
+        s_mask[k] = T.bmask[s0 + k];
+        s_sli[k] = (unsigned short)(bp.slice_inst[s0 + k] - il0);
+    }
+    for (int h = tid; h < nh; h += BLOCK) {
+        s_hrow[h] = T.halo_row[h0 + h];
+        s_hli[h] = ONE ? 0 : T.halo_li[h0 + h];
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (ONE && tid == 0) {  // the partials are per warp
+        li[0].seg_lo = 0;
+        li[0].seg_hi = kTileWarps;
+    }
+    __syncthreads();
+    const uint32_t tm_warp = s_tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    auto tm = [&](int k) { return tm_warp + (uint32_t)(kTileCols * (k >> 2)); };  // slice k of the CTA (k % 4 == warp % 4)
+    bool ok = true;
+    auto no_step = [](LocalInst&, const double*) {};
+    const int& c_U = creg.U;
+    const int& c_nq = creg.nq;
+    auto cw = [&](int i) { return c_nq == 4 ? __ldg(creg.w + i) : make_float4(0.f, 0.f, 0.f, 0.f); };
+    auto seg_one = [&](int, int& lo, int& hi, int& slot) {
+        lo = 0;
+        hi = kTileWarps;
+        slot = li[0].own_slot;
+    };
+    auto seg_inst = [&](int q, int& lo, int& hi, int& slot) {
+        lo = li[q].seg_lo;
+        hi = li[q].seg_hi;
+        slot = li[q].own_slot;
+    };
+    auto inst_of = [&](int k) { return ONE ? 0 : (int)s_sli[k]; };
+    auto ldp = [&](int j) { return f3(s_p[3 * j], s_p[3 * j + 1], s_p[3 * j + 2]); };
+    auto stp = [&](int j, float3 a) {
+        s_p[3 * j] = a.x;
+        s_p[3 * j + 1] = a.y;
+        s_p[3 * j + 2] = a.z;
+    };
+    // restriction of a slice's vector into its partial (spart entry `part`)
+    auto restrict_part = [&](float3 a, float4 w4, int part) { warp_restrict(c_nq, a, w4, slice_cpart(spart, part)); };
+    // the CTA's restrictions into the slots of this phase
+    auto publish_coarse = [&]() {
+        if (ONE) coarse_publish<BLOCK>(bp, c_U, spart, 1, seg_one, slot_set(ph), s_tmp);
+        else coarse_publish<BLOCK>(bp, c_U, spart, nloc, seg_inst, slot_set(ph), s_tmp);
+    };
+    // One reduction phase, after the partials and a __syncthreads: a warp per
+    // instance publishes the CTA's segment, thread 0 meets the other CTAs, a
+    // warp per instance reads the totals and applies `step`.
+    auto phase = [&](auto nv, bool exit_test, auto&& step) {
+        constexpr int NV = decltype(nv)::value;
+        const int set = slot_set(ph);
+        for (int q = warp; q < nloc; q += kTileWarps) {
+            const LocalInst& L = li[q];
+            if (L.done) continue;
+            double acc[NV];
+#pragma unroll
+            for (int u = 0; u < NV; ++u) acc[u] = 0.0;
+            for (int sl = L.seg_lo + lane; sl < L.seg_hi; sl += 32) {
+#pragma unroll
+                for (int u = 0; u < NV; ++u) acc[u] += spart[sl * kSlotW + u];
+            }
+#pragma unroll
+            for (int u = 0; u < NV; ++u) {
+                acc[u] = warp_sum(acc[u]);
+                if (lane == 0) bp.slots[((size_t)set * bp.n_slots + L.own_slot) * kSlotW + u] = acc[u];
+            }
+        }
+        __syncthreads();
+        if (tid == 0) {
+            if (!barrier_arrive_wait(bp.bar, target)) s_flag = 1;
+            else if (exit_test) s_exit = *(volatile unsigned*)&bp.bar->ndone >= (unsigned)bp.n_inst;
+        }
+        __syncthreads();
+        if (!s_flag) {
+            for (int q = warp; q < nloc; q += kTileWarps) {
+                LocalInst& L = li[q];
+                if (L.done) continue;
+                constexpr int KP = 5;  // one pass covers 160 CTAs
+                double tot[NV];
+#pragma unroll
+                for (int u = 0; u < NV; ++u) tot[u] = 0.0;
+                for (int c0 = L.slot_lo; c0 < L.slot_hi; c0 += 32 * KP) {
+                    constexpr int NP = NV > 2 ? 2 : NV;  // values in flight together (registers)
+#pragma unroll
+                    for (int u0 = 0; u0 < NV; u0 += NP) {
+                        double val[KP][NP];
+#pragma unroll
+                        for (int j = 0; j < KP; ++j)
+#pragma unroll
+                            for (int u = 0; u < NP; ++u) {
+                                const int k = c0 + j * 32 + lane;
+                                val[j][u] = k < L.slot_hi
+                                                ? __ldcg(bp.slots + ((size_t)set * bp.n_slots + k) * kSlotW + u0 + u)
+                                                : 0.0;
+                            }
+#pragma unroll
+                        for (int j = 0; j < KP; ++j)
+#pragma unroll
+                            for (int u = 0; u < NP; ++u) tot[u0 + u] += val[j][u];
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < NV; ++u) tot[u] = warp_sum(tot[u]);
+                if (lane == 0) step(L, tot);
+                __syncwarp();
+            }
+        }
+        ++ph;
+        __syncthreads();
+    };
+    using N1 = std::integral_constant<int, 1>;
+    using N2 = std::integral_constant<int, 2>;
+    using N8 = std::integral_constant<int, kStartW>;
+    // one exchange phase carrying only the restriction in the partials
+    auto coarse_exchange = [&](float* out) {
+        __syncthreads();
+        publish_coarse();
+        const int set = slot_set(ph);
+        phase(N1{}, false, no_step);
+        if (!s_flag) {
+            if (coarse) coarse_apply_dense<BLOCK>(bp, creg, set, c_vbuf, out);
+            if (coarse_b) {
+                coarse_apply_inst(bp, creg, li, nloc, set, c_inst, kCU, kTileWarps, false);
+                __syncthreads();
+            }
+        }
+        ok = s_flag == 0;
+    };
+    // (A p)_i = D'_i p_i + sum_j A_ij (p_j - p_i) of row `lane` of slice k, p in shared memory
+    auto row_product = [&](int k, float3 pi) {
+        const int s = s0 + k;
+        const int so = s_off[k], w = (s_off[k + 1] - so) >> 5;
+        const float* vb = t.val + (size_t)so * 6 + lane;
+        const unsigned short* lc = T.lcol + so + lane;
+        float3 acc = f3(0.f, 0.f, 0.f);
+        if (s * 32 + lane < t.n) acc = mul(ld6_na(t.dnl + (size_t)s * 192 + lane), pi);
+        if (w == 6) {
+#pragma unroll
+            for (int e = 0; e < 6; ++e) acc = acc + mul(ld6_na(vb + e * 192), ldp(ld_na(lc + e * 32)) - pi);
+        } else {
+            for (int e = 0; e < w; ++e) acc = acc + mul(ld6_na(vb + e * 192), ldp(ld_na(lc + e * 32)) - pi);
+        }
+        return acc;
+    };
+    // per-thread sums of a phase: added over the warp once (ONE) or per slice
+    struct Sums {
+        double a, b;
+        float3 c[4];
+    };
+    auto zero_sums = [](Sums& q) {
+        q.a = q.b = 0.0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) q.c[u] = f3(0.f, 0.f, 0.f);
+    };
+    auto add_restrict = [](Sums& q, float3 a, float4 w4) {
+        q.c[0] = q.c[0] + a;
+        q.c[1] = f3(fmaf(w4.x, a.x, q.c[1].x), fmaf(w4.x, a.y, q.c[1].y), fmaf(w4.x, a.z, q.c[1].z));
+        q.c[2] = f3(fmaf(w4.y, a.x, q.c[2].x), fmaf(w4.y, a.y, q.c[2].y), fmaf(w4.y, a.z, q.c[2].z));
+        q.c[3] = f3(fmaf(w4.z, a.x, q.c[3].x), fmaf(w4.z, a.y, q.c[3].y), fmaf(w4.z, a.z, q.c[3].z));
+    };
+    auto put_restrict = [&](const Sums& q) {  // the warp's 12 sums into its partial
+        const float a[16] = {q.c[0].x, q.c[0].y, q.c[0].z, q.c[1].x, q.c[1].y, q.c[1].z, q.c[2].x, q.c[2].y,
+                             q.c[2].z, q.c[3].x, q.c[3].y, q.c[3].z, 0.f, 0.f, 0.f, 0.f};
+        const float y = warp_sum16(a);
+        const int u = lane >> 1;
+        if ((lane & 1) == 0 && u < 12) slice_cpart(spart, warp)[u] = y;
+    };
+    // restriction of a per-row vector get(k, i) into the partials
+    auto restrict_all = [&](auto&& get) {
+        Sums sm;
+        zero_sums(sm);
+        for (int k = warp; k < ns; k += kTileWarps) {
+            const int i = (s0 + k) * 32 + lane;
+            const float3 a = get(k, i);
+            const float4 w4 = i < t.n ? cw(i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (ONE) add_restrict(sm, a, w4);
+            else {
+                if (lane == 0) spart[k * kSlotW] = 0.0;
+                restrict_part(a, w4, k);
+            }
+        }
+        if (ONE) {
+            if (lane == 0) spart[warp * kSlotW] = 0.0;
+            put_restrict(sm);
+        }
+    };
+    auto load_b = [&](int, int i) { return i < t.n ? xyz(v.b[i]) : f3(0.f, 0.f, 0.f); };
+    auto load_minv = [&](int s, int i) {
+        S6 m{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (i < t.n) m = ld6_na(t.minv + (size_t)s * 192 + lane);
+        return m;
+    };
+    auto publish_z = [&](int k, int i, float3 z) {
+        if ((s_mask[k] >> lane) & 1u) __stcg(v.z + i, f4(z));
+    };
+
+    // ---- start: r = b - A x0, z = M^-1 r, the instances' start values -------
+    if (any_c) {
+        restrict_all(load_b);
+        coarse_exchange(s_cb);  // A_c^-1 R^T b (coarse_b: into kCU)
+    }
+    if (ok && warm) {
+        for (int k = warp; k < ns; k += kTileWarps) {
+            const int i = (s0 + k) * 32 + lane;
+            stp(k * 32 + lane, i < t.n ? xyz(v.x[i]) : f3(0.f, 0.f, 0.f));
+        }
+        for (int h = tid; h < nh; h += BLOCK) stp(nown + h, xyz(ldcg4(v.x + s_hrow[h])));
+        __syncthreads();
+        for (int k = warp; k < ns; k += kTileWarps) {
+            const int i = (s0 + k) * 32 + lane;
+            const float3 ax = row_product(k, ldp(k * 32 + lane));
+            tm_st3(tm(k) + kTmR, load_b(k, i) - ax);
+        }
+        tm_wait_st();
+        if (coarse) {
+            restrict_all([&](int k, int) {
+                float3 r, d = f3(0.f, 0.f, 0.f);
+                tm_ld3(tm(k) + kTmR, r);
+                tm_wait_ld(r, d);
+                return r;
+            });
+            coarse_exchange(s_c0);  // A_c^-1 R^T r0
+        }
+    }
+    auto zb_of = [&](int k, int i, const S6& Mi, float3 b, float4 w4) {
+        float3 zb = mul(Mi, b);
+        if (coarse) zb = zb + coarse_prolong(c_nq, s_cb, w4);
+        if (coarse_b) zb = zb + coarse_prolong(c_nq, c_inst + inst_of(k) * kInstCoarseW + kCU, w4);
+        return zb;
+    };
+    if (ok) {
+        double tot[kStartW];
+#pragma unroll
+        for (int u = 0; u < kStartW; ++u) tot[u] = 0.0;
+        for (int k = warp; k < ns; k += kTileWarps) {
+            const int i = (s0 + k) * 32 + lane;
+            const S6 Mi = load_minv(s0 + k, i);
+            const float4 w4 = any_c && i < t.n ? cw(i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float3 b = load_b(k, i), zb = zb_of(k, i, Mi, b, w4);
+            float3 x0 = f3(0.f, 0.f, 0.f), r = b, z = zb;
+            if (warm) {
+                float3 d = f3(0.f, 0.f, 0.f);
+                tm_ld3(tm(k) + kTmR, r);
+                tm_wait_ld(r, d);
+                x0 = ldp(k * 32 + lane);
+                z = mul(Mi, r);
+                if (coarse) z = z + coarse_prolong(c_nq, s_c0, w4);
+            } else {
+                tm_st3(tm(k) + kTmX, x0);
+                tm_st3(tm(k) + kTmR, r);
+                tm_st3(tm(k) + kTmQ, z);
+                publish_z(k, i, z);
+            }
+            const double q8[kStartW] = {dot3d(r, z), dot3d(r, r), dot3d(b, b), dot3d(b, zb),
+                                        dot3d(x0, b), dot3d(x0, r), dot3d(b, z), dot3d(b, r)};
+            if (ONE) {
+#pragma unroll
+                for (int u = 0; u < kStartW; ++u) tot[u] += q8[u];
+            } else {
+#pragma unroll
+                for (int u = 0; u < kStartW; ++u) {
+                    const double y = warp_sum(q8[u]);
+                    if (lane == 0) spart[k * kSlotW + u] = y;
+                }
+            }
+        }
+        tm_wait_st();
+        if (ONE) {
+#pragma unroll
+            for (int u = 0; u < kStartW; ++u) {
+                const double y = warp_sum(tot[u]);
+                if (lane == 0) spart[warp * kSlotW + u] = y;
+            }
+        }
+        __syncthreads();
+        phase(N8{}, false, [&](LocalInst& L, const double* q) { step_start(bp, L, q, cfg, warm); });
+        ok = s_flag == 0;
+    }
+    if (ok && warm) {
+        // the scaled guess, or the zero guess where the instance fell back
+        for (int k = warp; k < ns; k += kTileWarps) {
+            const int i = (s0 + k) * 32 + lane;
+            const S6 Mi = load_minv(s0 + k, i);
+            const float4 w4 = any_c && i < t.n ? cw(i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float3 b = load_b(k, i);
+            float3 x = ldp(k * 32 + lane), r, z, d = f3(0.f, 0.f, 0.f);
+            tm_ld3(tm(k) + kTmR, r);
+            tm_wait_ld(r, d);
+            const LocalInst& L = li[inst_of(k)];
+            if (coarse) {
+                z = mul(Mi, r) + coarse_prolong(c_nq, s_c0, w4);
+                start_row_linear(L, b, zb_of(k, i, Mi, b, w4), x, r, z);
+            } else {
+                start_row(L, b, Mi, x, r, z);
+            }
+            tm_st3(tm(k) + kTmX, x);
+            tm_st3(tm(k) + kTmR, r);
+            tm_st3(tm(k) + kTmQ, z);
+            publish_z(k, i, z);
+        }
+        tm_wait_st();
+        // a data-free phase orders the new z before any halo read
+        for (int q = tid; q < (ONE ? kTileWarps : ns); q += BLOCK) spart[q * kSlotW] = 0.0;
+        __syncthreads();
+        phase(N1{}, false, no_step);
+        ok = s_flag == 0;
+    }
+    if (coarse && ok) {
+        const LocalInst& L0 = li[0];
+        const bool from_r0 = warm && !L0.fallback;
+        if (tid < c_U) s_cu[tid] = from_r0 ? fmaf(L0.scale, s_c0[tid], L0.scale_b * s_cb[tid]) : s_cb[tid];
+        __syncthreads();
+    }
+
+    // ---- iterations ---------------------------------------------------------
+    const int iter_cap = cfg.max_iter + 2;
+    for (int guard = 0; ok && guard < iter_cap; ++guard) {
+        if (ONE && li[0].done) break;  // uniform over the grid: every CTA forms the same totals
+        // p = z + beta p of the own rows and, from the published z, of the
+        // halo; x takes the previous iteration's alpha p
+        for (int k = warp; k < ns; k += kTileWarps) {
+            const LocalInst& L = li[inst_of(k)];
+            if (L.done) continue;
+            float3 z, x = f3(0.f, 0.f, 0.f);
+            tm_ld3(tm(k) + kTmQ, z);
+            if (L.iter > 0) {
+                tm_ld3(tm(k) + kTmX, x);
+                const float3 p = ldp(k * 32 + lane);
+                const float al = L.alpha, be = L.beta;
+                tm_wait_ld(z, x);
+                tm_st3(tm(k) + kTmX, f3(fmaf(al, p.x, x.x), fmaf(al, p.y, x.y), fmaf(al, p.z, x.z)));
+                z = f3(fmaf(be, p.x, z.x), fmaf(be, p.y, z.y), fmaf(be, p.z, z.z));
+            } else {
+                tm_wait_ld(z, x);
+            }
+            stp(k * 32 + lane, z);
+        }
+        for (int h = tid; h < nh; h += BLOCK) {
+            const LocalInst& L = li[ONE ? 0 : s_hli[h]];
+            if (L.done) continue;
+            float3 z = xyz(ldcg4(v.z + s_hrow[h]));
+            if (L.iter > 0) {
+                const float3 p = ldp(nown + h);
+                const float be = L.beta;
+                z = f3(fmaf(be, p.x, z.x), fmaf(be, p.y, z.y), fmaf(be, p.z, z.z));
+            }
+            stp(nown + h, z);
+        }
+        __syncthreads();
+        // A p, sigma = p.A p (and the restriction of A p)
+        {
+            Sums sm;
+            zero_sums(sm);
+            for (int k = warp; k < ns; k += kTileWarps) {
+                const LocalInst& L = li[inst_of(k)];
+                if (L.done) continue;
+                const int i = (s0 + k) * 32 + lane;
+                const float4 w4 = any_c && i < t.n ? cw(i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float3 pi = ldp(k * 32 + lane);
+                const float3 acc = row_product(k, pi);
+                tm_st3(tm(k) + kTmQ, acc);
+                const double sig = (double)pi.x * acc.x + (double)pi.y * acc.y + (double)pi.z * acc.z;
+                if (ONE) {
+                    sm.a += sig;
+                    if (CO == 1) add_restrict(sm, acc, w4);
+                } else {
+                    const double y = warp_sum(sig);
+                    if (lane == 0) spart[k * kSlotW] = y;
+                    if (coarse_b) restrict_part(acc, w4, k);
+                }
+            }
+            if (ONE) {
+                const double y = warp_sum(sm.a);
+                if (lane == 0) spart[warp * kSlotW] = y;
+                if (CO == 1) put_restrict(sm);
+            }
+            tm_wait_st();
+        }
+        __syncthreads();
+        if (any_c) publish_coarse();
+        const int set1 = slot_set(ph);
+        phase(N1{}, !ONE, [&](LocalInst& L, const double* q) { step_alpha(L, q); });
+        if (s_flag) {
+            ok = false;
+            break;
+        }
+        // every CTA reads ndone between the same two barriers, where it does not change
+        if (!ONE && s_exit) break;
+        if (coarse) {
+            coarse_apply_dense<BLOCK>(bp, creg, set1, c_vbuf, s_cw);
+            if (tid < c_U) s_cn[tid] = fmaf(-li[0].alpha, s_cw[tid], s_cu[tid]);
+            __syncthreads();
+        }
+        if (coarse_b) {
+            coarse_apply_inst(bp, creg, li, nloc, set1, c_inst, 0, kTileWarps, true);
+            __syncthreads();
+        }
+        // r -= alpha A p; z = M^-1 r (+ its coarse part)
+        {
+            Sums sm;
+            zero_sums(sm);
+            for (int k = warp; k < ns; k += kTileWarps) {
+                const int q = inst_of(k);
+                const LocalInst& L = li[q];
+                if (L.done) continue;
+                const int i = (s0 + k) * 32 + lane;
+                float3 r, ap;
+                __syncwarp();
+                tm_ld4(tm(k) + kTmR, r.x, r.y, r.z, ap.x);
+                tm_ld2(tm(k) + kTmQ + 1, ap.y, ap.z);
+                const S6 Mi = load_minv(s0 + k, i);
+                const float4 w4 = any_c && i < t.n ? cw(i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float al = L.alpha;
+                tm_wait_ld(r, ap);
+                const float3 rn = f3(fmaf(-al, ap.x, r.x), fmaf(-al, ap.y, r.y), fmaf(-al, ap.z, r.z));
+                float3 zn = mul(Mi, rn);
+                if (coarse) zn = zn + coarse_prolong(c_nq, s_cn, w4);
+                if (coarse_b) zn = zn + coarse_prolong(c_nq, c_inst + q * kInstCoarseW + kCN, w4);
+                __syncwarp();
+                tm_st4(tm(k) + kTmR, rn.x, rn.y, rn.z, zn.x);
+                tm_st2(tm(k) + kTmQ + 1, zn.y, zn.z);
+                publish_z(k, i, zn);
+                const double rz = dot3d(rn, zn), rr = dot3d(rn, rn);
+                if (ONE) {
+                    sm.a += rz;
+                    sm.b += rr;
+                    if (CO == 1) add_restrict(sm, rn, w4);
+                } else {
+                    const double y = warp_sum(rz), y2 = warp_sum(rr);
+                    if (lane == 0) {
+                        spart[k * kSlotW] = y;
+                        spart[k * kSlotW + 1] = y2;
+                    }
+                    if (coarse_b) restrict_part(rn, w4, k);
+                }
+            }
+            if (ONE) {
+                const double y = warp_sum(sm.a), y2 = warp_sum(sm.b);
+                if (lane == 0) {
+                    spart[warp * kSlotW] = y;
+                    spart[warp * kSlotW + 1] = y2;
+                }
+                if (CO == 1) put_restrict(sm);
+            }
+            tm_wait_st();
+        }
+        __syncthreads();
+        if (any_c) publish_coarse();
+        const int set2 = slot_set(ph);
+        phase(N2{}, false, [&](LocalInst& L, const double* q) { step_beta(bp, L, q, cfg); });
+        if (s_flag) {
+            ok = false;
+            break;
+        }
+        // the coarse part restarts from R^T r_new (no recurrence drift)
+        if (coarse) coarse_apply_dense<BLOCK>(bp, creg, set2, c_vbuf, s_cu);
+        if (coarse_b) {
+            coarse_apply_inst(bp, creg, li, nloc, set2, c_inst, kCU, kTileWarps, false);
+            __syncthreads();
+        }
+    }
+    // x with the last iteration's alpha p
+    for (int k = warp; k < ns; k += kTileWarps) {
+        const LocalInst& L = li[inst_of(k)];
+        const int i = (s0 + k) * 32 + lane;
+        float3 x, d = f3(0.f, 0.f, 0.f);
+        tm_ld3(tm(k) + kTmX, x);
+        tm_wait_ld(x, d);
+        if (L.iter > 0) {
+            const float3 p = ldp(k * 32 + lane);
+            x = f3(fmaf(L.alpha, p.x, x.x), fmaf(L.alpha, p.y, x.y), fmaf(L.alpha, p.z, x.z));
+        }
+        if (i < t.n) v.x[i] = f4(x);
+    }
+    if (!ok) instances_fail(bp, li, nloc);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s_tmem), "r"(T.tmem_cols) : "memory");
+}
+
+}  // namespace chysx_b200

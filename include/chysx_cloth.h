@@ -368,19 +368,22 @@ int chysx_cloth_instance_stats(chysx_cloth* h, int n, int* iterations, double* r
 
 /* Solver kernel selection (no counterpart in the reference, whose PCG is a
  * fixed chain of 8 launches per iteration, src/solver/pcg_solver.cu:542-592):
- * solver_path 0 = one persistent cooperative kernel per solve, with rows held
- * in registers when the system fits (default), 1 = CUDA-graph WHILE loop of
- * two kernels per iteration, 2 = the streamed persistent kernel forced.
- * block (0, 128, 256, 512) and grid (0 = automatic) size the streamed
- * persistent kernel; block 0 lets the planner choose (64-thread CTAs, a
- * build of its own, for batches that get the coarse level, whose blocks are
- * the instances' CTA segments; else 256). */
+ * solver_path 0 = one persistent kernel per solve, with rows held in
+ * registers when the system fits, else with the solver vectors on the SMs and
+ * the matrix streamed when those fit (default), 1 = CUDA-graph WHILE loop of
+ * two kernels per iteration, 2 = the streamed persistent kernel (vectors
+ * streamed too) forced.  block (0, 128, 256, 512) and grid (0 = automatic)
+ * size that kernel; block 0 lets the planner choose (1024 threads where the
+ * vectors stay on the SMs; else 64-thread CTAs, a build of its own, for
+ * batches that get the coarse level, whose blocks are the instances' CTA
+ * segments; else 256). */
 int chysx_cloth_set_tuning(chysx_cloth* h, int solver_path, int block, int grid);
 /* Synchronisation of the persistent PCG kernels (no counterpart in the
  * reference): 0 = one grid-wide counter barrier per reduction (default),
  * 1 = polled per-instance reduction slots, in which each instance waits only
  * for the CTAs holding its rows and the reduction read is the wait itself.
- * Both sum the same partials in the same order: identical iterates. */
+ * Both sum the same partials in the same order: identical iterates, except
+ * where mode 0 keeps the solver vectors on the SMs and mode 1 streams them. */
 int chysx_cloth_set_sync_mode(chysx_cloth* h, int mode);
 
 /* Autotuner (no counterpart in the reference).  Times, on the current state,
