@@ -1415,6 +1415,10 @@ private:
                        : reinterpret_cast<const void*>(&pcg_resident_kernel<8, kResidentMaxWidth, SYNC>);
         }
         if (tiled_) {
+            if (tile_mode_ == 2)
+                return cluster_ ? reinterpret_cast<const void*>(&pcg_tiled_kernel<true, 0, 2, true>)
+                                : reinterpret_cast<const void*>(&pcg_tiled_kernel<true, 0, 2, false>);
+            if (tile_mode_ == 1) return reinterpret_cast<const void*>(&pcg_tiled_kernel<true, 0, 1>);
             if (plan_.n_inst == 1)
                 return coarse_on_ ? reinterpret_cast<const void*>(&pcg_tiled_kernel<true, 1>)
                                   : reinterpret_cast<const void*>(&pcg_tiled_kernel<true, 0>);
@@ -1527,12 +1531,18 @@ private:
         const void* fn = persistent_fn();
         ck(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pers_smem_),
            "cudaFuncSetAttribute(cluster smem)");
+        cluster_ = cluster_fits(ctas, 512);  // else the grid-barrier build
+        return cluster_;
+    }
+    // whether the device can run the selected kernel as one cluster of `ctas`
+    bool cluster_fits(int ctas, int threads) const {
+        const void* fn = persistent_fn();
         if (ctas > 8)
             ck(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
                "cudaFuncSetAttribute(cluster size)");
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(ctas);
-        cfg.blockDim = dim3(512);
+        cfg.blockDim = dim3(threads);
         cfg.dynamicSmemBytes = pers_smem_;
         cudaLaunchAttribute attr{};
         attr.id = cudaLaunchAttributeClusterDimension;
@@ -1542,11 +1552,8 @@ private:
         cfg.numAttrs = 1;
         int fit = 0;
         const cudaError_t e = cudaOccupancyMaxActiveClusters(&fit, fn, &cfg);
-        if (e != cudaSuccess || fit < 1) {
-            cudaGetLastError();  // no room for the cluster on this device: the grid-barrier build
-            cluster_ = false;
-        }
-        return cluster_;
+        if (e != cudaSuccess) cudaGetLastError();
+        return e == cudaSuccess && fit >= 1;
     }
 
     // Coarse level of the two-level preconditioner (kind 2) of a
@@ -1799,12 +1806,34 @@ private:
     // block or grid request, synchronisation mode 1, general 3x3 blocks
     // (bending) and the contact operator keep the streamed kernel.
     bool plan_tiled(int sms) {
-        tiled_ = false;
         if (solver_path_ != kPathPersistent || pcg_block_req_ != 0 || pcg_grid_req_ != 0 || sync_mode_ != 0 ||
-            use_bending_ || co_active_)
+            co_active_)
             return false;
-        build_plan(topo_.inst_slice, std::min(sms, std::max(1, topo_.n_slices)), plan_);
+        const int ns = std::max(1, topo_.n_slices);
+        const bool one = topo_.inst_slice.size() <= 2, plain = one && pc_kind_ == 0;
+        // the matrix in shared memory: as one cluster (sixteen CTAs, or the
+        // eight of the portable size), else on every SM; else streamed
+        if (plain)
+            for (int ctas : {16, 8})
+                if (plan_tiled_with(std::min(ctas, ns), 2, true)) return true;
+        if (plain && plan_tiled_with(std::min(sms, ns), 2, false)) return true;
+        if (use_bending_) return plain && plan_tiled_with(std::min(sms, ns), 1, false);
+        return plan_tiled_with(std::min(sms, ns), 0, false);
+    }
+    bool plan_tiled_with(int ctas, int mode, bool cluster) {
+        tiled_ = cluster_ = false;
+        tile_mode_ = mode;
+        build_plan(topo_.inst_slice, ctas, plan_);
         if (plan_.max_slices_per_cta > kTileMaxSlices) return false;
+        int max_entries = 0;
+        if (mode == 2) {
+            for (int c = 0; c < plan_.grid; ++c)
+                max_entries = std::max(max_entries, topo_.slice_off[plan_.cta_slice[c + 1]] -
+                                                        topo_.slice_off[plan_.cta_slice[c]]);
+            max_entries = std::max(max_entries, 1);
+            // far above any SM's shared memory: no need to look for the halo
+            if ((size_t)max_entries * off_width() * sizeof(float) > ((size_t)1 << 18)) return false;
+        }
         // 16-bit columns: the CTA's own rows, then its halo in order of first use
         const int grid = plan_.grid;
         std::vector<unsigned short> lcol(std::max<size_t>(1, topo_.col.size())), halo_li;
@@ -1834,24 +1863,29 @@ private:
             max_halo = std::max(max_halo, halo_off[c + 1] - halo_off[c]);
         }
         tiled_ = true;
+        cluster_ = cluster;
         int cols = 32;
         while (cols < kTileCols * ((plan_.max_slices_per_cta + 3) / 4)) cols *= 2;
         int dev = 0, limit = 0;
         ck(cudaGetDevice(&dev), "cudaGetDevice");
         ck(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "cudaDeviceGetAttribute");
         plan_coarse();
+        const int ow = mode == 2 ? off_width() : 0;
         pers_smem_ = tile_smem(plan_.n_inst == 1 ? kTileWarps : plan_.max_slices_per_cta, plan_.max_inst_per_cta,
-                               coarse_stream_smem(), plan_.max_slices_per_cta, max_halo).bytes;
+                               coarse_stream_smem(), plan_.max_slices_per_cta, max_halo, max_entries, ow).bytes;
         cudaFuncAttributes fa{};
         ck(cudaFuncGetAttributes(&fa, persistent_fn()), "cudaFuncGetAttributes(tiled)");
-        if (pers_smem_ + fa.sharedSizeBytes > (size_t)limit) {
-            tiled_ = false;
+        bool fits = pers_smem_ + fa.sharedSizeBytes <= (size_t)limit;
+        if (fits)
+            ck(cudaFuncSetAttribute(persistent_fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pers_smem_),
+               "cudaFuncSetAttribute(tiled smem)");
+        if (fits && cluster) fits = cluster_fits(plan_.grid, kTileThreads);
+        if (!fits) {
+            tiled_ = cluster_ = false;
             coarse_on_ = false;
             coarse_batched_ = false;
             return false;
         }
-        ck(cudaFuncSetAttribute(persistent_fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pers_smem_),
-           "cudaFuncSetAttribute(tiled smem)");
         d_tile_lcol_.upload(lcol);
         d_tile_hoff_.upload(halo_off);
         d_tile_hrow_.upload(halo_row.empty() ? std::vector<int>{0} : halo_row);
@@ -1866,6 +1900,8 @@ private:
         ta.tmem_cols = cols;
         ta.max_slices = plan_.max_slices_per_cta;
         ta.max_halo = max_halo;
+        ta.max_entries = max_entries;
+        ta.ow = ow;
         d_tile_.upload(&ta, 1);
         return true;
     }
@@ -2457,6 +2493,7 @@ private:
     std::vector<int> order_;  // particles in row order (row_order_ 1)
     bool resident_ = false;
     bool tiled_ = false;    // the tiled kernel (streamed matrix, vectors on the SM)
+    int tile_mode_ = 0;     // its MODE
     DevBuf<unsigned short> d_tile_lcol_, d_tile_hli_;
     DevBuf<int> d_tile_hoff_, d_tile_hrow_;
     DevBuf<unsigned> d_tile_mask_;

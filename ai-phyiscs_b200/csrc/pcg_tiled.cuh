@@ -25,9 +25,16 @@
 //
 // Phases, per-instance logic, preconditioner (block-Jacobi, or with a coarse
 // level: CO = 1 dense, CO = 2 batched) and stopping rules are those of
-// pcg_persistent_kernel; symmetric blocks only, synchronisation by the
-// counter barrier.  ONE: a single instance, whose per-row sums are kept per
-// thread and added once per phase.
+// pcg_persistent_kernel, synchronisation by the counter barrier.  ONE: a
+// single instance, whose per-row sums are kept per thread and added once per
+// phase.  MODE 0 streams symmetric blocks, 1 general ones (bending); MODE 2
+// first copies the CTA's blocks of either kind, their columns, D' and M^-1
+// into shared memory, for systems whose rows are too wide for registers but
+// whose matrix fits the SMs: their iteration is latency, not bytes.  CLU
+// (MODE 2): the grid is one thread-block cluster, whose barrier and shared
+// memory carry the reductions, as in the resident kernel's cluster build.
+// A 61 x 47 garment with bending (18 neighbours a row, 16 CTAs): 11.9 us per
+// iteration streamed, 5.0 as a cluster.
 #pragma once
 
 #include "pcg_persistent.cuh"
@@ -48,16 +55,18 @@ struct TileArgs {
     int tmem_cols;                    // columns allocated (power of two >= 32)
     int max_slices;                   // per CTA
     int max_halo;
+    int max_entries;                  // ELL entries of a CTA (MODE 2; else 0)
+    int ow;                           // floats per block (MODE 2)
 };
 
 // Dynamic shared memory: slice partials, instance records, coarse values,
 // slice offsets / masks / instances, halo rows and instances, p.
 __host__ __device__ inline size_t tile_align(size_t v) { return (v + 15) & ~static_cast<size_t>(15); }
 struct TileSmem {
-    size_t li, vbuf, soff, mask, sli, hrow, hli, p, bytes;
+    size_t li, vbuf, soff, mask, sli, hrow, hli, p, mat, diag, col, bytes;
 };
 __host__ __device__ inline TileSmem tile_smem(int parts, int max_inst, size_t coarse_bytes, int max_slices,
-                                              int max_halo) {
+                                              int max_halo, int max_entries = 0, int ow = 0) {
     TileSmem s;
     s.li = (size_t)parts * kSlotW * sizeof(double);
     s.vbuf = tile_align(s.li + (size_t)max_inst * sizeof(LocalInst));
@@ -67,7 +76,11 @@ __host__ __device__ inline TileSmem tile_smem(int parts, int max_inst, size_t co
     s.hrow = tile_align(s.sli + (size_t)max_slices * sizeof(unsigned short));
     s.hli = s.hrow + (size_t)max_halo * sizeof(int);
     s.p = tile_align(s.hli + (size_t)max_halo * sizeof(unsigned short));
-    s.bytes = s.p + (size_t)3 * (32 * (size_t)max_slices + max_halo) * sizeof(float);
+    s.mat = tile_align(s.p + (size_t)3 * (32 * (size_t)max_slices + max_halo) * sizeof(float));
+    // MODE 2: blocks, D' and M^-1 (192 floats each per slice), columns
+    s.diag = s.mat + (size_t)max_entries * ow * sizeof(float);
+    s.col = s.diag + (max_entries ? (size_t)384 * max_slices * sizeof(float) : 0);
+    s.bytes = s.col + (size_t)max_entries * sizeof(unsigned short);
     return s;
 }
 
@@ -146,7 +159,7 @@ __device__ __forceinline__ int ld_na(const unsigned short* p) {
     return v;
 }
 
-template <bool ONE, int CO>
+template <bool ONE, int CO, int MODE = 0, bool CLU = false>
 __global__ void __launch_bounds__(kTileThreads, 1)
 pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const TileArgs* ta, void*) {
     constexpr int SYNC = 0;  // slot_set: two sets by parity
@@ -171,7 +184,8 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
     const size_t cbytes = CO == 1 ? (bp.cg ? (size_t)bp.cg->m * sizeof(float) + 16 : 0)
                                   : (CO == 2 ? (size_t)bp.max_inst_per_cta * kInstCoarseW * sizeof(float) + 16 : 0);
     const TileSmem lay = tile_smem(ONE ? kTileWarps : T.max_slices, bp.max_inst_per_cta, cbytes, T.max_slices,
-                                   T.max_halo);
+                                   T.max_halo, T.max_entries, T.ow);
+    __shared__ double s_cslot[CLU ? 2 : 1][kClusterMax][CLU ? kSlotW : 1];
     double* spart = reinterpret_cast<double*>(s_raw);
     LocalInst* li = reinterpret_cast<LocalInst*>(s_raw + lay.li);
     float* c_vbuf = reinterpret_cast<float*>(s_raw + lay.vbuf);
@@ -182,6 +196,9 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
     int* s_hrow = reinterpret_cast<int*>(s_raw + lay.hrow);
     unsigned short* s_hli = reinterpret_cast<unsigned short*>(s_raw + lay.hli);
     float* s_p = reinterpret_cast<float*>(s_raw + lay.p);
+    float* s_mat = reinterpret_cast<float*>(s_raw + lay.mat);
+    float* s_diag = reinterpret_cast<float*>(s_raw + lay.diag);
+    unsigned short* s_col = reinterpret_cast<unsigned short*>(s_raw + lay.col);
     unsigned target = 0;
     int ph = 0;
     if (warp == 0) {
@@ -206,7 +223,20 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
         s_hrow[h] = T.halo_row[h0 + h];
         s_hli[h] = ONE ? 0 : T.halo_li[h0 + h];
     }
+    if (MODE == 2) {
+        const int e0 = t.slice_off[s0], ne = t.slice_off[s1] - e0;
+        const float4* src = reinterpret_cast<const float4*>(t.val + (size_t)e0 * T.ow);
+        for (int x = tid; x < ne * T.ow / 4; x += BLOCK) reinterpret_cast<float4*>(s_mat)[x] = src[x];
+        const float4* d = reinterpret_cast<const float4*>(t.dnl + (size_t)s0 * 192);
+        const float4* mi = reinterpret_cast<const float4*>(t.minv + (size_t)s0 * 192);
+        for (int x = tid; x < ns * 48; x += BLOCK) {
+            reinterpret_cast<float4*>(s_diag)[x] = d[x];
+            reinterpret_cast<float4*>(s_diag)[ns * 48 + x] = mi[x];
+        }
+        for (int x = tid; x < ne; x += BLOCK) s_col[x] = T.lcol[e0 + x];
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (CLU) cluster_sync_all();  // the other CTAs' shared memory is live before any store into it
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (ONE && tid == 0) {  // the partials are per warp
@@ -251,60 +281,64 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
     auto phase = [&](auto nv, bool exit_test, auto&& step) {
         constexpr int NV = decltype(nv)::value;
         const int set = slot_set(ph);
-        for (int q = warp; q < nloc; q += kTileWarps) {
-            const LocalInst& L = li[q];
-            if (L.done) continue;
-            double acc[NV];
-#pragma unroll
-            for (int u = 0; u < NV; ++u) acc[u] = 0.0;
-            for (int sl = L.seg_lo + lane; sl < L.seg_hi; sl += 32) {
-#pragma unroll
-                for (int u = 0; u < NV; ++u) acc[u] += spart[sl * kSlotW + u];
-            }
-#pragma unroll
-            for (int u = 0; u < NV; ++u) {
-                acc[u] = warp_sum(acc[u]);
-                if (lane == 0) bp.slots[((size_t)set * bp.n_slots + L.own_slot) * kSlotW + u] = acc[u];
-            }
-        }
-        __syncthreads();
-        if (tid == 0) {
-            if (!barrier_arrive_wait(bp.bar, target)) s_flag = 1;
-            else if (exit_test) s_exit = *(volatile unsigned*)&bp.bar->ndone >= (unsigned)bp.n_inst;
-        }
-        __syncthreads();
-        if (!s_flag) {
+        if constexpr (CLU) {
+            cluster_phase<NV>(spart, li, 1, s_cslot, set, step);
+        } else {
             for (int q = warp; q < nloc; q += kTileWarps) {
-                LocalInst& L = li[q];
+                const LocalInst& L = li[q];
                 if (L.done) continue;
-                constexpr int KP = 5;  // one pass covers 160 CTAs
-                double tot[NV];
+                double acc[NV];
 #pragma unroll
-                for (int u = 0; u < NV; ++u) tot[u] = 0.0;
-                for (int c0 = L.slot_lo; c0 < L.slot_hi; c0 += 32 * KP) {
-                    constexpr int NP = NV > 2 ? 2 : NV;  // values in flight together (registers)
+                for (int u = 0; u < NV; ++u) acc[u] = 0.0;
+                for (int sl = L.seg_lo + lane; sl < L.seg_hi; sl += 32) {
 #pragma unroll
-                    for (int u0 = 0; u0 < NV; u0 += NP) {
-                        double val[KP][NP];
-#pragma unroll
-                        for (int j = 0; j < KP; ++j)
-#pragma unroll
-                            for (int u = 0; u < NP; ++u) {
-                                const int k = c0 + j * 32 + lane;
-                                val[j][u] = k < L.slot_hi
-                                                ? __ldcg(bp.slots + ((size_t)set * bp.n_slots + k) * kSlotW + u0 + u)
-                                                : 0.0;
-                            }
-#pragma unroll
-                        for (int j = 0; j < KP; ++j)
-#pragma unroll
-                            for (int u = 0; u < NP; ++u) tot[u0 + u] += val[j][u];
-                    }
+                    for (int u = 0; u < NV; ++u) acc[u] += spart[sl * kSlotW + u];
                 }
 #pragma unroll
-                for (int u = 0; u < NV; ++u) tot[u] = warp_sum(tot[u]);
-                if (lane == 0) step(L, tot);
-                __syncwarp();
+                for (int u = 0; u < NV; ++u) {
+                    acc[u] = warp_sum(acc[u]);
+                    if (lane == 0) bp.slots[((size_t)set * bp.n_slots + L.own_slot) * kSlotW + u] = acc[u];
+                }
+            }
+            __syncthreads();
+            if (tid == 0) {
+                if (!barrier_arrive_wait(bp.bar, target)) s_flag = 1;
+                else if (exit_test) s_exit = *(volatile unsigned*)&bp.bar->ndone >= (unsigned)bp.n_inst;
+            }
+            __syncthreads();
+            if (!s_flag) {
+                for (int q = warp; q < nloc; q += kTileWarps) {
+                    LocalInst& L = li[q];
+                    if (L.done) continue;
+                    constexpr int KP = 5;  // one pass covers 160 CTAs
+                    double tot[NV];
+#pragma unroll
+                    for (int u = 0; u < NV; ++u) tot[u] = 0.0;
+                    for (int c0 = L.slot_lo; c0 < L.slot_hi; c0 += 32 * KP) {
+                        constexpr int NP = NV > 2 ? 2 : NV;  // values in flight together (registers)
+#pragma unroll
+                        for (int u0 = 0; u0 < NV; u0 += NP) {
+                            double val[KP][NP];
+#pragma unroll
+                            for (int j = 0; j < KP; ++j)
+#pragma unroll
+                                for (int u = 0; u < NP; ++u) {
+                                    const int k = c0 + j * 32 + lane;
+                                    val[j][u] = k < L.slot_hi
+                                                    ? __ldcg(bp.slots + ((size_t)set * bp.n_slots + k) * kSlotW + u0 + u)
+                                                    : 0.0;
+                                }
+#pragma unroll
+                            for (int j = 0; j < KP; ++j)
+#pragma unroll
+                                for (int u = 0; u < NP; ++u) tot[u0 + u] += val[j][u];
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < NV; ++u) tot[u] = warp_sum(tot[u]);
+                    if (lane == 0) step(L, tot);
+                    __syncwarp();
+                }
             }
         }
         ++ph;
@@ -332,10 +366,31 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
     auto row_product = [&](int k, float3 pi) {
         const int s = s0 + k;
         const int so = s_off[k], w = (s_off[k + 1] - so) >> 5;
-        const float* vb = t.val + (size_t)so * 6 + lane;
-        const unsigned short* lc = T.lcol + so + lane;
         float3 acc = f3(0.f, 0.f, 0.f);
+        if constexpr (MODE == 2) {
+            const int sl = so - s_off[0];
+            const float* vb = s_mat + (size_t)sl * T.ow + lane;
+            const unsigned short* lc = s_col + sl + lane;
+            if (s * 32 + lane < t.n) acc = mul(ld6(s_diag + k * 192 + lane), pi);
+            const int nsym = T.ow == 9;
+#pragma unroll 2
+            for (int e = 0; e < w; ++e) acc = acc + mul_off(vb + e * T.ow * 32, nsym, ldp(lc[e * 32]) - pi);
+            return acc;
+        }
+        const unsigned short* lc = T.lcol + so + lane;
         if (s * 32 + lane < t.n) acc = mul(ld6_na(t.dnl + (size_t)s * 192 + lane), pi);
+        if constexpr (MODE == 1) {
+            const float* vb = t.val + (size_t)so * 9 + lane;
+            for (int e = 0; e < w; ++e) {
+                const float* q = vb + e * 288;
+                const float3 d = ldp(ld_na(lc + e * 32)) - pi;
+                acc = acc + f3(ld_na(q) * d.x + ld_na(q + 32) * d.y + ld_na(q + 64) * d.z,
+                               ld_na(q + 96) * d.x + ld_na(q + 128) * d.y + ld_na(q + 160) * d.z,
+                               ld_na(q + 192) * d.x + ld_na(q + 224) * d.y + ld_na(q + 256) * d.z);
+            }
+            return acc;
+        }
+        const float* vb = t.val + (size_t)so * 6 + lane;
         if (w == 6) {
 #pragma unroll
             for (int e = 0; e < 6; ++e) acc = acc + mul(ld6_na(vb + e * 192), ldp(ld_na(lc + e * 32)) - pi);
@@ -389,7 +444,8 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
     auto load_b = [&](int, int i) { return i < t.n ? xyz(v.b[i]) : f3(0.f, 0.f, 0.f); };
     auto load_minv = [&](int s, int i) {
         S6 m{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (i < t.n) m = ld6_na(t.minv + (size_t)s * 192 + lane);
+        if (i < t.n)
+            m = MODE == 2 ? ld6(s_diag + (ns + s - s0) * 192 + lane) : ld6_na(t.minv + (size_t)s * 192 + lane);
         return m;
     };
     auto publish_z = [&](int k, int i, float3 z) {

@@ -130,8 +130,8 @@ int chysx_cloth_build_fem_shear(chysx_cloth* h, float stiffness, const float* k_
  * interior edge of the (consistently oriented) mesh, rest angles from the
  * current positions, stiffness k for all (constraint/cloth/
  * bending_constraint.h).  Its Hessian blocks are not symmetric, so a step
- * with bending stores full 3x3 off-diagonal blocks and runs the streamed or
- * graph-loop PCG kernel. */
+ * with bending stores full 3x3 off-diagonal blocks, and no kernel holds its
+ * rows in registers (chysx_cloth_solver_info path 1 or 2). */
 int chysx_cloth_build_bending(chysx_cloth* h, float stiffness, uintptr_t stream);
 int chysx_cloth_num_dihedrals(const chysx_cloth* h, int* out);
 

@@ -106,3 +106,32 @@ def test_two_level_converges_to_the_streamed_solution():
     assert a.stats()[2] == capi.SOLVE_CONVERGED and a.stats()[1] <= 1e-6
     assert a.stats()[0] < 1.5 * b.stats()[0]
     assert np.abs(a.positions() - b.positions()).max() < 1e-5
+
+
+# general 3x3 blocks (bending) and the matrix in shared memory: one cluster (3 and 16 CTAs), every SM, and above
+# what fits the SMs (230 x 230) streamed; the last slices are ragged
+@pytest.mark.parametrize("w,h", [(9, 9), (61, 47), (91, 90), (231, 230)])
+def test_bending_systems(w, h):
+    sc = _rect(w, h)
+    sc["k_bend"], sc["k_shear"] = 5.0e-3, 5.0e3
+    a, b = _run(sc, 0), _run(sc, 2)
+    assert a.sim.solver_info()[0] == b.sim.solver_info()[0] == "streamed"
+    assert a.sim.solver_info()[2] == 1024
+    assert (a.sim.solver_info()[1] <= 16) == (w * h < 4000)
+    assert np.abs(a.positions() - b.positions()).max() < 5e-7
+
+
+@pytest.mark.parametrize("warm", ["previous", "previous_scaled"])
+@pytest.mark.parametrize("w,h", [(30, 31), (91, 90)])
+def test_bending_warm_starts_and_stops(w, h, warm):
+    sc = _rect(w, h)
+    sc["k_bend"] = 5.0e-3
+    a, b = (_run(sc, p, warm, steps=2) for p in (0, 2))
+    assert np.abs(a.positions() - b.positions()).max() < 2e-6  # as test_warm_starts
+    for n in (3, 0):  # other limits on the same graph
+        a.sim.set_solver(n, 0.0, warm)
+        a.step()
+        assert a.stats()[0] == n and a.stats()[2] == capi.SOLVE_CONVERGED
+    a.sim.set_solver(20000, 1e-6, "zero")
+    a.step()
+    assert a.stats()[2] == capi.SOLVE_CONVERGED and a.stats()[1] <= 1e-6
