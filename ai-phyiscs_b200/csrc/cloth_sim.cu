@@ -1655,6 +1655,10 @@ private:
         coarse_on_ = false;
         coarse_batched_ = false;
         if (pc_kind_ != 2 || sync_mode_ != 0) return;
+        if (tiled_) {
+            plan_coarse_tiled();
+            return;
+        }
         if (plan_.n_inst != 1) {
             // several instances on the streamed kernel, zero-guess solves:
             // one coarse block per instance
@@ -1718,12 +1722,18 @@ private:
             }
         for (int B = 0; B < nb; ++B)
             for (int sl = row0[B] / 32; sl < row0[B + 1] / 32; ++sl) slice_cb[sl] = B;
+        d_blk_slot_.upload(blk_slot);
+        d_slot_cb_.upload(slot_cb);
+        return finish_batched(slice_cb, row0, nb, nq, inst_blk, inst_aoff, mmax);
+    }
+    // the buffers of a block-diagonal coarse level (blocks inside instances)
+    bool finish_batched(const std::vector<int>& slice_cb, const std::vector<int>& row0, int nb, int nq,
+                        const std::vector<int>& inst_blk, const std::vector<int>& inst_aoff, int mmax) {
+        const int U = 3 * nq, ni = plan_.n_inst;
         int mn = 0;
         if (!coarse_neighbours(slice_cb, row0, nb, mn)) return false;
-        d_blk_slot_.upload(blk_slot);
         d_inst_blk_.upload(inst_blk);
         d_inst_aoff_.upload(inst_aoff);
-        d_slot_cb_.upload(slot_cb);
         d_cw_.resize((size_t)std::max(1, row0[nb]));
         d_cw_.zero();
         d_cac_.resize((size_t)nb * mn * U * U);
@@ -1757,11 +1767,79 @@ private:
            "cudaFuncSetAttribute(batched coarse inverse smem)");
         return true;
     }
+    // The tiled kernel's coarse blocks (kTileBlockRows): per CTA, or inside the
+    // instances of a batch (zero-guess solves).
+    void plan_coarse_tiled() {
+        const int grid = plan_.grid, ns = topo_.n_slices, ni = plan_.n_inst;
+        std::vector<int> cta_blk(grid + 1, 0), blk_row0{0}, blk_inst;
+        if (ni == 1) {
+            const int rows_per_cta = std::max(1, 32 * ns / std::max(1, grid));
+            const int G = std::max(1, (kTileBlockRows + rows_per_cta / 2) / rows_per_cta);
+            if ((grid + G - 1) / G < 2 || !plan_coarse_with(G, 4, kCoarseShift)) return;
+            for (int c = 0; c <= grid; ++c) cta_blk[c] = c;
+            blk_row0.assign(grid + 1, 0);
+            for (int c = 0; c <= grid; ++c) blk_row0[c] = plan_.cta_slice[c] * 32;
+            blk_inst.assign(grid, 0);
+        } else {
+            if (warm_mode_ != CHYSX_WARM_ZERO) return;
+            // per instance: blocks of t slices or more in every segment (its
+            // slices in one CTA), t the least that keeps kBatchMaxBlocks
+            std::vector<int> inst_blk(ni + 1, 0), inst_aoff(ni + 1, 0), slice_cb(std::max(1, ns), 0);
+            int mmax = 12;
+            blk_row0.clear();
+            for (int b = 0; b < ni; ++b) {
+                const int lo = plan_.inst_slice[b], hi = plan_.inst_slice[b + 1];
+                const int c0 = plan_.inst_cta_lo[b], nc = plan_.inst_slot[b + 1] - plan_.inst_slot[b];
+                auto seg = [&](int c, int& a, int& z) {
+                    a = std::max(lo, plan_.cta_slice[c]);
+                    z = std::min(hi, plan_.cta_slice[c + 1]);
+                };
+                if (nc > kBatchMaxBlocks) return;  // an instance across more CTAs than blocks
+                int t = std::max(kTileBatchSlices, (hi - lo + kBatchMaxBlocks - 1) / kBatchMaxBlocks);
+                for (;; ++t) {
+                    int total = 0;
+                    for (int c = c0; c < c0 + nc; ++c) {
+                        int a, z;
+                        seg(c, a, z);
+                        total += std::max(1, (z - a + t / 2) / t);
+                    }
+                    if (total <= kBatchMaxBlocks) break;
+                }
+                for (int c = c0; c < c0 + nc; ++c) {
+                    int a, z;
+                    seg(c, a, z);
+                    const int n = std::max(1, (z - a + t / 2) / t);
+                    for (int q = 0; q < n; ++q) {
+                        const int k0 = a + (int)((long long)(z - a) * q / n), k1 = a + (int)((long long)(z - a) * (q + 1) / n);
+                        for (int k = k0; k < k1; ++k) slice_cb[k] = (int)blk_inst.size();
+                        blk_row0.push_back(k0 * 32);
+                        blk_inst.push_back(b);
+                        cta_blk[c + 1] = (int)blk_inst.size();
+                    }
+                }
+                inst_blk[b + 1] = (int)blk_inst.size();
+                const int m = 12 * (inst_blk[b + 1] - inst_blk[b]);
+                mmax = std::max(mmax, m);
+                inst_aoff[b + 1] = inst_aoff[b] + m * m;
+            }
+            blk_row0.push_back(ns * 32);
+            if (!finish_batched(slice_cb, blk_row0, (int)blk_inst.size(), 4, inst_blk, inst_aoff, mmax)) return;
+        }
+        tile_max_blk_ = 1;
+        for (int c = 0; c < grid; ++c) tile_max_blk_ = std::max(tile_max_blk_, cta_blk[c + 1] - cta_blk[c]);
+        d_cta_blk_.upload(cta_blk);
+        d_blk_row0_.upload(blk_row0);
+        d_blk_inst_.upload(blk_inst);
+        d_cvals_.resize((size_t)2 * 12 * blk_inst.size());
+        d_cvals_.zero();
+        const CoarseArgs cargs = coarse_args();
+        d_cargs_.upload(&cargs, 1);
+    }
     // the streamed kernel's shared memory for its coarse level: the block
     // values (dense level) or the per-instance values (batched level)
     size_t coarse_stream_smem() const {
         if (!coarse_on_) return 0;
-        if (coarse_batched_) return (size_t)plan_.max_inst_per_cta * kInstCoarseW * sizeof(float) + 16;
+        if (coarse_batched_) return tiled_ ? 0 : (size_t)plan_.max_inst_per_cta * kInstCoarseW * sizeof(float) + 16;
         return (size_t)3 * coarse_nq_ * coarse_nb_ * sizeof(float) + 16;
     }
     // per-lane partial sums of the coarse assembly: [nq][9][max_nbr][32] floats
@@ -1789,10 +1867,14 @@ private:
         c.ainv = d_cainv_.get();
         c.dense = resident_ || coarse_batched_ ? 0 : 1;
         c.batched = coarse_batched_ ? 1 : 0;
-        c.blk_slot = coarse_batched_ ? d_blk_slot_.get() : nullptr;
+        c.blk_slot = coarse_batched_ && !tiled_ ? d_blk_slot_.get() : nullptr;
         c.inst_blk = coarse_batched_ ? d_inst_blk_.get() : nullptr;
         c.inst_aoff = coarse_batched_ ? d_inst_aoff_.get() : nullptr;
-        c.slot_cb = coarse_batched_ ? d_slot_cb_.get() : nullptr;
+        c.slot_cb = coarse_batched_ && !tiled_ ? d_slot_cb_.get() : nullptr;
+        c.cta_blk = tiled_ ? d_cta_blk_.get() : nullptr;
+        c.blk_row0 = tiled_ ? d_blk_row0_.get() : nullptr;
+        c.blk_inst = tiled_ ? d_blk_inst_.get() : nullptr;
+        c.cvals = tiled_ ? d_cvals_.get() : nullptr;
         c.shift = coarse_shift_;
         c.work = d_cwork_.get();
         c.fail = d_cfail_.get();
@@ -1818,7 +1900,18 @@ private:
                 if (plan_tiled_with(std::min(ctas, ns), 2, true)) return true;
         if (plain && plan_tiled_with(std::min(sms, ns), 2, false)) return true;
         if (use_bending_) return plain && plan_tiled_with(std::min(sms, ns), 1, false);
-        return plan_tiled_with(std::min(sms, ns), 0, false);
+        int ctas = std::min(sms, ns);
+        if (!one && pc_kind_ == 2 && warm_mode_ == CHYSX_WARM_ZERO) {
+            // the coarse level wants every instance inside kBatchMaxBlocks
+            // CTAs: fewer, fuller CTAs for a few large instances
+            int largest = 1;
+            for (size_t b = 0; b + 1 < topo_.inst_slice.size(); ++b)
+                largest = std::max(largest, topo_.inst_slice[b + 1] - topo_.inst_slice[b]);
+            const int per = (largest + kBatchMaxBlocks - 2) / (kBatchMaxBlocks - 1);  // one CTA more by its place
+            ctas = std::max(1, std::min(ctas, ns / std::max(1, per)));
+            if (ns > ctas * kTileMaxSlices) return false;  // the streamed kernel keeps the level
+        }
+        return plan_tiled_with(ctas, 0, false);
     }
     bool plan_tiled_with(int ctas, int mode, bool cluster) {
         tiled_ = cluster_ = false;
@@ -1871,8 +1964,10 @@ private:
         ck(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "cudaDeviceGetAttribute");
         plan_coarse();
         const int ow = mode == 2 ? off_width() : 0;
+        if (!coarse_on_) tile_max_blk_ = 1;
         pers_smem_ = tile_smem(plan_.n_inst == 1 ? kTileWarps : plan_.max_slices_per_cta, plan_.max_inst_per_cta,
-                               coarse_stream_smem(), plan_.max_slices_per_cta, max_halo, max_entries, ow).bytes;
+                               coarse_stream_smem(), tile_max_blk_, plan_.max_slices_per_cta, max_halo, max_entries,
+                               ow).bytes;
         cudaFuncAttributes fa{};
         ck(cudaFuncGetAttributes(&fa, persistent_fn()), "cudaFuncGetAttributes(tiled)");
         bool fits = pers_smem_ + fa.sharedSizeBytes <= (size_t)limit;
@@ -1902,6 +1997,7 @@ private:
         ta.max_halo = max_halo;
         ta.max_entries = max_entries;
         ta.ow = ow;
+        ta.max_blk = tile_max_blk_;
         d_tile_.upload(&ta, 1);
         return true;
     }
@@ -2494,6 +2590,9 @@ private:
     bool resident_ = false;
     bool tiled_ = false;    // the tiled kernel (streamed matrix, vectors on the SM)
     int tile_mode_ = 0;     // its MODE
+    int tile_max_blk_ = 1;  // coarse blocks of one of its CTAs
+    DevBuf<int> d_cta_blk_, d_blk_row0_, d_blk_inst_;
+    DevBuf<float> d_cvals_;
     DevBuf<unsigned short> d_tile_lcol_, d_tile_hli_;
     DevBuf<int> d_tile_hoff_, d_tile_hrow_;
     DevBuf<unsigned> d_tile_mask_;

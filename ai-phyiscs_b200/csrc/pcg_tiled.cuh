@@ -11,7 +11,7 @@
 //     into it, so a gather is a shared-memory read;
 //   * x, r and A p (then z in the same place) lie in tensor memory, used as
 //     plain storage: 9 columns of one warp's 32 lanes per 32-row slice, 512
-//     columns, i.e. up to 224 slices (7,168 rows) per SM;
+//     columns, i.e. 7 slices per warp and up to 224 (7,168 rows) per SM;
 //   * x takes alpha p one iteration later, when p is at hand anyway;
 //   * only z of rows in another CTA's halo goes through global memory: the
 //     owner writes it with the update, every CTA forms the halo's p = z +
@@ -44,7 +44,7 @@ namespace chysx_b200 {
 constexpr int kTileThreads = 1024;
 constexpr int kTileWarps = kTileThreads / 32;
 constexpr int kTileCols = 9;          // TMEM columns per slice: x, r, A p / z
-constexpr int kTileMaxSlices = 224;   // 4 lane quarters x 56 slices x 9 columns <= 512
+constexpr int kTileMaxSlices = 224;   // 7 per warp: 8 warps per lane quarter x 7 slices x 9 columns <= 512
 
 struct TileArgs {
     const unsigned short* lcol;       // [ELL entries] own row (< the CTA's rows) or rows + halo index
@@ -57,23 +57,29 @@ struct TileArgs {
     int max_halo;
     int max_entries;                  // ELL entries of a CTA (MODE 2; else 0)
     int ow;                           // floats per block (MODE 2)
+    int max_blk;                      // coarse blocks of a CTA
 };
+// Coarse values of one of the CTA's blocks, per phase and state: A_c^-1 R^T of
+// r (kCU), of the new r (kCN), of b and of r0 (start only).
+constexpr int kTileCoarseW = 48, kTcB = 24, kTc0 = 36;
+static_assert(kCU == 0 && kCN == 12 && kInstCoarseW == 24, "the first two are the batched level's");
 
 // Dynamic shared memory: slice partials, instance records, coarse values,
 // slice offsets / masks / instances, halo rows and instances, p.
 __host__ __device__ inline size_t tile_align(size_t v) { return (v + 15) & ~static_cast<size_t>(15); }
 struct TileSmem {
-    size_t li, vbuf, soff, mask, sli, hrow, hli, p, mat, diag, col, bytes;
+    size_t li, vbuf, blk, soff, mask, sli, hrow, hli, p, mat, diag, col, bytes;
 };
-__host__ __device__ inline TileSmem tile_smem(int parts, int max_inst, size_t coarse_bytes, int max_slices,
-                                              int max_halo, int max_entries = 0, int ow = 0) {
+__host__ __device__ inline TileSmem tile_smem(int parts, int max_inst, size_t coarse_bytes, int max_blk,
+                                              int max_slices, int max_halo, int max_entries = 0, int ow = 0) {
     TileSmem s;
     s.li = (size_t)parts * kSlotW * sizeof(double);
     s.vbuf = tile_align(s.li + (size_t)max_inst * sizeof(LocalInst));
-    s.soff = tile_align(s.vbuf + coarse_bytes);
+    s.blk = tile_align(s.vbuf + coarse_bytes);  // per block: values, first slice (+ 1), instance
+    s.soff = tile_align(s.blk + (size_t)max_blk * (kTileCoarseW + 2) * sizeof(float) + sizeof(int));
     s.mask = s.soff + (size_t)(max_slices + 1) * sizeof(int);
     s.sli = s.mask + (size_t)max_slices * sizeof(unsigned);
-    s.hrow = tile_align(s.sli + (size_t)max_slices * sizeof(unsigned short));
+    s.hrow = tile_align(s.sli + (size_t)max_slices * 2 * sizeof(unsigned short));  // instance, coarse block
     s.hli = s.hrow + (size_t)max_halo * sizeof(int);
     s.p = tile_align(s.hli + (size_t)max_halo * sizeof(unsigned short));
     s.mat = tile_align(s.p + (size_t)3 * (32 * (size_t)max_slices + max_halo) * sizeof(float));
@@ -168,8 +174,6 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
     __shared__ int s_flag, s_exit;
     __shared__ uint32_t s_tmem;
     __shared__ float s_tmp[CO ? BLOCK : 1];
-    __shared__ float s_cb[12], s_c0[12], s_cw[12], s_cu[12], s_cn[12];
-    __shared__ CoarseRegs creg;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int s0 = bp.cta_slice[blockIdx.x], s1 = bp.cta_slice[blockIdx.x + 1], ns = s1 - s0;
     const int il0 = bp.cta_inst_lo[blockIdx.x], il1 = bp.cta_inst_hi[blockIdx.x];
@@ -181,18 +185,20 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
     const bool coarse_b =
         CO == 2 && !warm && bp.cg != nullptr && bp.cg->on && bp.cg->batched && *(volatile int*)bp.cg->fail == 0;
     const bool any_c = coarse || coarse_b;
-    const size_t cbytes = CO == 1 ? (bp.cg ? (size_t)bp.cg->m * sizeof(float) + 16 : 0)
-                                  : (CO == 2 ? (size_t)bp.max_inst_per_cta * kInstCoarseW * sizeof(float) + 16 : 0);
-    const TileSmem lay = tile_smem(ONE ? kTileWarps : T.max_slices, bp.max_inst_per_cta, cbytes, T.max_slices,
-                                   T.max_halo, T.max_entries, T.ow);
+    const size_t cbytes = CO == 1 && bp.cg ? (size_t)bp.cg->m * sizeof(float) + 16 : 0;
+    const TileSmem lay = tile_smem(ONE ? kTileWarps : T.max_slices, bp.max_inst_per_cta, cbytes, T.max_blk,
+                                   T.max_slices, T.max_halo, T.max_entries, T.ow);
     __shared__ double s_cslot[CLU ? 2 : 1][kClusterMax][CLU ? kSlotW : 1];
     double* spart = reinterpret_cast<double*>(s_raw);
     LocalInst* li = reinterpret_cast<LocalInst*>(s_raw + lay.li);
     float* c_vbuf = reinterpret_cast<float*>(s_raw + lay.vbuf);
-    float* c_inst = c_vbuf;
+    float* c_blk = reinterpret_cast<float*>(s_raw + lay.blk);                  // [max_blk][kTileCoarseW]
+    int* s_bk0 = reinterpret_cast<int*>(c_blk + (size_t)T.max_blk * kTileCoarseW);  // first slice of every block
+    int* s_binst = s_bk0 + T.max_blk + 1;                                      // its instance, relative
     int* s_off = reinterpret_cast<int*>(s_raw + lay.soff);
     unsigned* s_mask = reinterpret_cast<unsigned*>(s_raw + lay.mask);
     unsigned short* s_sli = reinterpret_cast<unsigned short*>(s_raw + lay.sli);
+    unsigned short* s_slb = s_sli + T.max_slices;
     int* s_hrow = reinterpret_cast<int*>(s_raw + lay.hrow);
     unsigned short* s_hli = reinterpret_cast<unsigned short*>(s_raw + lay.hli);
     float* s_p = reinterpret_cast<float*>(s_raw + lay.p);
@@ -211,13 +217,46 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
     if (tid == 0) {
         s_flag = 0;
         s_exit = 0;
-        creg = coarse_regs(bp, any_c);
     }
     init_local(bp, li, s0, s1, il0, il1);
     for (int k = tid; k <= ns; k += BLOCK) s_off[k] = t.slice_off[s0 + k];
     for (int k = tid; k < ns; k += BLOCK) {
         s_mask[k] = T.bmask[s0 + k];
         s_sli[k] = (unsigned short)(bp.slice_inst[s0 + k] - il0);
+    }
+    // the CTA's coarse blocks (runs of its slices)
+    // (their parameters wait in shared memory: registers are short)
+    __shared__ struct {
+        const float4* w;
+        const float* ainv;
+        float* vals;
+        const int *inst_blk, *inst_aoff;
+        int m, g, nv, B0, nbl;  // nv: values per set
+    } co;
+    if (tid == 0) {
+        co.nbl = 1;
+        if (any_c) {
+            const CoarseArgs& cg = *bp.cg;
+            co.w = cg.w;
+            co.ainv = cg.ainv;
+            co.vals = cg.cvals;
+            co.inst_blk = cg.inst_blk;
+            co.inst_aoff = cg.inst_aoff;
+            co.m = cg.m;
+            co.g = cg.g;
+            co.nv = 12 * cg.cta_blk[gridDim.x];
+            co.B0 = cg.cta_blk[blockIdx.x];
+            co.nbl = cg.cta_blk[blockIdx.x + 1] - co.B0;
+        }
+    }
+    __syncthreads();
+    if (any_c) {
+        const int B0 = co.B0, nbl = co.nbl;
+        for (int q = tid; q <= nbl; q += BLOCK) {
+            s_bk0[q] = bp.cg->blk_row0[B0 + q] / 32 - s0;
+            if (q < nbl) s_binst[q] = ONE ? 0 : bp.cg->blk_inst[B0 + q] - il0;
+        }
+        for (int x = tid; x < nbl * kTileCoarseW; x += BLOCK) c_blk[x] = 0.0f;
     }
     for (int h = tid; h < nh; h += BLOCK) {
         s_hrow[h] = T.halo_row[h0 + h];
@@ -243,24 +282,17 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
         li[0].seg_lo = 0;
         li[0].seg_hi = kTileWarps;
     }
+    if (any_c)
+        for (int q = warp; q < co.nbl; q += kTileWarps)
+            for (int k = s_bk0[q] + lane; k < s_bk0[q + 1]; k += 32) s_slb[k] = (unsigned short)q;
     __syncthreads();
-    const uint32_t tm_warp = s_tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    auto tm = [&](int k) { return tm_warp + (uint32_t)(kTileCols * (k >> 2)); };  // slice k of the CTA (k % 4 == warp % 4)
+    // tensor memory of the warp's j-th slice
+    const uint32_t tm0 = s_tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(kTileCols * (warp >> 2));
+    constexpr uint32_t kTmStep = kTileCols * (kTileWarps / 4);
     bool ok = true;
     auto no_step = [](LocalInst&, const double*) {};
-    const int& c_U = creg.U;
-    const int& c_nq = creg.nq;
-    auto cw = [&](int i) { return c_nq == 4 ? __ldg(creg.w + i) : make_float4(0.f, 0.f, 0.f, 0.f); };
-    auto seg_one = [&](int, int& lo, int& hi, int& slot) {
-        lo = 0;
-        hi = kTileWarps;
-        slot = li[0].own_slot;
-    };
-    auto seg_inst = [&](int q, int& lo, int& hi, int& slot) {
-        lo = li[q].seg_lo;
-        hi = li[q].seg_hi;
-        slot = li[q].own_slot;
-    };
+    auto cw = [&](int i) { return __ldg(co.w + i); };  // four fields per block always
+    auto cblk = [&](int k) { return c_blk + (ONE ? 0 : (int)s_slb[k]) * kTileCoarseW; };
     auto inst_of = [&](int k) { return ONE ? 0 : (int)s_sli[k]; };
     auto ldp = [&](int j) { return f3(s_p[3 * j], s_p[3 * j + 1], s_p[3 * j + 2]); };
     auto stp = [&](int j, float3 a) {
@@ -269,11 +301,112 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
         s_p[3 * j + 2] = a.z;
     };
     // restriction of a slice's vector into its partial (spart entry `part`)
-    auto restrict_part = [&](float3 a, float4 w4, int part) { warp_restrict(c_nq, a, w4, slice_cpart(spart, part)); };
-    // the CTA's restrictions into the slots of this phase
+    auto restrict_part = [&](float3 a, float4 w4, int part) { warp_restrict(4, a, w4, slice_cpart(spart, part)); };
+    // the CTA's restrictions, 12 values per block, into this phase's set: P
+    // threads per value add every P-th partial, then one adds the P sums
     auto publish_coarse = [&]() {
-        if (ONE) coarse_publish<BLOCK>(bp, c_U, spart, 1, seg_one, slot_set(ph), s_tmp);
-        else coarse_publish<BLOCK>(bp, c_U, spart, nloc, seg_inst, slot_set(ph), s_tmp);
+        float* dst = co.vals + (size_t)slot_set(ph) * co.nv + 12 * co.B0;
+        const int nv = ONE ? 12 : co.nbl * 12;
+        const int P = min(8, max(1, BLOCK / nv));
+        for (int x = tid; x < nv * P; x += BLOCK) {
+            const int h = x % P, qu = x / P, q = qu / 12, u = qu - 12 * q;
+            const int lo = ONE ? 0 : s_bk0[q], hi = ONE ? kTileWarps : s_bk0[q + 1];
+            float acc = 0.0f;
+            for (int sl = lo + h; sl < hi; sl += P) acc += slice_cpart(spart, sl)[u];
+            if (P > 1) s_tmp[x] = acc;
+            else dst[qu] = acc;
+        }
+        if (P > 1) {
+            __syncthreads();
+            for (int x = tid; x < nv; x += BLOCK) {
+                float acc = 0.0f;
+                for (int h = 0; h < P; ++h) acc += s_tmp[x * P + h];
+                dst[x] = acc;
+            }
+        }
+        __syncthreads();
+    };
+    // y = A_c^-1 v on the CTA's own blocks, v the values of `set`: into entry
+    // `off`, or (with_alpha) kCN = kCU - alpha y.  Ends with a __syncthreads.
+    auto apply_coarse = [&](int set, int off, bool with_alpha) {
+        const float* src = co.vals + (size_t)set * co.nv;
+        const int nbl = co.nbl;
+        if (CO == 1) {
+            const int c_m = co.m, c_g = co.g;
+            // v of every block (G CTAs each where they are small), then half
+            // a row of A_c^-1 per warp, 16-byte pieces
+            if (c_g == 1) {
+                for (int x = tid; x < c_m / 4; x += BLOCK)
+                    reinterpret_cast<float4*>(c_vbuf)[x] = __ldcg(reinterpret_cast<const float4*>(src) + x);
+            } else {
+                for (int x = tid; x < c_m / 4; x += BLOCK) {
+                    const int B = x / 3, q = x - 3 * B;
+                    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int c = B * c_g; c < min((B + 1) * c_g, (int)gridDim.x); ++c) {
+                        const float4 v4 = __ldcg(reinterpret_cast<const float4*>(src + 12 * c) + q);
+                        acc.x += v4.x;
+                        acc.y += v4.y;
+                        acc.z += v4.z;
+                        acc.w += v4.w;
+                    }
+                    reinterpret_cast<float4*>(c_vbuf)[x] = acc;
+                }
+            }
+            __syncthreads();
+            constexpr int rows = 12, parts = 2;
+            const int m4 = c_m / 4;
+            const float4* A = reinterpret_cast<const float4*>(co.ainv + (size_t)(12 * (co.B0 / c_g)) * c_m);
+            for (int x = warp; x < rows * parts; x += kTileWarps) {
+                const int r = x / parts, h = x - r * parts;
+                const float4* a4 = A + (size_t)r * m4;
+                float acc = 0.0f;
+#pragma unroll 4
+                for (int j = h * 32 + lane; j < m4; j += 32 * parts) {
+                    const float4 av = __ldg(a4 + j), vv = reinterpret_cast<const float4*>(c_vbuf)[j];
+                    acc = fmaf(av.x, vv.x, fmaf(av.y, vv.y, fmaf(av.z, vv.z, fmaf(av.w, vv.w, acc))));
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                if (lane == 0) s_tmp[x] = acc;
+            }
+            __syncthreads();
+            if (tid < rows) {
+                const float y = s_tmp[2 * tid] + s_tmp[2 * tid + 1];
+                float* o = c_blk + tid;
+                if (with_alpha) o[kCN] = fmaf(-li[0].alpha, y, o[kCU]);
+                else o[off] = y;
+            }
+        }
+        if (CO == 2) {
+            // a warp per block: the instance's values (at most 160, five per
+            // lane) times the block's 12 rows of the instance's inverse
+            for (int q = warp; q < nbl; q += kTileWarps) {
+                const LocalInst& L = li[s_binst[q]];
+                if (L.done) continue;
+                const int I0 = co.inst_blk[L.b], m = 12 * (co.inst_blk[L.b + 1] - I0);
+                const float* A = co.ainv + co.inst_aoff[L.b] + (size_t)(12 * (co.B0 + q - I0)) * m;
+                float c[5], prod[16];
+#pragma unroll
+                for (int z = 0; z < 5; ++z) c[z] = lane + 32 * z < m ? __ldcg(src + 12 * I0 + lane + 32 * z) : 0.0f;
+#pragma unroll
+                for (int r = 0; r < 16; ++r) prod[r] = 0.0f;
+#pragma unroll
+                for (int z = 0; z < 5; ++z)
+                    if (lane + 32 * z < m) {
+#pragma unroll
+                        for (int r = 0; r < 12; ++r)
+                            prod[r] = fmaf(__ldg(A + (size_t)r * m + lane + 32 * z), c[z], prod[r]);
+                    }
+                const float y = warp_sum16(prod);
+                const int u = lane >> 1;
+                float* o = c_blk + q * kTileCoarseW;
+                if ((lane & 1) == 0 && u < 12) {
+                    if (with_alpha) o[kCN + u] = fmaf(-L.alpha, y, o[kCU + u]);
+                    else o[off + u] = y;
+                }
+            }
+        }
+        __syncthreads();
     };
     // One reduction phase, after the partials and a __syncthreads: a warp per
     // instance publishes the CTA's segment, thread 0 meets the other CTAs, a
@@ -348,18 +481,12 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
     using N2 = std::integral_constant<int, 2>;
     using N8 = std::integral_constant<int, kStartW>;
     // one exchange phase carrying only the restriction in the partials
-    auto coarse_exchange = [&](float* out) {
+    auto coarse_exchange = [&](int off) {
         __syncthreads();
         publish_coarse();
         const int set = slot_set(ph);
         phase(N1{}, false, no_step);
-        if (!s_flag) {
-            if (coarse) coarse_apply_dense<BLOCK>(bp, creg, set, c_vbuf, out);
-            if (coarse_b) {
-                coarse_apply_inst(bp, creg, li, nloc, set, c_inst, kCU, kTileWarps, false);
-                __syncthreads();
-            }
-        }
+        if (!s_flag) apply_coarse(set, off, false);
         ok = s_flag == 0;
     };
     // (A p)_i = D'_i p_i + sum_j A_ij (p_j - p_i) of row `lane` of slice k, p in shared memory
@@ -426,9 +553,10 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
     auto restrict_all = [&](auto&& get) {
         Sums sm;
         zero_sums(sm);
-        for (int k = warp; k < ns; k += kTileWarps) {
+        uint32_t tm = tm0;
+        for (int k = warp; k < ns; k += kTileWarps, tm += kTmStep) {
             const int i = (s0 + k) * 32 + lane;
-            const float3 a = get(k, i);
+            const float3 a = get(tm, i);
             const float4 w4 = i < t.n ? cw(i) : make_float4(0.f, 0.f, 0.f, 0.f);
             if (ONE) add_restrict(sm, a, w4);
             else {
@@ -441,7 +569,7 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
             put_restrict(sm);
         }
     };
-    auto load_b = [&](int, int i) { return i < t.n ? xyz(v.b[i]) : f3(0.f, 0.f, 0.f); };
+    auto load_b = [&](uint32_t, int i) { return i < t.n ? xyz(v.b[i]) : f3(0.f, 0.f, 0.f); };
     auto load_minv = [&](int s, int i) {
         S6 m{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         if (i < t.n)
@@ -455,58 +583,60 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
     // ---- start: r = b - A x0, z = M^-1 r, the instances' start values -------
     if (any_c) {
         restrict_all(load_b);
-        coarse_exchange(s_cb);  // A_c^-1 R^T b (coarse_b: into kCU)
+        coarse_exchange(kTcB);  // A_c^-1 R^T b
     }
     if (ok && warm) {
-        for (int k = warp; k < ns; k += kTileWarps) {
+        uint32_t tm = tm0;
+        for (int k = warp; k < ns; k += kTileWarps, tm += kTmStep) {
             const int i = (s0 + k) * 32 + lane;
             stp(k * 32 + lane, i < t.n ? xyz(v.x[i]) : f3(0.f, 0.f, 0.f));
         }
         for (int h = tid; h < nh; h += BLOCK) stp(nown + h, xyz(ldcg4(v.x + s_hrow[h])));
         __syncthreads();
-        for (int k = warp; k < ns; k += kTileWarps) {
+        tm = tm0;
+        for (int k = warp; k < ns; k += kTileWarps, tm += kTmStep) {
             const int i = (s0 + k) * 32 + lane;
             const float3 ax = row_product(k, ldp(k * 32 + lane));
-            tm_st3(tm(k) + kTmR, load_b(k, i) - ax);
+            tm_st3(tm + kTmR, load_b(0u, i) - ax);
         }
         tm_wait_st();
         if (coarse) {
-            restrict_all([&](int k, int) {
+            restrict_all([&](uint32_t tm, int) {
                 float3 r, d = f3(0.f, 0.f, 0.f);
-                tm_ld3(tm(k) + kTmR, r);
+                tm_ld3(tm + kTmR, r);
                 tm_wait_ld(r, d);
                 return r;
             });
-            coarse_exchange(s_c0);  // A_c^-1 R^T r0
+            coarse_exchange(kTc0);  // A_c^-1 R^T r0
         }
     }
     auto zb_of = [&](int k, int i, const S6& Mi, float3 b, float4 w4) {
         float3 zb = mul(Mi, b);
-        if (coarse) zb = zb + coarse_prolong(c_nq, s_cb, w4);
-        if (coarse_b) zb = zb + coarse_prolong(c_nq, c_inst + inst_of(k) * kInstCoarseW + kCU, w4);
+        if (any_c) zb = zb + coarse_prolong(4, cblk(k) + kTcB, w4);
         return zb;
     };
     if (ok) {
         double tot[kStartW];
 #pragma unroll
         for (int u = 0; u < kStartW; ++u) tot[u] = 0.0;
-        for (int k = warp; k < ns; k += kTileWarps) {
+        uint32_t tm = tm0;
+        for (int k = warp; k < ns; k += kTileWarps, tm += kTmStep) {
             const int i = (s0 + k) * 32 + lane;
             const S6 Mi = load_minv(s0 + k, i);
             const float4 w4 = any_c && i < t.n ? cw(i) : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float3 b = load_b(k, i), zb = zb_of(k, i, Mi, b, w4);
+            const float3 b = load_b(0u, i), zb = zb_of(k, i, Mi, b, w4);
             float3 x0 = f3(0.f, 0.f, 0.f), r = b, z = zb;
             if (warm) {
                 float3 d = f3(0.f, 0.f, 0.f);
-                tm_ld3(tm(k) + kTmR, r);
+                tm_ld3(tm + kTmR, r);
                 tm_wait_ld(r, d);
                 x0 = ldp(k * 32 + lane);
                 z = mul(Mi, r);
-                if (coarse) z = z + coarse_prolong(c_nq, s_c0, w4);
+                if (coarse) z = z + coarse_prolong(4, cblk(k) + kTc0, w4);
             } else {
-                tm_st3(tm(k) + kTmX, x0);
-                tm_st3(tm(k) + kTmR, r);
-                tm_st3(tm(k) + kTmQ, z);
+                tm_st3(tm + kTmX, x0);
+                tm_st3(tm + kTmR, r);
+                tm_st3(tm + kTmQ, z);
                 publish_z(k, i, z);
             }
             const double q8[kStartW] = {dot3d(r, z), dot3d(r, r), dot3d(b, b), dot3d(b, zb),
@@ -536,24 +666,25 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
     }
     if (ok && warm) {
         // the scaled guess, or the zero guess where the instance fell back
-        for (int k = warp; k < ns; k += kTileWarps) {
+        uint32_t tm = tm0;
+        for (int k = warp; k < ns; k += kTileWarps, tm += kTmStep) {
             const int i = (s0 + k) * 32 + lane;
             const S6 Mi = load_minv(s0 + k, i);
             const float4 w4 = any_c && i < t.n ? cw(i) : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float3 b = load_b(k, i);
+            const float3 b = load_b(0u, i);
             float3 x = ldp(k * 32 + lane), r, z, d = f3(0.f, 0.f, 0.f);
-            tm_ld3(tm(k) + kTmR, r);
+            tm_ld3(tm + kTmR, r);
             tm_wait_ld(r, d);
             const LocalInst& L = li[inst_of(k)];
             if (coarse) {
-                z = mul(Mi, r) + coarse_prolong(c_nq, s_c0, w4);
+                z = mul(Mi, r) + coarse_prolong(4, cblk(k) + kTc0, w4);
                 start_row_linear(L, b, zb_of(k, i, Mi, b, w4), x, r, z);
             } else {
                 start_row(L, b, Mi, x, r, z);
             }
-            tm_st3(tm(k) + kTmX, x);
-            tm_st3(tm(k) + kTmR, r);
-            tm_st3(tm(k) + kTmQ, z);
+            tm_st3(tm + kTmX, x);
+            tm_st3(tm + kTmR, r);
+            tm_st3(tm + kTmQ, z);
             publish_z(k, i, z);
         }
         tm_wait_st();
@@ -563,10 +694,13 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
         phase(N1{}, false, no_step);
         ok = s_flag == 0;
     }
-    if (coarse && ok) {
-        const LocalInst& L0 = li[0];
-        const bool from_r0 = warm && !L0.fallback;
-        if (tid < c_U) s_cu[tid] = from_r0 ? fmaf(L0.scale, s_c0[tid], L0.scale_b * s_cb[tid]) : s_cb[tid];
+    if (any_c && ok) {
+        // A_c^-1 R^T r of the start: of r0, of the scaled mix of r0 and b, or of b
+        const bool from_r0 = coarse && warm && !li[0].fallback;
+        for (int x = tid; x < 12 * co.nbl; x += BLOCK) {
+            float* o = c_blk + (x / 12) * kTileCoarseW + x % 12;
+            o[kCU] = from_r0 ? fmaf(li[0].scale, o[kTc0], li[0].scale_b * o[kTcB]) : o[kTcB];
+        }
         __syncthreads();
     }
 
@@ -576,17 +710,18 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
         if (ONE && li[0].done) break;  // uniform over the grid: every CTA forms the same totals
         // p = z + beta p of the own rows and, from the published z, of the
         // halo; x takes the previous iteration's alpha p
-        for (int k = warp; k < ns; k += kTileWarps) {
+        uint32_t tm = tm0;
+        for (int k = warp; k < ns; k += kTileWarps, tm += kTmStep) {
             const LocalInst& L = li[inst_of(k)];
             if (L.done) continue;
             float3 z, x = f3(0.f, 0.f, 0.f);
-            tm_ld3(tm(k) + kTmQ, z);
+            tm_ld3(tm + kTmQ, z);
             if (L.iter > 0) {
-                tm_ld3(tm(k) + kTmX, x);
+                tm_ld3(tm + kTmX, x);
                 const float3 p = ldp(k * 32 + lane);
                 const float al = L.alpha, be = L.beta;
                 tm_wait_ld(z, x);
-                tm_st3(tm(k) + kTmX, f3(fmaf(al, p.x, x.x), fmaf(al, p.y, x.y), fmaf(al, p.z, x.z)));
+                tm_st3(tm + kTmX, f3(fmaf(al, p.x, x.x), fmaf(al, p.y, x.y), fmaf(al, p.z, x.z)));
                 z = f3(fmaf(be, p.x, z.x), fmaf(be, p.y, z.y), fmaf(be, p.z, z.z));
             } else {
                 tm_wait_ld(z, x);
@@ -609,14 +744,15 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
         {
             Sums sm;
             zero_sums(sm);
-            for (int k = warp; k < ns; k += kTileWarps) {
+            uint32_t tm = tm0;
+            for (int k = warp; k < ns; k += kTileWarps, tm += kTmStep) {
                 const LocalInst& L = li[inst_of(k)];
                 if (L.done) continue;
                 const int i = (s0 + k) * 32 + lane;
                 const float4 w4 = any_c && i < t.n ? cw(i) : make_float4(0.f, 0.f, 0.f, 0.f);
                 const float3 pi = ldp(k * 32 + lane);
                 const float3 acc = row_product(k, pi);
-                tm_st3(tm(k) + kTmQ, acc);
+                tm_st3(tm + kTmQ, acc);
                 const double sig = (double)pi.x * acc.x + (double)pi.y * acc.y + (double)pi.z * acc.z;
                 if (ONE) {
                     sm.a += sig;
@@ -644,39 +780,31 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
         }
         // every CTA reads ndone between the same two barriers, where it does not change
         if (!ONE && s_exit) break;
-        if (coarse) {
-            coarse_apply_dense<BLOCK>(bp, creg, set1, c_vbuf, s_cw);
-            if (tid < c_U) s_cn[tid] = fmaf(-li[0].alpha, s_cw[tid], s_cu[tid]);
-            __syncthreads();
-        }
-        if (coarse_b) {
-            coarse_apply_inst(bp, creg, li, nloc, set1, c_inst, 0, kTileWarps, true);
-            __syncthreads();
-        }
+        if (any_c) apply_coarse(set1, 0, true);
         // r -= alpha A p; z = M^-1 r (+ its coarse part)
         {
             Sums sm;
             zero_sums(sm);
-            for (int k = warp; k < ns; k += kTileWarps) {
+            uint32_t tm = tm0;
+            for (int k = warp; k < ns; k += kTileWarps, tm += kTmStep) {
                 const int q = inst_of(k);
                 const LocalInst& L = li[q];
                 if (L.done) continue;
                 const int i = (s0 + k) * 32 + lane;
                 float3 r, ap;
                 __syncwarp();
-                tm_ld4(tm(k) + kTmR, r.x, r.y, r.z, ap.x);
-                tm_ld2(tm(k) + kTmQ + 1, ap.y, ap.z);
+                tm_ld4(tm + kTmR, r.x, r.y, r.z, ap.x);
+                tm_ld2(tm + kTmQ + 1, ap.y, ap.z);
                 const S6 Mi = load_minv(s0 + k, i);
                 const float4 w4 = any_c && i < t.n ? cw(i) : make_float4(0.f, 0.f, 0.f, 0.f);
                 const float al = L.alpha;
                 tm_wait_ld(r, ap);
                 const float3 rn = f3(fmaf(-al, ap.x, r.x), fmaf(-al, ap.y, r.y), fmaf(-al, ap.z, r.z));
                 float3 zn = mul(Mi, rn);
-                if (coarse) zn = zn + coarse_prolong(c_nq, s_cn, w4);
-                if (coarse_b) zn = zn + coarse_prolong(c_nq, c_inst + q * kInstCoarseW + kCN, w4);
+                if (any_c) zn = zn + coarse_prolong(4, cblk(k) + kCN, w4);
                 __syncwarp();
-                tm_st4(tm(k) + kTmR, rn.x, rn.y, rn.z, zn.x);
-                tm_st2(tm(k) + kTmQ + 1, zn.y, zn.z);
+                tm_st4(tm + kTmR, rn.x, rn.y, rn.z, zn.x);
+                tm_st2(tm + kTmQ + 1, zn.y, zn.z);
                 publish_z(k, i, zn);
                 const double rz = dot3d(rn, zn), rr = dot3d(rn, rn);
                 if (ONE) {
@@ -711,18 +839,15 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
             break;
         }
         // the coarse part restarts from R^T r_new (no recurrence drift)
-        if (coarse) coarse_apply_dense<BLOCK>(bp, creg, set2, c_vbuf, s_cu);
-        if (coarse_b) {
-            coarse_apply_inst(bp, creg, li, nloc, set2, c_inst, kCU, kTileWarps, false);
-            __syncthreads();
-        }
+        if (any_c) apply_coarse(set2, kCU, false);
     }
     // x with the last iteration's alpha p
-    for (int k = warp; k < ns; k += kTileWarps) {
+    uint32_t tm = tm0;
+    for (int k = warp; k < ns; k += kTileWarps, tm += kTmStep) {
         const LocalInst& L = li[inst_of(k)];
         const int i = (s0 + k) * 32 + lane;
         float3 x, d = f3(0.f, 0.f, 0.f);
-        tm_ld3(tm(k) + kTmX, x);
+        tm_ld3(tm + kTmX, x);
         tm_wait_ld(x, d);
         if (L.iter > 0) {
             const float3 p = ldp(k * 32 + lane);
