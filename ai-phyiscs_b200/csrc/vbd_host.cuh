@@ -1,8 +1,8 @@
 // Host side of the cloth VBD solver (the reference's ClothVBDSolver,
 // src/bindings.cpp:1868-1957, solver/vbd_solver.h:134-176): colouring,
-// per-vertex adjacency, and the step, which runs as one CUDA graph (predictor,
-// iterations x colours sweep kernels, velocity update) rebuilt only when the
-// step's arguments change.  Included by cloth_sim.cu (shares its error
+// per-vertex adjacency, and the step, which runs as one CUDA graph (one
+// cooperative kernel, or predictor, iterations x colours sweep kernels and
+// velocity update) rebuilt only when the step's arguments change.  Included by cloth_sim.cu (shares its error
 // handling and device buffers).
 #pragma once
 
@@ -117,9 +117,17 @@ public:
                 d_edge_off_.upload(edge_off_);
                 d_edge_adj_.upload(edge_adj_);
             }
+            plan_records();
             dirty_ = false;
         }
-        if (d_q_prev_.size() != 3 * (size_t)n) {
+        if (one_launch_) {
+            if (d_state_.size() != (size_t)n) {
+                d_state_.resize((size_t)n);
+                d_own_.resize((size_t)n);
+                d_bar_.resize(1);
+                drop_graph();
+            }
+        } else if (d_q_prev_.size() != 3 * (size_t)n) {
             d_q_prev_.resize(3 * (size_t)n);
             d_inertia_.resize(3 * (size_t)n);
             d_disp_.resize(3 * (size_t)n);
@@ -152,7 +160,10 @@ public:
         a.gy = gy;
         a.gz = gz;
         a.dt = dt;
-        if (!exec_ || !same_bytes(a, graph_args_) || iterations != graph_iters_) build_graph(a, iterations);
+        if (!exec_ || !same_bytes(a, graph_args_) || iterations != graph_iters_) {
+            if (one_launch_) build_graph_one(a, iterations);
+            else build_graph(a, iterations);
+        }
         ck(cudaGraphLaunch(exec_, reinterpret_cast<cudaStream_t>(stream)), "cudaGraphLaunch(vbd step)");
     }
 
@@ -186,6 +197,65 @@ private:
         drop_graph();
     }
 
+    // Whether the step runs as one cooperative kernel, its lanes per vertex and
+    // the element records' places.  One kernel where 4 lanes per vertex of
+    // every colour fit the GPU at once (512 threads per SM: 18,944 vertices a
+    // colour, e.g. a 275 x 275 grid in four): there a sweep is latency.  16
+    // lanes take a regular mesh's 6 triangles and 12 hinges in one round each;
+    // colours that would not fit with 16 take 8 or 4.  Larger meshes keep a
+    // launch per colour: one kernel measured 2.16 against 2.86 ms on 701 x 513
+    // vertices, but steps at such resolutions can tear elements at a pinned
+    // corner (velocities of 1e4 m/s), and then any change of rounding shows in
+    // the result.
+    void plan_records() {
+        int dev = 0, sms = 148;
+        ck(cudaGetDevice(&dev), "cudaGetDevice");
+        ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
+        const long cap = 512L * sms;
+        const int nc = num_colors();
+        one_launch_ = nc > 0;
+        for (int c = 0; c < nc; ++c) one_launch_ = one_launch_ && 4L * (group_off_[c + 1] - group_off_[c]) <= cap;
+        drop_graph();
+        if (!one_launch_) return;
+        std::vector<vbd::ColorPlan> plan(std::max(1, nc));
+        std::vector<int> tri_rec{0}, hinge_rec{0};
+        max_tiles_ = 1;
+        for (int c = 0; c < nc; ++c) {
+            vbd::ColorPlan& p = plan[c];
+            p.first = group_off_[c];
+            p.count = group_off_[c + 1] - group_off_[c];
+            p.log_lanes = 16L * p.count <= cap ? 4 : (8L * p.count <= cap ? 3 : 2);
+            p.tile0 = (int)tri_rec.size() - 1;
+            const int V = 32 >> p.log_lanes, L = 1 << p.log_lanes;
+            const int tiles = (p.count + V - 1) / V;
+            max_tiles_ = std::max(max_tiles_, tiles);
+            for (int t = 0; t < tiles; ++t) {
+                int wt = 0, wh = 0;
+                for (int k = t * V; k < std::min(p.count, (t + 1) * V); ++k) {
+                    const int i = ids_[p.first + k];
+                    if (tri_n_ == n_) wt = std::max(wt, (tri_off_[i + 1] - tri_off_[i]) / 2);
+                    if (edge_n_ == n_) wh = std::max(wh, (edge_off_[i + 1] - edge_off_[i]) / 2);
+                }
+                tri_rec.push_back(next_offset(tri_rec.back(), (wt + L - 1) / L));
+                hinge_rec.push_back(next_offset(hinge_rec.back(), (wh + L - 1) / L));
+            }
+        }
+        d_colors_.upload(plan);
+        d_tri_rec_.upload(tri_rec);
+        d_hinge_rec_.upload(hinge_rec);
+        const size_t nt = (size_t)std::max(1, tri_rec.back()), nh = (size_t)std::max(1, hinge_rec.back());
+        d_tri_v_.resize(nt);
+        d_tri_dm_.resize(nt);
+        d_tri_m_.resize(nt);
+        d_hinge_v_.resize(nh);
+        d_hinge_m_.resize(nh);
+    }
+    static int next_offset(int o, int rounds) {
+        const long long v = (long long)o + 32LL * rounds;
+        if (v > 0x7fffffffLL) throw std::invalid_argument("step_cloth: more than 2^31 element records");
+        return (int)v;
+    }
+
     // lanes per vertex: as many (up to 8) as keep the colour's threads within
     // four times what the GPU holds at two 256-thread CTAs per SM
     static int lanes_for(int count) {
@@ -201,6 +271,59 @@ private:
     void drop_graph() {
         if (exec_) cudaGraphExecDestroy(exec_);
         exec_ = nullptr;
+    }
+
+    // one graph: the barrier's reset and the cooperative step kernel
+    void build_graph_one(const vbd::ClothArgs& a, int iterations) {
+        drop_graph();
+        int dev = 0, sms = 0, per_sm = 0;
+        ck(cudaGetDevice(&dev), "cudaGetDevice");
+        ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
+        ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, vbd::vbd_step_kernel, vbd::kVbdThreads, 0),
+           "cudaOccupancyMaxActiveBlocksPerMultiprocessor(vbd)");
+        // no more CTAs than the largest colour has warps for: fewer arrivals per barrier
+        const int want = (max_tiles_ + vbd::kVbdThreads / 32 - 1) / (vbd::kVbdThreads / 32);
+        cudaGraph_t g;
+        ck(cudaGraphCreate(&g, 0), "cudaGraphCreate(vbd)");
+        cudaGraphNode_t reset, node;
+        cudaMemsetParams mp{};
+        vbd::StepPlan sp{};
+        sp.state = d_state_.get();
+        sp.own = d_own_.get();
+        sp.ids = d_ids_.get();
+        sp.colors = d_colors_.get();
+        sp.tri_rec = d_tri_rec_.get();
+        sp.hinge_rec = d_hinge_rec_.get();
+        sp.rec.tri_v = d_tri_v_.get();
+        sp.rec.tri_dm = d_tri_dm_.get();
+        sp.rec.tri_m = d_tri_m_.get();
+        sp.rec.hinge_v = d_hinge_v_.get();
+        sp.rec.hinge_m = d_hinge_m_.get();
+        sp.bar = d_bar_.get();
+        sp.n_colors = num_colors();
+        sp.iterations = iterations;
+        mp.dst = sp.bar;
+        mp.value = 0;
+        mp.elementSize = 4;
+        mp.width = sizeof(GridBarrier) / 4;
+        mp.height = 1;
+        cudaError_t e = cudaGraphAddMemsetNode(&reset, g, nullptr, 0, &mp);
+        vbd::ClothArgs args = a;
+        void* prm[] = {&args, &sp};
+        cudaKernelNodeParams p{};
+        p.func = reinterpret_cast<void*>(&vbd::vbd_step_kernel);
+        p.gridDim = dim3(std::max(1, std::min(want, std::max(1, per_sm) * sms)));
+        p.blockDim = dim3(vbd::kVbdThreads);
+        p.kernelParams = prm;
+        if (e == cudaSuccess) e = cudaGraphAddKernelNode(&node, g, &reset, 1, &p);
+        cudaLaunchAttributeValue av{};
+        av.cooperative = 1;
+        if (e == cudaSuccess) e = cudaGraphKernelNodeSetAttribute(node, cudaLaunchAttributeCooperative, &av);
+        if (e == cudaSuccess) e = cudaGraphInstantiate(&exec_, g, 0);
+        cudaGraphDestroy(g);
+        ck(e, "vbd step graph");
+        graph_args_ = a;
+        graph_iters_ = iterations;
     }
 
     // predictor, iterations x colours sweeps, velocity: all in one graph
@@ -257,6 +380,16 @@ private:
     bool dirty_ = false;
     DevBuf<int> d_ids_, d_tri_off_, d_tri_adj_, d_edge_off_, d_edge_adj_;
     DevBuf<float> d_q_prev_, d_inertia_, d_disp_, d_mass_;
+    // the one-kernel step
+    bool one_launch_ = false;
+    DevBuf<vbd::VertexState> d_state_;
+    DevBuf<vbd::VertexOwn> d_own_;
+    DevBuf<vbd::ColorPlan> d_colors_;
+    DevBuf<int> d_tri_rec_, d_hinge_rec_;  // record offsets per tile
+    DevBuf<int4> d_tri_v_, d_hinge_v_;     // element records
+    DevBuf<float4> d_tri_dm_, d_tri_m_, d_hinge_m_;
+    DevBuf<GridBarrier> d_bar_;
+    int max_tiles_ = 1;
     cudaGraphExec_t exec_ = nullptr;
     vbd::ClothArgs graph_args_{};
     int graph_iters_ = -1;

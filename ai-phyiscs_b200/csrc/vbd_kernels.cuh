@@ -18,6 +18,8 @@
 
 #include <cuda_runtime.h>
 
+#include "pcg_persistent.cuh"  // GridBarrier
+
 namespace chysx_b200 {
 namespace vbd {
 
@@ -80,6 +82,54 @@ __device__ __forceinline__ M3 inv3(const M3& a, float d) {
     return r;
 }
 
+// The upper triangle of a vertex Hessian (xx, xy, xz, yy, yz, zz): all its
+// terms are symmetric.  The element functions below work on either form.
+struct H6 {
+    float xx, xy, xz, yy, yz, zz;
+};
+__device__ __forceinline__ void set_zero(M3& h) { h = zero3(); }
+__device__ __forceinline__ void set_zero(H6& h) { h = H6{0.f, 0.f, 0.f, 0.f, 0.f, 0.f}; }
+__device__ __forceinline__ void add_scaled_identity(H6& h, float s) {
+    h.xx += s;
+    h.yy += s;
+    h.zz += s;
+}
+// h += s a a^T
+__device__ __forceinline__ void add_outer(H6& h, V3 a, V3, float s) {
+    const V3 b = a * s;
+    h.xx += b.x * a.x;
+    h.xy += b.x * a.y;
+    h.xz += b.x * a.z;
+    h.yy += b.y * a.y;
+    h.yz += b.y * a.z;
+    h.zz += b.z * a.z;
+}
+__device__ __forceinline__ void add_to(M3& h, const M3& a) {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) h.m[k] += a.m[k];
+}
+__device__ __forceinline__ void add_to(H6& h, const H6& a) {
+    h.xx += a.xx;
+    h.xy += a.xy;
+    h.xz += a.xz;
+    h.yy += a.yy;
+    h.yz += a.yz;
+    h.zz += a.zz;
+}
+__device__ __forceinline__ float det6(const H6& a) {
+    return a.xx * (a.yy * a.zz - a.yz * a.yz) - a.xy * (a.xy * a.zz - a.yz * a.xz) +
+           a.xz * (a.xy * a.yz - a.yy * a.xz);
+}
+// a^-1 v by the adjugate over the determinant d
+__device__ __forceinline__ V3 solve6(const H6& a, float d, V3 v) {
+    const float s = 1.0f / d;
+    const float ixx = (a.yy * a.zz - a.yz * a.yz) * s, ixy = (a.xz * a.yz - a.xy * a.zz) * s,
+                ixz = (a.xy * a.yz - a.xz * a.yy) * s, iyy = (a.xx * a.zz - a.xz * a.xz) * s,
+                iyz = (a.xz * a.xy - a.xx * a.yz) * s, izz = (a.xx * a.yy - a.xy * a.xy) * s;
+    return v3(ixx * v.x + ixy * v.y + ixz * v.z, ixy * v.x + iyy * v.y + iyz * v.z,
+              ixz * v.x + iyz * v.y + izz * v.z);
+}
+
 __device__ __forceinline__ V3 ld(const float* p, int i) { return v3(p[3 * i], p[3 * i + 1], p[3 * i + 2]); }
 __device__ __forceinline__ void st(float* p, int i, V3 v) {
     p[3 * i] = v.x;
@@ -92,8 +142,9 @@ __device__ __forceinline__ void st(float* p, int i, V3 v) {
 // Hessian kd / dt gc gc^T, both times the element area (the reference's
 // Rayleigh-style damping of the membrane's two strain measures and of the
 // hinge angle).
+template <class H>
 __device__ __forceinline__ void add_damping(float kd, V3 gc, float cdot, float inv_dt, float area, V3& force,
-                                            M3& hm) {
+                                            H& hm) {
     force = force - gc * (kd * cdot * area);
     add_outer(hm, gc, gc, kd * inv_dt * area);
 }
@@ -116,8 +167,9 @@ __device__ __forceinline__ void add_damping(float kd, V3 gc, float cdot, float i
 // Damping acts on the Green strain G = (F^T F - I) / 2 through its norm |G|
 // (weight mu * damping) and its trace (weight lambda * damping), with rates
 // from the step's displacement (x - p) / dt.
+template <class H>
 __device__ void membrane(int which, V3 x0, V3 x1, V3 x2, V3 p0, V3 p1, V3 p2, const float* dmi, float area,
-                         float mu, float lambda, float damping, float dt, V3& f, M3& h) {
+                         float mu, float lambda, float damping, float dt, V3& f, H& h) {
     const float d00 = dmi[0], d01 = dmi[1], d10 = dmi[2], d11 = dmi[3];
     const V3 e1 = x1 - x0, e2 = x2 - x0;
     const V3 f0 = e1 * d00 + e2 * d10, f1 = e1 * d01 + e2 * d11;
@@ -145,7 +197,8 @@ __device__ void membrane(int which, V3 x0, V3 x1, V3 x2, V3 p0, V3 p1, V3 p2, co
     V3 force = ((f0 * q0 + f1 * q1) * mu + dJ * vol) * (-area);
     const float r = fmaxf(vol, 0.0f) / J;
     const float ww = dot(w, w);
-    M3 hm = zero3();
+    H hm;
+    set_zero(hm);
     add_scaled_identity(hm, (mu * (q0 * q0 + q1 * q1) + r * ww) * area);
     add_outer(hm, dJ, dJ, (lam - r) * area);
     add_outer(hm, w, w, -r * area);
@@ -170,8 +223,7 @@ __device__ void membrane(int which, V3 x0, V3 x1, V3 x2, V3 p0, V3 p1, V3 p2, co
         }
     }
     f = f + force;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) h.m[k] += hm.m[k];
+    add_to(h, hm);
 }
 
 // Hinge bending force and Hessian block of vertex `which` (0..3) of one
@@ -189,8 +241,9 @@ __device__ void membrane(int which, V3 x0, V3 x1, V3 x2, V3 p0, V3 p1, V3 p2, co
 // (they sum to zero).  Gauss-Newton Hessian k g g^T; damping on the angle's
 // rate sum_i g_i . (x_i - p_i) / dt with weight damping * k.  A hinge with
 // a collapsed face or edge contributes nothing.
+template <class H>
 __device__ void bending(int which, const V3 (&x)[4], const V3 (&p)[4], float rest_angle, float rest_length,
-                        float stiffness, float damping, float dt, V3& f, M3& h) {
+                        float stiffness, float damping, float dt, V3& f, H& h) {
     constexpr float kMin = 1.0e-6f;
     const V3 e = x[3] - x[2];
     const V3 n1 = cross(x[2] - x[0], x[3] - x[0]);
@@ -210,7 +263,8 @@ __device__ void bending(int which, const V3 (&x)[4], const V3 (&p)[4], float res
     const V3 gv = which == 0 ? g[0] : (which == 1 ? g[1] : (which == 2 ? g[2] : g[3]));
     const float k = stiffness * rest_length;
     V3 force = gv * (-k * (theta - rest_angle));
-    M3 hb = zero3();
+    H hb;
+    set_zero(hb);
     add_outer(hb, gv, gv, k);
     if (damping > 0.0f) {
         const float inv_dt = 1.0f / dt;
@@ -220,8 +274,7 @@ __device__ void bending(int which, const V3 (&x)[4], const V3 (&p)[4], float res
         add_damping(damping * k, gv, rate * inv_dt, inv_dt, 1.0f, force, hb);
     }
     f = f + force;
-#pragma unroll
-    for (int q = 0; q < 9; ++q) h.m[q] += hb.m[q];
+    add_to(h, hb);
 }
 
 // ---------------------------------------------------------------------------
@@ -352,6 +405,297 @@ __global__ void vbd_velocity_kernel(ClothArgs a) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.n) return;
     st(a.vel, i, (ld(a.pos, i) - ld(a.q_prev, i)) * (1.0f / a.dt));
+}
+
+// ---------------------------------------------------------------------------
+// The whole step in one cooperative launch, for meshes whose colours the GPU
+// holds at once (VbdSolver::one_launch): the launch-per-colour kernels above
+// spend such a sweep on a launch and on four dependent loads (vertex ->
+// adjacency -> element -> neighbours).
+// ---------------------------------------------------------------------------
+
+// A vertex between sweeps: its position (with the mass) and its position at
+// the start of the step, one 32-byte sector for the neighbours' reads; and
+// what only its own update reads, the displacement and the inertia target.
+struct VertexState {
+    float4 xm;
+    float4 q;
+};
+struct VertexOwn {
+    float4 d;
+    float4 y;
+};
+// A triangle or hinge as one of its vertices sees it, packed each step from
+// the caller's arrays into planes: the element's vertices in element order
+// with -1 in place of the vertex itself (first entry -2: no element), and
+// what the element's term needs.
+struct Records {
+    int4* tri_v;      // v0, v1, v2, unused
+    float4* tri_dm;   // Dm^-1
+    float4* tri_m;    // area, mu, lambda, damping
+    int4* hinge_v;    // o0, o1, v2, v3
+    float4* hinge_m;  // rest angle, rest length, stiffness, damping
+};
+
+// One colour: `count` vertices from `first` in colour order, 2^log_lanes
+// lanes each, so a warp takes 32 >> log_lanes of them (a tile); the tile's
+// element records lie at tri_off / hinge_off[tile0 + tile] in rounds of 32,
+// lane by lane.
+struct ColorPlan {
+    int first, count, log_lanes, tile0;
+};
+
+struct StepPlan {
+    VertexState* state;
+    VertexOwn* own;
+    const int* ids;        // vertices in colour order
+    const ColorPlan* colors;
+    const int* tri_rec;    // [tiles + 1] record offsets
+    const int* hinge_rec;
+    Records rec;
+    GridBarrier* bar;
+    int n_colors, iterations;
+};
+
+// Before the first barrier: the predictor (q_prev = x, m = 1/w, inertia y = x + dt v', x = y with v' = v +
+// dt g; a particle with w == 0 stays, vbd_solver.cu:64-92) and the packing of
+// every vertex's element records; then iterations x colours sweeps
+// (vbd_solver.cu:304-407) with a grid barrier each; then x and v = (x -
+// q_prev) / dt (vbd_solver.cu:284-293).  The caller's positions are q_prev
+// until the end.
+//
+// Records are read in lane order and fetched one round, one tile and one
+// barrier ahead, so a sweep waits for its neighbours' state and nothing else.
+// 64 x 64 vertices, 10 iterations of 4 colours: 352 us with a launch per
+// colour, 244 us here.
+constexpr int kVbdThreads = 256;
+__global__ void __launch_bounds__(kVbdThreads, 2) vbd_step_kernel(ClothArgs a, StepPlan s) {
+    __shared__ int s_ok;
+    const int lane = threadIdx.x & 31;
+    const int gt = blockIdx.x * kVbdThreads + threadIdx.x, gn = gridDim.x * kVbdThreads;
+    const int gw = gt >> 5, nw = gn >> 5;
+    unsigned target = 0;
+    auto grid_sync = [&]() -> bool {
+        __syncthreads();
+        if (threadIdx.x == 0) s_ok = barrier_arrive_wait(s.bar, target) ? 1 : 0;
+        __syncthreads();
+        return s_ok != 0;
+    };
+    const float dt = a.dt;
+    for (int i = gt; i < a.n; i += gn) {
+        const V3 x = ld(a.pos, i);
+        const float w = a.inv_mass[i];
+        V3 d = v3(0.f, 0.f, 0.f), y = x;
+        if (w != 0.0f) {
+            const V3 vn = ld(a.vel, i) + v3(a.gx, a.gy, a.gz) * dt;
+            d = vn * dt;
+            y = x + d;
+        }
+        s.state[i].xm = make_float4(y.x, y.y, y.z, (w > 1.0e-12f) ? (1.0f / w) : 0.0f);
+        s.state[i].q = make_float4(x.x, x.y, x.z, 0.f);
+        s.own[i].d = make_float4(d.x, d.y, d.z, 0.f);
+        s.own[i].y = make_float4(y.x, y.y, y.z, 0.f);
+    }
+    for (int c = 0; c < s.n_colors; ++c) {
+        const ColorPlan cp = s.colors[c];
+        const int V = 32 >> cp.log_lanes, L = 1 << cp.log_lanes;
+        const int vl = lane >> cp.log_lanes, l = lane & (L - 1);
+        for (int tile = gw; tile * V < cp.count; tile += nw) {
+            const int t = tile * V + vl;
+            const int i = t < cp.count ? s.ids[cp.first + t] : -1;
+            if (a.tris) {
+                const int o = s.tri_rec[cp.tile0 + tile], o1 = s.tri_rec[cp.tile0 + tile + 1];
+                const int q0 = i >= 0 ? a.tri_off[i] : 0, q1 = i >= 0 ? a.tri_off[i + 1] : 0;
+                for (int r = 0; o + 32 * r < o1; ++r) {
+                    int4 rv = make_int4(-2, 0, 0, 0);
+                    float4 rd = make_float4(0.f, 0.f, 0.f, 0.f), rm = rd;
+                    const int q = q0 + 2 * (r * L + l);
+                    if (q < q1) {
+                        const int tri = a.tri_adj[q], which = a.tri_adj[q + 1];
+                        const float mu = a.mats[3 * tri], lambda = a.mats[3 * tri + 1];
+                        if (!(mu <= 0.0f && lambda <= 0.0f)) {
+                            int v[3] = {a.tris[3 * tri], a.tris[3 * tri + 1], a.tris[3 * tri + 2]};
+                            rv = make_int4(which == 0 ? -1 : v[0], which == 1 ? -1 : v[1], which == 2 ? -1 : v[2], 0);
+                            const float* dm = a.poses + 4 * (size_t)tri;
+                            rd = make_float4(dm[0], dm[1], dm[2], dm[3]);
+                            rm = make_float4(a.areas[tri], mu, lambda, a.mats[3 * tri + 2]);
+                        }
+                    }
+                    s.rec.tri_v[o + 32 * r + lane] = rv;
+                    s.rec.tri_dm[o + 32 * r + lane] = rd;
+                    s.rec.tri_m[o + 32 * r + lane] = rm;
+                }
+            }
+            if (a.edges) {
+                const int o = s.hinge_rec[cp.tile0 + tile], o1 = s.hinge_rec[cp.tile0 + tile + 1];
+                const int q0 = i >= 0 ? a.edge_off[i] : 0, q1 = i >= 0 ? a.edge_off[i + 1] : 0;
+                for (int r = 0; o + 32 * r < o1; ++r) {
+                    int4 rv = make_int4(-2, 0, 0, 0);
+                    float4 rm = make_float4(0.f, 0.f, 0.f, 0.f);
+                    const int q = q0 + 2 * (r * L + l);
+                    if (q < q1) {
+                        const int e = a.edge_adj[q], which = a.edge_adj[q + 1];
+                        const float ks = a.bend[2 * e];
+                        const int* ev = a.edges + 4 * (size_t)e;
+                        if (!(ks <= 0.0f) && ev[0] >= 0 && ev[1] >= 0) {  // not a boundary edge
+                            rv = make_int4(which == 0 ? -1 : ev[0], which == 1 ? -1 : ev[1], which == 2 ? -1 : ev[2],
+                                           which == 3 ? -1 : ev[3]);
+                            rm = make_float4(a.rest_angle[e], a.rest_length[e], ks, a.bend[2 * e + 1]);
+                        }
+                    }
+                    s.rec.hinge_v[o + 32 * r + lane] = rv;
+                    s.rec.hinge_m[o + 32 * r + lane] = rm;
+                }
+            }
+        }
+    }
+    // What a warp reads of a tile that no sweep writes; fetched one tile ahead,
+    // across the barrier too, so only the neighbours' state is waited for.
+    struct Element {
+        int4 tv, hv;
+        float4 dm, tm, hm;
+    };
+    struct Tile {
+        int i, ot, ot1, oh, oh1;  // vertex, record ranges of this lane
+        V3 y;                     // inertia target
+        Element e;                // first round's records
+    };
+    auto fetch_element = [&](int ot, int ot1, int oh, int oh1) {
+        Element e;
+        e.tv = e.hv = make_int4(-2, 0, 0, 0);
+        e.dm = e.tm = e.hm = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (ot < ot1) {
+            e.tv = __ldcg(s.rec.tri_v + ot);
+            e.dm = __ldcg(s.rec.tri_dm + ot);
+            e.tm = __ldcg(s.rec.tri_m + ot);
+        }
+        if (oh < oh1) {
+            e.hv = __ldcg(s.rec.hinge_v + oh);
+            e.hm = __ldcg(s.rec.hinge_m + oh);
+        }
+        return e;
+    };
+    auto fetch_tile = [&](const ColorPlan& cp, int tile) {
+        Tile x;
+        const int V = 32 >> cp.log_lanes, t = tile * V + (lane >> cp.log_lanes);
+        x.i = -1;
+        x.ot = x.ot1 = x.oh = x.oh1 = 0;
+        x.y = v3(0.f, 0.f, 0.f);
+        if (tile * V < cp.count) {
+            if (t < cp.count) x.i = s.ids[cp.first + t];
+            if (a.tris) {
+                x.ot = s.tri_rec[cp.tile0 + tile] + lane;
+                x.ot1 = s.tri_rec[cp.tile0 + tile + 1];
+            }
+            if (a.edges) {
+                x.oh = s.hinge_rec[cp.tile0 + tile] + lane;
+                x.oh1 = s.hinge_rec[cp.tile0 + tile + 1];
+            }
+        }
+        x.e = fetch_element(x.ot, x.ot1, x.oh, x.oh1);
+        if (x.i >= 0 && (lane & ((1 << cp.log_lanes) - 1)) == 0) {
+            const float4 y = s.own[x.i].y;
+            x.y = v3(y.x, y.y, y.z);
+        }
+        return x;
+    };
+    if (!grid_sync()) return;
+    const long sweeps = (long)s.iterations * s.n_colors;
+    ColorPlan cp = s.colors[0];
+    Tile cur = fetch_tile(cp, gw);
+    int c = 0;
+    for (long sw = 0; sw < sweeps; ++sw) {
+        const int V = 32 >> cp.log_lanes, L = 1 << cp.log_lanes;
+        const int c_next = c + 1 < s.n_colors ? c + 1 : 0;
+        const ColorPlan cn = s.colors[c_next];
+        int tile = gw;
+        if (tile * V >= cp.count) cur = fetch_tile(cn, gw);  // none of this colour's
+        for (; tile * V < cp.count; tile += nw) {
+            const int i = cur.i;
+            float4 xm = make_float4(0.f, 0.f, 0.f, 0.f), qq = xm, dd = xm;
+            if (i >= 0) {
+                xm = s.state[i].xm;
+                qq = s.state[i].q;
+                if ((lane & (L - 1)) == 0) dd = s.own[i].d;
+            }
+            const V3 xi = v3(xm.x, xm.y, xm.z), qi = v3(qq.x, qq.y, qq.z);
+            const float m = xm.w;
+            const bool free = m != 0.0f;
+            V3 f = v3(0.f, 0.f, 0.f);
+            H6 h;
+            set_zero(h);
+            auto vert = [&](int j, V3& x, V3& p) {
+                x = xi;
+                p = qi;
+                if (j >= 0) {
+                    const float4 u = s.state[j].xm, w = s.state[j].q;
+                    x = v3(u.x, u.y, u.z);
+                    p = v3(w.x, w.y, w.z);
+                }
+            };
+            Element e = cur.e;
+            int ot = cur.ot, oh = cur.oh;
+            const int ot1 = cur.ot1, oh1 = cur.oh1;
+            while (ot < ot1 || oh < oh1) {
+                const bool tri = e.tv.x != -2 && free, hinge = e.hv.x != -2 && free;
+                V3 x0, x1, x2, p0, p1, p2, x[4], p[4];
+                if (tri) {
+                    vert(e.tv.x, x0, p0);
+                    vert(e.tv.y, x1, p1);
+                    vert(e.tv.z, x2, p2);
+                }
+                if (hinge) {
+                    vert(e.hv.x, x[0], p[0]);
+                    vert(e.hv.y, x[1], p[1]);
+                    vert(e.hv.z, x[2], p[2]);
+                    vert(e.hv.w, x[3], p[3]);
+                }
+                ot += 32;
+                oh += 32;
+                const Element nx = fetch_element(ot, ot1, oh, oh1);
+                if (tri) {
+                    const float dm[4] = {e.dm.x, e.dm.y, e.dm.z, e.dm.w};
+                    membrane(e.tv.x < 0 ? 0 : (e.tv.y < 0 ? 1 : 2), x0, x1, x2, p0, p1, p2, dm, e.tm.x, e.tm.y,
+                             e.tm.z, e.tm.w, dt, f, h);
+                }
+                if (hinge)
+                    bending(e.hv.x < 0 ? 0 : (e.hv.y < 0 ? 1 : (e.hv.z < 0 ? 2 : 3)), x, p, e.hm.x, e.hm.y, e.hm.z,
+                            e.hm.w, dt, f, h);
+                e = nx;
+            }
+            const V3 y = cur.y;
+            cur = (tile + nw) * V < cp.count ? fetch_tile(cp, tile + nw) : fetch_tile(cn, gw);
+            __syncwarp();
+            // the lanes' sums, fixed order
+            float acc[9] = {f.x, f.y, f.z, h.xx, h.xy, h.xz, h.yy, h.yz, h.zz};
+            for (int o = L >> 1; o > 0; o >>= 1)
+#pragma unroll
+                for (int q = 0; q < 9; ++q) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+            if (i >= 0 && free && (lane & (L - 1)) == 0) {
+                // inertia term, then the elements' sums; 3x3 Newton step
+                const float md = m * (1.0f / (dt * dt));
+                f = (y - xi) * md + v3(acc[0], acc[1], acc[2]);
+                h = H6{acc[3], acc[4], acc[5], acc[6], acc[7], acc[8]};
+                add_scaled_identity(h, md);
+                const float det = det6(h);
+                if (fabsf(det) > 1.0e-8f) {
+                    const V3 dn = v3(dd.x, dd.y, dd.z) + solve6(h, det, f);
+                    const V3 xn = qi + dn;
+                    s.state[i].xm = make_float4(xn.x, xn.y, xn.z, m);
+                    s.own[i].d = make_float4(dn.x, dn.y, dn.z, 0.f);
+                }
+            }
+        }
+        if (!grid_sync()) return;
+        cp = cn;
+        c = c_next;
+    }
+    for (int i = gt; i < a.n; i += gn) {
+        const float4 p = s.state[i].xm;
+        const V3 x = v3(p.x, p.y, p.z);
+        st(a.vel, i, (x - ld(a.pos, i)) * (1.0f / dt));
+        st(a.pos, i, x);
+    }
 }
 
 }  // namespace vbd
