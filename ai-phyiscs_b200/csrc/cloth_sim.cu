@@ -878,7 +878,7 @@ public:
         if (grid) *grid = used == 1 ? 0 : plan_.grid;
         if (block) *block = used == 1 ? kVecBlock : solver_block();
     }
-    int solver_block() const { return resident_ ? resident_warps_ * 32 : (tiled_ ? kTileThreads : pcg_block_); }
+    int solver_block() const { return resident_ ? resident_warps_ * 32 : (tiled_ ? tile_threads(tile_mode_) : pcg_block_); }
 
     // ---- autotuner (no counterpart in the reference) -------------------
     // Times the solver configurations that apply to the current system on
@@ -1965,16 +1965,22 @@ private:
         plan_coarse();
         const int ow = mode == 2 ? off_width() : 0;
         if (!coarse_on_) tile_max_blk_ = 1;
-        pers_smem_ = tile_smem(plan_.n_inst == 1 ? kTileWarps : plan_.max_slices_per_cta, plan_.max_inst_per_cta,
-                               coarse_stream_smem(), tile_max_blk_, plan_.max_slices_per_cta, max_halo, max_entries,
-                               ow).bytes;
         cudaFuncAttributes fa{};
         ck(cudaFuncGetAttributes(&fa, persistent_fn()), "cudaFuncGetAttributes(tiled)");
-        bool fits = pers_smem_ + fa.sharedSizeBytes <= (size_t)limit;
+        // a warp's stage holds as many blocks of a slice as there is room for
+        int stage = mode == 0 && !coarse_on_ ? std::min(6, topo_.max_width) : 0;
+        bool fits = false;
+        for (; stage >= 0 && !fits; --stage) {
+            pers_smem_ = tile_smem(plan_.n_inst == 1 ? tile_threads(mode) / 32 : plan_.max_slices_per_cta, plan_.max_inst_per_cta,
+                                   coarse_stream_smem(), tile_max_blk_, plan_.max_slices_per_cta, max_halo,
+                                   max_entries, ow, stage).bytes;
+            fits = pers_smem_ + fa.sharedSizeBytes <= (size_t)limit;
+            if (fits) break;
+        }
         if (fits)
             ck(cudaFuncSetAttribute(persistent_fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pers_smem_),
                "cudaFuncSetAttribute(tiled smem)");
-        if (fits && cluster) fits = cluster_fits(plan_.grid, kTileThreads);
+        if (fits && cluster) fits = cluster_fits(plan_.grid, tile_threads(mode));
         if (!fits) {
             tiled_ = cluster_ = false;
             coarse_on_ = false;
@@ -1998,6 +2004,7 @@ private:
         ta.max_entries = max_entries;
         ta.ow = ow;
         ta.max_blk = tile_max_blk_;
+        ta.stage = stage;
         d_tile_.upload(&ta, 1);
         return true;
     }

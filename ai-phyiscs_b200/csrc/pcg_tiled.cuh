@@ -13,6 +13,12 @@
 //     plain storage: 9 columns of one warp's 32 lanes per 32-row slice, 512
 //     columns, i.e. 7 slices per warp and up to 224 (7,168 rows) per SM;
 //   * x takes alpha p one iteration later, when p is at hand anyway;
+//   * the blocks of a warp's next slice are already on their way: each warp
+//     owns a stage in shared memory that the copy engine fills (cp.async.bulk)
+//     while the warp works on, across the barriers too, so the stream does not
+//     stop for the reductions (801 x 643: 25 -> 21 us per iteration; not with
+//     the coarse level, whose rows of A_c^-1 live in the L1 that the stages
+//     would take: 1024 x 1024 went from 96 to 117 ms with them);
 //   * only z of rows in another CTA's halo goes through global memory: the
 //     owner writes it with the update, every CTA forms the halo's p = z +
 //     beta p itself, with the arithmetic of the owner (identical values).
@@ -43,6 +49,10 @@ namespace chysx_b200 {
 
 constexpr int kTileThreads = 1024;
 constexpr int kTileWarps = kTileThreads / 32;
+// threads per CTA: 512 where the matrix lies in shared memory (a few slices
+// per CTA, the rest is synchronisation: the 61 x 47 garment 4.6 us per
+// iteration against 5.0 with 1024)
+__host__ __device__ constexpr int tile_threads(int mode) { return mode == 2 ? 512 : kTileThreads; }
 constexpr int kTileCols = 9;          // TMEM columns per slice: x, r, A p / z
 constexpr int kTileMaxSlices = 224;   // 7 per warp: 8 warps per lane quarter x 7 slices x 9 columns <= 512
 
@@ -58,6 +68,7 @@ struct TileArgs {
     int max_entries;                  // ELL entries of a CTA (MODE 2; else 0)
     int ow;                           // floats per block (MODE 2)
     int max_blk;                      // coarse blocks of a CTA
+    int stage;                        // blocks of a slice that a warp's stage holds (MODE 0; 0: no stages)
 };
 // Coarse values of one of the CTA's blocks, per phase and state: A_c^-1 R^T of
 // r (kCU), of the new r (kCN), of b and of r0 (start only).
@@ -68,10 +79,10 @@ static_assert(kCU == 0 && kCN == 12 && kInstCoarseW == 24, "the first two are th
 // slice offsets / masks / instances, halo rows and instances, p.
 __host__ __device__ inline size_t tile_align(size_t v) { return (v + 15) & ~static_cast<size_t>(15); }
 struct TileSmem {
-    size_t li, vbuf, blk, soff, mask, sli, hrow, hli, p, mat, diag, col, bytes;
+    size_t li, vbuf, blk, soff, mask, sli, hrow, hli, p, mat, diag, col, stage, bytes;
 };
 __host__ __device__ inline TileSmem tile_smem(int parts, int max_inst, size_t coarse_bytes, int max_blk,
-                                              int max_slices, int max_halo, int max_entries = 0, int ow = 0) {
+                                              int max_slices, int max_halo, int max_entries, int ow, int stage) {
     TileSmem s;
     s.li = (size_t)parts * kSlotW * sizeof(double);
     s.vbuf = tile_align(s.li + (size_t)max_inst * sizeof(LocalInst));
@@ -86,7 +97,8 @@ __host__ __device__ inline TileSmem tile_smem(int parts, int max_inst, size_t co
     // MODE 2: blocks, D' and M^-1 (192 floats each per slice), columns
     s.diag = s.mat + (size_t)max_entries * ow * sizeof(float);
     s.col = s.diag + (max_entries ? (size_t)384 * max_slices * sizeof(float) : 0);
-    s.bytes = s.col + (size_t)max_entries * sizeof(unsigned short);
+    s.stage = (s.col + (size_t)max_entries * sizeof(unsigned short) + 127) & ~static_cast<size_t>(127);
+    s.bytes = s.stage + (size_t)stage * (kTileThreads / 32) * 192 * sizeof(float);
     return s;
 }
 
@@ -165,14 +177,40 @@ __device__ __forceinline__ int ld_na(const unsigned short* p) {
     return v;
 }
 
+// ---- a warp's stage: one bulk copy at a time, completion on its mbarrier ----
+__device__ __forceinline__ void stage_fetch(uint32_t dst, const float* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+// waits for the copy of phase `parity`, at most kBarrierTimeoutNs
+__device__ __forceinline__ bool stage_wait(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    unsigned long long t0 = 0;
+    for (unsigned spins = 0;; ++spins) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.b32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (done) return true;
+        if (spins == 0) t0 = global_ns();
+        else if ((spins & 63u) == 0 && global_ns() - t0 > kBarrierTimeoutNs) return false;
+    }
+}
+
 template <bool ONE, int CO, int MODE = 0, bool CLU = false>
-__global__ void __launch_bounds__(kTileThreads, 1)
+__global__ void __launch_bounds__(tile_threads(MODE), 1)
 pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const TileArgs* ta, void*) {
     constexpr int SYNC = 0;  // slot_set: two sets by parity
-    constexpr int BLOCK = kTileThreads;
+    constexpr int BLOCK = tile_threads(MODE), kW = BLOCK / 32;
     extern __shared__ __align__(16) unsigned char s_raw[];
     __shared__ int s_flag, s_exit;
     __shared__ uint32_t s_tmem;
+    constexpr bool STG = MODE == 0 && CO == 0;
+    __shared__ __align__(8) uint64_t s_mbar[STG ? kW : 1];
     __shared__ float s_tmp[CO ? BLOCK : 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int s0 = bp.cta_slice[blockIdx.x], s1 = bp.cta_slice[blockIdx.x + 1], ns = s1 - s0;
@@ -186,8 +224,8 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
         CO == 2 && !warm && bp.cg != nullptr && bp.cg->on && bp.cg->batched && *(volatile int*)bp.cg->fail == 0;
     const bool any_c = coarse || coarse_b;
     const size_t cbytes = CO == 1 && bp.cg ? (size_t)bp.cg->m * sizeof(float) + 16 : 0;
-    const TileSmem lay = tile_smem(ONE ? kTileWarps : T.max_slices, bp.max_inst_per_cta, cbytes, T.max_blk,
-                                   T.max_slices, T.max_halo, T.max_entries, T.ow);
+    const TileSmem lay = tile_smem(ONE ? kW : T.max_slices, bp.max_inst_per_cta, cbytes, T.max_blk,
+                                   T.max_slices, T.max_halo, T.max_entries, T.ow, T.stage);
     __shared__ double s_cslot[CLU ? 2 : 1][kClusterMax][CLU ? kSlotW : 1];
     double* spart = reinterpret_cast<double*>(s_raw);
     LocalInst* li = reinterpret_cast<LocalInst*>(s_raw + lay.li);
@@ -218,6 +256,10 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
         s_flag = 0;
         s_exit = 0;
     }
+    if (STG && lane == 0)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n\tfence.mbarrier_init.release.cluster;" ::"r"(
+                         static_cast<uint32_t>(__cvta_generic_to_shared(&s_mbar[STG ? warp : 0])))
+                     : "memory");
     init_local(bp, li, s0, s1, il0, il1);
     for (int k = tid; k <= ns; k += BLOCK) s_off[k] = t.slice_off[s0 + k];
     for (int k = tid; k < ns; k += BLOCK) {
@@ -280,15 +322,46 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (ONE && tid == 0) {  // the partials are per warp
         li[0].seg_lo = 0;
-        li[0].seg_hi = kTileWarps;
+        li[0].seg_hi = kW;
     }
     if (any_c)
-        for (int q = warp; q < co.nbl; q += kTileWarps)
+        for (int q = warp; q < co.nbl; q += kW)
             for (int k = s_bk0[q] + lane; k < s_bk0[q + 1]; k += 32) s_slb[k] = (unsigned short)q;
     __syncthreads();
+    // The warp's stage: blocks of slice `staged` (-1: none under way)
+    float* s_stage = reinterpret_cast<float*>(s_raw + lay.stage) + (size_t)warp * T.stage * 192;
+    const uint32_t mbar = static_cast<uint32_t>(__cvta_generic_to_shared(&s_mbar[STG ? warp : 0]));
+    const int n_stage = STG ? T.stage : 0;
+    int staged = -1;
+    uint32_t stage_par = 0;
+    auto stage_blocks = [&](int k) { return min((s_off[k + 1] - s_off[k]) >> 5, n_stage); };
+    auto stage_slice = [&](int k) {  // the warp's reads of the stage are done (__syncwarp)
+        const int c = stage_blocks(k);
+        __syncwarp();
+        if (c == 0) return;
+        staged = k;
+        if (lane == 0)
+            stage_fetch(static_cast<uint32_t>(__cvta_generic_to_shared(s_stage)), t.val + (size_t)s_off[k] * 6,
+                        (uint32_t)c * 768u, mbar);
+    };
+    auto stage_done = [&]() {
+        if (staged < 0) return;
+        staged = -1;
+        if (!stage_wait(mbar, stage_par)) {
+            s_flag = 1;
+            *(volatile int*)&bp.bar->error = 1;
+        }
+        stage_par ^= 1u;
+    };
+    // the next slice of this warp whose instance is not done
+    auto next_k = [&](int k) {
+        k += kW;
+        while (!ONE && k < ns && li[s_sli[k]].done) k += kW;
+        return k;
+    };
     // tensor memory of the warp's j-th slice
     const uint32_t tm0 = s_tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(kTileCols * (warp >> 2));
-    constexpr uint32_t kTmStep = kTileCols * (kTileWarps / 4);
+    constexpr uint32_t kTmStep = kTileCols * (kW / 4);
     bool ok = true;
     auto no_step = [](LocalInst&, const double*) {};
     auto cw = [&](int i) { return __ldg(co.w + i); };  // four fields per block always
@@ -310,7 +383,7 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
         const int P = min(8, max(1, BLOCK / nv));
         for (int x = tid; x < nv * P; x += BLOCK) {
             const int h = x % P, qu = x / P, q = qu / 12, u = qu - 12 * q;
-            const int lo = ONE ? 0 : s_bk0[q], hi = ONE ? kTileWarps : s_bk0[q + 1];
+            const int lo = ONE ? 0 : s_bk0[q], hi = ONE ? kW : s_bk0[q + 1];
             float acc = 0.0f;
             for (int sl = lo + h; sl < hi; sl += P) acc += slice_cpart(spart, sl)[u];
             if (P > 1) s_tmp[x] = acc;
@@ -356,7 +429,7 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
             constexpr int rows = 12, parts = 2;
             const int m4 = c_m / 4;
             const float4* A = reinterpret_cast<const float4*>(co.ainv + (size_t)(12 * (co.B0 / c_g)) * c_m);
-            for (int x = warp; x < rows * parts; x += kTileWarps) {
+            for (int x = warp; x < rows * parts; x += kW) {
                 const int r = x / parts, h = x - r * parts;
                 const float4* a4 = A + (size_t)r * m4;
                 float acc = 0.0f;
@@ -380,7 +453,7 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
         if (CO == 2) {
             // a warp per block: the instance's values (at most 160, five per
             // lane) times the block's 12 rows of the instance's inverse
-            for (int q = warp; q < nbl; q += kTileWarps) {
+            for (int q = warp; q < nbl; q += kW) {
                 const LocalInst& L = li[s_binst[q]];
                 if (L.done) continue;
                 const int I0 = co.inst_blk[L.b], m = 12 * (co.inst_blk[L.b + 1] - I0);
@@ -417,7 +490,7 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
         if constexpr (CLU) {
             cluster_phase<NV>(spart, li, 1, s_cslot, set, step);
         } else {
-            for (int q = warp; q < nloc; q += kTileWarps) {
+            for (int q = warp; q < nloc; q += kW) {
                 const LocalInst& L = li[q];
                 if (L.done) continue;
                 double acc[NV];
@@ -440,7 +513,7 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
             }
             __syncthreads();
             if (!s_flag) {
-                for (int q = warp; q < nloc; q += kTileWarps) {
+                for (int q = warp; q < nloc; q += kW) {
                     LocalInst& L = li[q];
                     if (L.done) continue;
                     constexpr int KP = 5;  // one pass covers 160 CTAs
@@ -518,12 +591,43 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
             return acc;
         }
         const float* vb = t.val + (size_t)so * 6 + lane;
-        if (w == 6) {
+        if (!STG || n_stage == 0) {
+            if (w == 6) {
 #pragma unroll
-            for (int e = 0; e < 6; ++e) acc = acc + mul(ld6_na(vb + e * 192), ldp(ld_na(lc + e * 32)) - pi);
-        } else {
-            for (int e = 0; e < w; ++e) acc = acc + mul(ld6_na(vb + e * 192), ldp(ld_na(lc + e * 32)) - pi);
+                for (int e = 0; e < 6; ++e) acc = acc + mul(ld6_na(vb + e * 192), ldp(ld_na(lc + e * 32)) - pi);
+            } else {
+                for (int e = 0; e < w; ++e) acc = acc + mul(ld6_na(vb + e * 192), ldp(ld_na(lc + e * 32)) - pi);
+            }
+            return acc;
         }
+        if (staged != k) {  // first use, or another slice's instance has finished since
+            stage_done();
+            stage_slice(k);
+        }
+        const int c = min(w, n_stage);
+        if (w == 6) {
+            int col[6];
+#pragma unroll
+            for (int e = 0; e < 6; ++e) col[e] = ld_na(lc + e * 32);
+            stage_done();
+            if (c == 6) {
+#pragma unroll
+                for (int e = 0; e < 6; ++e) acc = acc + mul(ld6(s_stage + e * 192 + lane), ldp(col[e]) - pi);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 6; ++e)
+                    acc = acc + mul(e < c ? ld6(s_stage + e * 192 + lane) : ld6_na(vb + e * 192), ldp(col[e]) - pi);
+            }
+        } else {
+            stage_done();
+            for (int e = 0; e < w; ++e)
+                acc = acc + mul(e < c ? ld6(s_stage + e * 192 + lane) : ld6_na(vb + e * 192),
+                                ldp(ld_na(lc + e * 32)) - pi);
+        }
+        // the warp's next slice, of the next iteration after the last one
+        int kn = next_k(k);
+        if (kn >= ns) kn = next_k(warp - kW);
+        if (kn < ns) stage_slice(kn);
         return acc;
     };
     // per-thread sums of a phase: added over the warp once (ONE) or per slice
@@ -554,7 +658,7 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
         Sums sm;
         zero_sums(sm);
         uint32_t tm = tm0;
-        for (int k = warp; k < ns; k += kTileWarps, tm += kTmStep) {
+        for (int k = warp; k < ns; k += kW, tm += kTmStep) {
             const int i = (s0 + k) * 32 + lane;
             const float3 a = get(tm, i);
             const float4 w4 = i < t.n ? cw(i) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -587,14 +691,14 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
     }
     if (ok && warm) {
         uint32_t tm = tm0;
-        for (int k = warp; k < ns; k += kTileWarps, tm += kTmStep) {
+        for (int k = warp; k < ns; k += kW, tm += kTmStep) {
             const int i = (s0 + k) * 32 + lane;
             stp(k * 32 + lane, i < t.n ? xyz(v.x[i]) : f3(0.f, 0.f, 0.f));
         }
         for (int h = tid; h < nh; h += BLOCK) stp(nown + h, xyz(ldcg4(v.x + s_hrow[h])));
         __syncthreads();
         tm = tm0;
-        for (int k = warp; k < ns; k += kTileWarps, tm += kTmStep) {
+        for (int k = warp; k < ns; k += kW, tm += kTmStep) {
             const int i = (s0 + k) * 32 + lane;
             const float3 ax = row_product(k, ldp(k * 32 + lane));
             tm_st3(tm + kTmR, load_b(0u, i) - ax);
@@ -620,7 +724,7 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
 #pragma unroll
         for (int u = 0; u < kStartW; ++u) tot[u] = 0.0;
         uint32_t tm = tm0;
-        for (int k = warp; k < ns; k += kTileWarps, tm += kTmStep) {
+        for (int k = warp; k < ns; k += kW, tm += kTmStep) {
             const int i = (s0 + k) * 32 + lane;
             const S6 Mi = load_minv(s0 + k, i);
             const float4 w4 = any_c && i < t.n ? cw(i) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -667,7 +771,7 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
     if (ok && warm) {
         // the scaled guess, or the zero guess where the instance fell back
         uint32_t tm = tm0;
-        for (int k = warp; k < ns; k += kTileWarps, tm += kTmStep) {
+        for (int k = warp; k < ns; k += kW, tm += kTmStep) {
             const int i = (s0 + k) * 32 + lane;
             const S6 Mi = load_minv(s0 + k, i);
             const float4 w4 = any_c && i < t.n ? cw(i) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -689,7 +793,7 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
         }
         tm_wait_st();
         // a data-free phase orders the new z before any halo read
-        for (int q = tid; q < (ONE ? kTileWarps : ns); q += BLOCK) spart[q * kSlotW] = 0.0;
+        for (int q = tid; q < (ONE ? kW : ns); q += BLOCK) spart[q * kSlotW] = 0.0;
         __syncthreads();
         phase(N1{}, false, no_step);
         ok = s_flag == 0;
@@ -711,7 +815,7 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
         // p = z + beta p of the own rows and, from the published z, of the
         // halo; x takes the previous iteration's alpha p
         uint32_t tm = tm0;
-        for (int k = warp; k < ns; k += kTileWarps, tm += kTmStep) {
+        for (int k = warp; k < ns; k += kW, tm += kTmStep) {
             const LocalInst& L = li[inst_of(k)];
             if (L.done) continue;
             float3 z, x = f3(0.f, 0.f, 0.f);
@@ -740,12 +844,19 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
             stp(nown + h, z);
         }
         __syncthreads();
-        // A p, sigma = p.A p (and the restriction of A p)
+        // A p, sigma = p.A p (and the restriction of A p); M^-1 of the update's
+        // first slice comes in behind the barrier (registers permitting)
+        S6 mi_n{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        auto fetch_diag = [&](int k) {
+            if (k >= ns) return;
+            const int i = (s0 + k) * 32 + lane;
+            mi_n = load_minv(s0 + k, i);
+        };
         {
             Sums sm;
             zero_sums(sm);
             uint32_t tm = tm0;
-            for (int k = warp; k < ns; k += kTileWarps, tm += kTmStep) {
+            for (int k = warp; k < ns; k += kW, tm += kTmStep) {
                 const LocalInst& L = li[inst_of(k)];
                 if (L.done) continue;
                 const int i = (s0 + k) * 32 + lane;
@@ -770,6 +881,7 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
             }
             tm_wait_st();
         }
+        if (STG) fetch_diag(next_k(warp - kW));
         __syncthreads();
         if (any_c) publish_coarse();
         const int set1 = slot_set(ph);
@@ -785,19 +897,21 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
         {
             Sums sm;
             zero_sums(sm);
-            uint32_t tm = tm0;
-            for (int k = warp; k < ns; k += kTileWarps, tm += kTmStep) {
-                const int q = inst_of(k);
-                const LocalInst& L = li[q];
-                if (L.done) continue;
+            int kn = 0;
+            for (int k = next_k(warp - kW); k < ns; k = kn) {
+                const LocalInst& L = li[inst_of(k)];
+                const uint32_t tm = tm0 + kTmStep * (uint32_t)(k / kW);
                 const int i = (s0 + k) * 32 + lane;
                 float3 r, ap;
                 __syncwarp();
                 tm_ld4(tm + kTmR, r.x, r.y, r.z, ap.x);
                 tm_ld2(tm + kTmQ + 1, ap.y, ap.z);
-                const S6 Mi = load_minv(s0 + k, i);
+                kn = next_k(k);
+                if (!STG) fetch_diag(k);
+                const S6 Mi = mi_n;
                 const float4 w4 = any_c && i < t.n ? cw(i) : make_float4(0.f, 0.f, 0.f, 0.f);
                 const float al = L.alpha;
+                if (STG) fetch_diag(kn);
                 tm_wait_ld(r, ap);
                 const float3 rn = f3(fmaf(-al, ap.x, r.x), fmaf(-al, ap.y, r.y), fmaf(-al, ap.z, r.z));
                 float3 zn = mul(Mi, rn);
@@ -843,7 +957,7 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
     }
     // x with the last iteration's alpha p
     uint32_t tm = tm0;
-    for (int k = warp; k < ns; k += kTileWarps, tm += kTmStep) {
+    for (int k = warp; k < ns; k += kW, tm += kTmStep) {
         const LocalInst& L = li[inst_of(k)];
         const int i = (s0 + k) * 32 + lane;
         float3 x, d = f3(0.f, 0.f, 0.f);
@@ -856,6 +970,7 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
         if (i < t.n) v.x[i] = f4(x);
     }
     if (!ok) instances_fail(bp, li, nloc);
+    stage_done();  // the copy for the iteration that does not come
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
