@@ -1498,6 +1498,8 @@ private:
             if (W == 16 && plan_cluster()) return true;
             plan_coarse();
             pers_smem_ = (size_t)W * kSlotW * sizeof(double) + (size_t)plan_.max_inst_per_cta * sizeof(LocalInst);
+            if (pc_kind_ >= 1 && sync_mode_ == 0)  // the local preconditioner's columns
+                pers_smem_ += (size_t)(topo_.max_width <= 6 ? 6 : kResidentMaxWidth) * W * 32 * sizeof(int);
             if (coarse_on_)  // the coarse block's rows of A_c^-1, a phase's block values and its staged slots
                 pers_smem_ += ((size_t)9 * coarse_nq_ * coarse_nq_ * coarse_nb_ + (size_t)3 * coarse_nq_ * coarse_nb_) *
                                   sizeof(float) + 16 + (size_t)plan_.inst_slot.back() * kSlotW * sizeof(double) + 16;
@@ -2080,7 +2082,10 @@ private:
             return;
         }
         const size_t li_bytes = (size_t)plan_.max_inst_per_cta * sizeof(LocalInst);
-        size_t need = resident_ ? (size_t)resident_warps_ * kSlotW * sizeof(double) + li_bytes
+        const size_t cols = resident_ && pc_kind_ >= 1 && sync_mode_ == 0
+                                ? (size_t)(topo_.max_width <= 6 ? 6 : kResidentMaxWidth) * resident_warps_ * 32 * sizeof(int)
+                                : 0;
+        size_t need = resident_ ? (size_t)resident_warps_ * kSlotW * sizeof(double) + cols + li_bytes
                                 : (size_t)plan_.max_slices_per_cta * kSlotW * sizeof(double) + li_bytes;
         if (!resident_) need += coarse_stream_smem();
         if (pers_smem_ < need || (resident_ && plan_.max_slices_per_cta > resident_warps_) ||

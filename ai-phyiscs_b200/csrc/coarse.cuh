@@ -232,15 +232,16 @@ __global__ void __launch_bounds__(288) coarse_assemble_kernel(DevTopo t, CoarseA
 // (m_b = U x blocks <= U kBatchMaxBlocks) from their block rows, adding the
 // assembly's splits in order and rounding once to FP32 (the stored A_c),
 // scales by S = diag^-1/2, shifts by ca.shift I and inverts by Gauss-Jordan
-// without pivoting in FP64 shared memory (per pivot the pivot row and column
-// are copied aside, then every entry updated: two CTA barriers per pivot);
+// without pivoting in FP64 shared memory, two pivots a step (the pivot rows
+// and columns are copied aside, then every entry updated: two CTA barriers
+// and one division per step; m_b is a multiple of 12);
 // an unknown whose field has zero weight on its whole block gets an identity
 // row.  Output S W S (FP32) into ca.ainv + ca.inst_aoff[b]; a non-positive
 // pivot sets ca.fail (the level is then off in the step's solve).  Dynamic
 // shared memory: batched_invert_smem(max m_b) bytes.
 constexpr int kBatchInvThreads = 256;
 __host__ __device__ constexpr size_t batched_invert_smem(int m) {
-    return ((size_t)m * (m + 1) + 3 * (size_t)m) * sizeof(double);
+    return ((size_t)m * (m + 1) + 5 * (size_t)m) * sizeof(double);
 }
 __global__ void __launch_bounds__(kBatchInvThreads) coarse_invert_batched_kernel(CoarseArgs ca) {
     extern __shared__ double inv_s[];
@@ -248,8 +249,8 @@ __global__ void __launch_bounds__(kBatchInvThreads) coarse_invert_batched_kernel
     const int B0 = ca.inst_blk[b], nbk = ca.inst_blk[b + 1] - B0, m = U * nbk, ld = m + 1;
     double* a = inv_s;
     double* prow = a + (size_t)m * ld;
-    double* pcol = prow + m;
-    double* s_sc = pcol + m;
+    double* pcol = prow + 2 * m;
+    double* s_sc = pcol + 2 * m;
     const size_t total = (size_t)ca.nb * mn * U * U;
     for (int x = tid; x < m * ld; x += kBatchInvThreads) a[x] = 0.0;
     __syncthreads();
@@ -279,23 +280,33 @@ __global__ void __launch_bounds__(kBatchInvThreads) coarse_invert_batched_kernel
     }
     __syncthreads();
     bool bad = false;
-    for (int k = 0; k < m; ++k) {
-        const double p = a[(size_t)k * ld + k];
-        const bool good = p > 1.0e-12;
+    for (int k = 0; k < m; k += 2) {
+        const double pa = a[(size_t)k * ld + k], pb = a[(size_t)k * ld + k + 1], pc = a[(size_t)(k + 1) * ld + k],
+                     pd = a[(size_t)(k + 1) * ld + k + 1];
+        const double det = fma(pa, pd, -pb * pc);
+        const bool good = pa > 1.0e-12 && det > 1.0e-12 * pa;  // both pivots, pa and det / pa
         bad = bad || !good;
-        const double ip = good ? 1.0 / p : 0.0;
+        const double id = good ? 1.0 / det : 0.0;
+        const double i00 = pd * id, i01 = -pb * id, i10 = -pc * id, i11 = pa * id;
+        // rows k, k + 1 times the pivot block's inverse (its columns in columns
+        // k, k + 1) and the two pivot columns, aside
         for (int x = tid; x < m; x += kBatchInvThreads) {
-            prow[x] = a[(size_t)k * ld + x];
+            const bool piv = (x & ~1) == k;
+            const double c0 = piv ? (x == k ? 1.0 : 0.0) : a[(size_t)k * ld + x];
+            const double c1 = piv ? (x == k ? 0.0 : 1.0) : a[(size_t)(k + 1) * ld + x];
+            prow[x] = fma(i00, c0, i01 * c1);
+            prow[m + x] = fma(i10, c0, i11 * c1);
             pcol[x] = a[(size_t)x * ld + k];
+            pcol[m + x] = a[(size_t)x * ld + k + 1];
         }
         __syncthreads();
-        // row k: (j == k ? 1 : a_kj) / p; the others subtract a_ik times it
         // (warp w takes rows w, w + 8, ..., lane l columns l, l + 32, ...)
         for (int j = tid & 31; j < m; j += 32) {
-            const double rk = (j == k ? 1.0 : prow[j]) * ip;
+            const bool piv = (j & ~1) == k;
+            const double r0 = prow[j], r1 = prow[m + j];
             for (int i = tid >> 5; i < m; i += kBatchInvThreads / 32) {
                 double& v = a[(size_t)i * ld + j];
-                v = i == k ? rk : fma(-pcol[i], rk, j == k ? 0.0 : v);
+                v = i == k ? r0 : (i == k + 1 ? r1 : fma(-pcol[i], r0, fma(-pcol[m + i], r1, piv ? 0.0 : v)));
             }
         }
         __syncthreads();
@@ -428,29 +439,43 @@ __global__ void __launch_bounds__(kCoarseInvertThreads) coarse_invert_kernel(Coa
             break;
         }
         // P1: T = W_KK^-1 by Gauss-Jordan in shared memory (the last CTA,
-        // the others being busy with P4 above): every pivot step reads the
-        // tile of the previous step and writes the other of two buffers, so
-        // one CTA barrier per pivot; every thread forms 1 / pivot itself
+        // the others being busy with P4 above), two pivots a step: the chain
+        // of a step is its division, so a 2 x 2 pivot block (one division, by
+        // its determinant) halves it.  Every step reads the tile of the
+        // previous one and writes the other of two buffers, one CTA barrier
+        // per step; every thread inverts the pivot block itself.  The
+        // kernel, one pivot a step -> two: 768 unknowns 579 -> 530 us, 384
+        // unknowns 129 -> 110 us.
         if (blockIdx.x == gridDim.x - 1) {
             ld_tile(sa, tile_at(K, K));
             __syncthreads();
             double(*cur)[kInvTile + 1] = sa;
             double(*nxt)[kInvTile + 1] = sc_;
             bool bad = false;
-            for (int k = 0; k < kInvTile; ++k) {
-                const double p = cur[k][k];
-                const bool good = p > 1.0e-12;
+            for (int k = 0; k < kInvTile; k += 2) {
+                const double pa = cur[k][k], pb = cur[k][k + 1], pc = cur[k + 1][k], pd = cur[k + 1][k + 1];
+                const double det = fma(pa, pd, -pb * pc);
+                // both pivots of the elimination, pa and det / pa, positive
+                const bool good = pa > 1.0e-12 && det > 1.0e-12 * pa;
                 bad = bad || !good;
-                const double ip = good ? 1.0 / p : 0.0;
+                const double id = good ? 1.0 / det : 0.0;
+                const double i00 = pd * id, i01 = -pb * id, i10 = -pc * id, i11 = pa * id;
                 // the thread's outputs (tid / 32 + j * R, tid % 32), as in tile_mul;
-                // row k: (q == k ? 1 : a_kq) / p; the others subtract a_rk times it
+                // rows k, k + 1: the block's inverse times their entries (its
+                // columns in columns k, k + 1); the others subtract their two
+                // pivot-column entries times those rows
                 constexpr int R = kCoarseInvertThreads / kInvTile;
                 const int r0 = tid / kInvTile, q = tid % kInvTile;
-                const double rk = (q == k ? 1.0 : cur[k][q]) * ip;
+                const bool piv = (q & ~1) == k;
+                const double c0 = piv ? (q == k ? 1.0 : 0.0) : cur[k][q], c1 = piv ? (q == k ? 0.0 : 1.0) : cur[k + 1][q];
+                const double rk0 = fma(i00, c0, i01 * c1), rk1 = fma(i10, c0, i11 * c1);
 #pragma unroll
                 for (int j = 0; j < kTileOut; ++j) {
                     const int r = r0 + j * R;
-                    nxt[r][q] = r == k ? rk : fma(-cur[r][k], rk, q == k ? 0.0 : cur[r][q]);
+                    nxt[r][q] = r == k ? rk0
+                                       : (r == k + 1 ? rk1
+                                                     : fma(-cur[r][k], rk0,
+                                                           fma(-cur[r][k + 1], rk1, piv ? 0.0 : cur[r][q])));
                 }
                 __syncthreads();
                 double(*t)[kInvTile + 1] = cur;

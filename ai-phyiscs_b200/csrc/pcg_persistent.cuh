@@ -1591,7 +1591,8 @@ pcg_resident_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, ZP
     __shared__ float4 s_z[W * 32], s_p[2][W * 32];
     // CTA-local preconditioner: exchange buffers, block sums, Chebyshev
     // constants (theta, 1/theta, sigma, 2/delta) of this CTA's block
-    __shared__ float4 s_d[PC ? 2 : 1][PC ? W * 32 : 1];
+    // (entry W * 32 stays zero: it stands for columns outside the CTA)
+    __shared__ float4 s_d[PC ? 2 : 1][PC ? W * 32 + 1 : 1];
     __shared__ double s_bsum[PC ? W : 1];
     __shared__ float s_cheb[4];
     __shared__ float2 s_ccoef[PC ? 64 : 1];  // per term m of the polynomial: (rn rho, rn 2/delta)
@@ -1604,7 +1605,8 @@ pcg_resident_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, ZP
     const int nloc = il1 - il0 + 1;
     const int row0 = s0 * 32, nrows = (s1 - s0) * 32;  // the CTA's rows
     double* spart = s_mem;  // [W * kSlotW]
-    LocalInst* li = reinterpret_cast<LocalInst*>(s_mem + (size_t)W * kSlotW);
+    // (the local preconditioner's build keeps its columns between the two)
+    LocalInst* li = reinterpret_cast<LocalInst*>(s_mem + (size_t)W * kSlotW + (PC ? MAXW * W * 16 : 0));
     unsigned target = 0;
     int ph = 0;  // reduction phase (SYNC = 1 slot set ph % 3)
     if (threadIdx.x == 0) {
@@ -1628,12 +1630,14 @@ pcg_resident_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, ZP
     // difference form D'_i p_i + sum_k B_k (p_j - p_i)
     S6 D{0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, Mi{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     S6 B[MAXW];
-    // column indices: registers, or shared memory in the slot-polling build
-    // (its waits need the registers)
-    int cols_r[SYNC == 1 ? 1 : MAXW];
-    __shared__ int s_cols[SYNC == 1 ? MAXW * W * 32 : 1];
+    // column indices: registers, or shared memory in the builds that are
+    // short of them (the slot-polling waits, the local preconditioner)
+    constexpr bool kColsShared = SYNC == 1 || PC;
+    int cols_r[kColsShared ? 1 : MAXW];
+    __shared__ int s_cols1[SYNC == 1 ? MAXW * W * 32 : 1];
+    int* s_cols = PC ? reinterpret_cast<int*>(s_mem + (size_t)W * kSlotW) : s_cols1;
     auto col_at = [&](int k) -> int & {
-        return SYNC == 1 ? s_cols[k * W * 32 + threadIdx.x] : cols_r[SYNC == 1 ? 0 : k];
+        return kColsShared ? s_cols[k * W * 32 + threadIdx.x] : cols_r[kColsShared ? 0 : k];
     };
     // cluster mode: every CTA's partial sums of a phase, two sets by parity
     __shared__ double s_cslot[SYNC == 2 ? 2 : 1][kClusterMax][SYNC == 2 ? kSlotW : 1];
@@ -1658,6 +1662,22 @@ pcg_resident_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, ZP
             }
         }
     }
+    // the columns as entries of the CTA's exchange buffers, two to a register
+    unsigned lcol[PC ? (MAXW + 1) / 2 : 1];
+    if (PC) {
+#pragma unroll
+        for (int k = 0; k < (MAXW + 1) / 2; ++k) {
+            unsigned e[2] = {(unsigned)(W * 32), (unsigned)(W * 32)};
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                if (2 * k + h < MAXW) {
+                    const unsigned lr = (unsigned)(col_at(2 * k + h) - row0);
+                    if (lr < (unsigned)nrows) e[h] = lr;
+                }
+            lcol[PC ? k : 0] = e[0] | e[1] << 16;
+        }
+        if (threadIdx.x < 2) s_d[PC ? threadIdx.x : 0][PC ? W * 32 : 0] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     __syncthreads();  // init_local
 
     // ---- CTA-local Chebyshev preconditioner (PC) ---------------------------
@@ -1670,12 +1690,11 @@ pcg_resident_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, ZP
     // blocks still enter the row's implied diagonal.
     auto local_spmv = [&](const float4* buf, float3 in) {
         float3 acc = mul(D, in);
+        // unused entries have zero blocks and the row itself as column: no test
 #pragma unroll
         for (int k = 0; k < MAXW; ++k) {
-            if (k >= w) continue;
-            const int lr = col_at(k) - row0;
-            const float3 nb = (unsigned)lr < (unsigned)nrows ? xyz(buf[lr]) : f3(0.f, 0.f, 0.f);
-            acc = acc + mul(B[k], nb - in);
+            const unsigned lr = k & 1 ? lcol[PC ? k >> 1 : 0] >> 16 : lcol[PC ? k >> 1 : 0] & 0xFFFFu;
+            acc = acc + mul(B[k], xyz(buf[lr]) - in);
         }
         return acc;
     };
@@ -1762,21 +1781,41 @@ pcg_resident_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, ZP
     // quad.  Warps 1..3 form this block of A_c^-1 R^T v during the phases.
     constexpr bool kCoarse = PC == 2;
     const bool coarse = kCoarse && bp.cg != nullptr && bp.cg->on && *(volatile int*)bp.cg->fail == 0;
-    const CoarseRegs creg = coarse_regs(bp, coarse);
-    const int c_U = creg.U, c_nq = creg.nq, c_g = creg.G, c_m = creg.m;
-    float* c_ainv = reinterpret_cast<float*>(li + bp.max_inst_per_cta);
-    // a phase's coarse block values ([m]) behind c_ainv, then its staged
-    // slot set ([n_slots][kSlotW] doubles), each 16-byte aligned
-    float* c_stage = reinterpret_cast<float*>(
-        (reinterpret_cast<uintptr_t>(c_ainv + (coarse ? c_U * c_m : 0)) + 15) & ~static_cast<uintptr_t>(15));
-    double* c_slots = reinterpret_cast<double*>(
-        (reinterpret_cast<uintptr_t>(c_stage + (coarse ? c_m : 0)) + 15) & ~static_cast<uintptr_t>(15));
+    // its parameters and places in shared memory too (registers are short):
+    // a phase's coarse block values ([m]) behind the rows of A_c^-1, then its
+    // staged slot set ([n_slots][kSlotW] doubles), each 16-byte aligned
+    __shared__ struct {
+        float *ainv, *stage;
+        double* slots;
+        const float* src;
+        const float4* w;
+        int U, nq, g, m;
+    } co;
+    if (kCoarse && threadIdx.x == 0) {
+        const CoarseRegs creg = coarse_regs(bp, coarse);
+        co.U = creg.U;
+        co.nq = creg.nq;
+        co.g = creg.G;
+        co.m = creg.m;
+        co.w = creg.w;
+        const int um = coarse ? creg.U * creg.m : 0;
+        co.src = creg.ainv + (size_t)(blockIdx.x / creg.G) * um;
+        co.ainv = reinterpret_cast<float*>(li + bp.max_inst_per_cta);
+        co.stage = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(co.ainv + um) + 15) & ~static_cast<uintptr_t>(15));
+        co.slots = reinterpret_cast<double*>(
+            (reinterpret_cast<uintptr_t>(co.stage + (coarse ? creg.m : 0)) + 15) & ~static_cast<uintptr_t>(15));
+    }
+    if (kCoarse) __syncthreads();
+    const int &c_U = co.U, &c_nq = co.nq, &c_g = co.g, &c_m = co.m;
+    float *&c_ainv = co.ainv, *&c_stage = co.stage;
+    double*& c_slots = co.slots;
     float4 c_w = make_float4(0.f, 0.f, 0.f, 0.f);
     if (coarse) {
-        const int m = c_m;
-        const float* src = creg.ainv + (size_t)(blockIdx.x / c_g) * c_U * m;
-        for (int q = threadIdx.x; q < c_U * m; q += blockDim.x) c_ainv[q] = src[q];
-        if (c_nq == 4 && row) c_w = creg.w[i];
+        const int um = c_U * c_m;
+        const float* src = co.src;
+        float* dst = c_ainv;
+        for (int q = threadIdx.x; q < um; q += blockDim.x) dst[q] = src[q];
+        if (c_nq == 4 && row) c_w = co.w[i];
         __syncthreads();
     }
 
