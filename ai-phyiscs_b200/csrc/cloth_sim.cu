@@ -1373,6 +1373,8 @@ private:
     }
 
     static constexpr int kResidentMaxWidth = 8;
+    // contact entries a CTA of the resident kernel keeps in shared memory: four per row and the alignment
+    static constexpr size_t kContactStageBytes = 4 * 512 * sizeof(ContactEntry) + 16;
     template <int SYNC>
     const void* persistent_fn_sync() const {
         if (resident_) {
@@ -1500,6 +1502,7 @@ private:
             pers_smem_ = (size_t)W * kSlotW * sizeof(double) + (size_t)plan_.max_inst_per_cta * sizeof(LocalInst);
             if (pc_kind_ >= 1 && sync_mode_ == 0)  // the local preconditioner's columns
                 pers_smem_ += (size_t)(topo_.max_width <= 6 ? 6 : kResidentMaxWidth) * W * 32 * sizeof(int);
+            if (co_active_) pers_smem_ += kContactStageBytes;
             if (coarse_on_)  // the coarse block's rows of A_c^-1, a phase's block values and its staged slots
                 pers_smem_ += ((size_t)9 * coarse_nq_ * coarse_nq_ * coarse_nb_ + (size_t)3 * coarse_nq_ * coarse_nb_) *
                                   sizeof(float) + 16 + (size_t)plan_.inst_slot.back() * kSlotW * sizeof(double) + 16;
@@ -1530,6 +1533,7 @@ private:
         coarse_batched_ = false;
         cluster_ = true;
         pers_smem_ = (size_t)16 * kSlotW * sizeof(double) + (size_t)plan_.max_inst_per_cta * sizeof(LocalInst);
+        if (co_active_) pers_smem_ += kContactStageBytes;
         const void* fn = persistent_fn();
         ck(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pers_smem_),
            "cudaFuncSetAttribute(cluster smem)");

@@ -186,6 +186,40 @@ __device__ __forceinline__ float3 contact_spmv_row(const ContactOp& co, int i, P
     return acc;
 }
 
+// One slot's contact as its row applies it, 48 B: the other slots' rows in
+// slot order (-1: none) and alpha, their weights and the slot's own, and the
+// normal with k - alpha.
+struct ContactEntry {
+    int4 o;     // rows, alpha (bits)
+    float4 w;   // weights, own weight
+    float4 nk;
+};
+__device__ __forceinline__ ContactEntry contact_entry(const ContactOp& co, int e) {
+    const int code = co.ent[e], s = code & 3;
+    const PrepContact& r = co.rec[code >> 2];
+    const int4 q = r.rows;
+    const float4 w = r.w;
+    ContactEntry c;
+    c.o = make_int4(s == 0 ? q.y : q.x, s <= 1 ? q.z : q.y, s <= 2 ? q.w : q.z, __float_as_int(r.ga.w));
+    c.w = make_float4(s == 0 ? w.y : w.x, s <= 1 ? w.z : w.y, s <= 2 ? w.w : w.z, sel4(w, s));
+    c.nk = r.nk;
+    return c;
+}
+// contact_spmv_row's term of one entry from the other slots' p
+__device__ __forceinline__ void contact_apply(const ContactEntry& c, float3 p0, float3 p1, float3 p2, float3& acc) {
+    float3 t = f3(0.f, 0.f, 0.f);
+    auto add = [&](int row, float w, float3 p) {
+        if (row >= 0) t = f3(fmaf(w, p.x, t.x), fmaf(w, p.y, t.y), fmaf(w, p.z, t.z));
+    };
+    add(c.o.x, c.w.x, p0);
+    add(c.o.y, c.w.y, p1);
+    add(c.o.z, c.w.z, p2);
+    const float dn = c.nk.x * t.x + c.nk.y * t.y + c.nk.z * t.z;
+    const float nc = c.w.w * c.nk.w * dn;
+    const float wa = c.w.w * __int_as_float(c.o.w);
+    acc = f3(acc.x + nc * c.nk.x + wa * t.x, acc.y + nc * c.nk.y + wa * t.y, acc.z + nc * c.nk.z + wa * t.z);
+}
+
 // ---------------------------------------------------------------------------
 // Per-step list build
 // ---------------------------------------------------------------------------

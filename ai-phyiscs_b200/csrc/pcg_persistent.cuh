@@ -1576,11 +1576,15 @@ namespace chysx_b200 {
 // against 137 us, 32 x 32 (2) 328 / 230, 64 x 64 (8) 371 / 239, 90 x 90 (16)
 // 376 / 256.
 //
-// CT = 1 adds the contact operator: a row's contact slots are read from the
-// step's list (L2) and their particles' p formed from the exchanged (z, p),
-// as a neighbour's is; only the few rows in contact take the extra loads.
-// Two 160 x 160 sheets with 8,500 contacts: 15.1 us per iteration streamed,
-// 11.1 resident.
+// CT = 1 adds the contact operator: the particles' p of a row's contact slots
+// are formed from the exchanged (z, p), as a neighbour's is.  A CTA's rows are
+// consecutive in the step's list, so their entries are brought into shared
+// memory once per solve (as many as the dynamic allocation holds, the rest
+// // are read from L2): from the list, each entry was three dependent L2 reads
+// before its gathers, one entry after the other.  Two 160 x 160 sheets with
+// 8,500 contacts: 15.1 us per iteration streamed, 10.9 resident from the list,
+// 8.8 from shared memory (9.4 with the entries dealt out to all threads and
+// two at a time 9.7, for the registers).
 // ---------------------------------------------------------------------------
 template <int W, int MAXW, int SYNC = 0, int PC = 0, int CT = 0>
 __global__ void __launch_bounds__(W * 32, 512 / (W * 32))  // 512 threads of rows per SM
@@ -1648,6 +1652,37 @@ pcg_resident_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, ZP
         B[k] = S6{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         col_at(k) = row ? i : 0;
     }
+    // contact entries of this row, [ct_lo, ct_hi); the CTA's first ct_cap are staged
+    int ct_lo = 0, ct_hi = 0, ct_base = 0, ct_cap = 0;
+    float4* ct_st = nullptr;  // planes of ct_cap: rows and alpha, weights, normal
+    if (CT) {
+        uint32_t dyn;
+        asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
+        const uint32_t base = (uint32_t)__cvta_generic_to_shared(s_mem);
+        const uint32_t end = base + (uint32_t)(W * kSlotW * sizeof(double)) + nloc * (uint32_t)sizeof(LocalInst);
+        const uint32_t used = ((end + 15u) & ~15u) - base;  // 16-byte aligned planes
+        ct_cap = dyn > used ? (int)((dyn - used) / sizeof(ContactEntry)) : 0;
+        ct_st = reinterpret_cast<float4*>(reinterpret_cast<char*>(s_mem) + used);
+        if (row) {
+            ct_base = t.co.off[row0];
+            ct_lo = t.co.off[i];
+            ct_hi = t.co.off[i + 1];
+            for (int e = ct_lo; e < min(ct_hi, ct_base + ct_cap); ++e) {
+                const ContactEntry c = contact_entry(t.co, e);
+                reinterpret_cast<int4*>(ct_st)[e - ct_base] = c.o;
+                ct_st[ct_cap + e - ct_base] = c.w;
+                ct_st[2 * ct_cap + e - ct_base] = c.nk;
+            }
+        }
+    }
+    auto ct_entry = [&](int e) {  // this thread staged it
+        if (e - ct_base >= ct_cap) return contact_entry(t.co, e);
+        ContactEntry c;
+        c.o = reinterpret_cast<const int4*>(ct_st)[e - ct_base];
+        c.w = ct_st[ct_cap + e - ct_base];
+        c.nk = ct_st[2 * ct_cap + e - ct_base];
+        return c;
+    };
     if (row) {
         D = ld6(t.dnl + (size_t)s * 192 + lane);
         Mi = ld6(t.minv + (size_t)s * 192 + lane);
@@ -1968,15 +2003,32 @@ pcg_resident_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, ZP
                     acc = acc + mul(B[k0 + k], q - p);
                 }
             }
-            if (CT)
-                acc = acc + contact_spmv_row(t.co, i, [&](int j) {
-                          const int lr = j - row0;
-                          const bool own = (unsigned)lr < (unsigned)nrows;
-                          const float4 zj = own ? s_z[lr] : __ldcg(&E[j].z);
-                          if (first) return xyz(zj);
-                          const float4 pj = own ? sp_old[lr] : __ldcg(&E[j].p);
-                          return f3(fmaf(beta, pj.x, zj.x), fmaf(beta, pj.y, zj.y), fmaf(beta, pj.z, zj.z));
-                      });
+            if (CT && ct_lo < ct_hi) {
+                float3 cacc = f3(0.f, 0.f, 0.f);
+                for (int e = ct_lo; e < ct_hi; ++e) {
+                    const ContactEntry c = ct_entry(e);
+                    const int o[3] = {c.o.x, c.o.y, c.o.z};
+                    float4 zj[3], pj[3];
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) {
+                        const int j = o[q] < 0 ? i : o[q], lr = j - row0;
+                        if ((unsigned)lr < (unsigned)nrows) {
+                            zj[q] = s_z[lr];
+                            pj[q] = sp_old[lr];
+                        } else {
+                            zj[q] = __ldcg(&E[j].z);
+                            pj[q] = __ldcg(&E[j].p);
+                        }
+                    }
+                    auto form = [&](int q) {
+                        return first ? xyz(zj[q])
+                                     : f3(fmaf(beta, pj[q].x, zj[q].x), fmaf(beta, pj[q].y, zj[q].y),
+                                          fmaf(beta, pj[q].z, zj[q].z));
+                    };
+                    contact_apply(c, form(0), form(1), form(2), cacc);
+                }
+                acc = acc + cacc;
+            }
             ap = acc;
             sig = (double)p.x * acc.x + (double)p.y * acc.y + (double)p.z * acc.z;
         }

@@ -16,13 +16,14 @@ pytestmark = pytest.mark.gpu
 class Contacts:
     """Random four-particle contacts, some on one particle twice as often, with slips."""
 
-    def __init__(self, n, m, seed):
+    def __init__(self, n, m, seed, same=None):
         import torch
 
         rng = np.random.default_rng(seed)
         pairs = np.stack([rng.choice(n, 4, replace=False) for _ in range(m)]).astype(np.int32)
-        pairs[: m // 4, 0] = pairs[0, 0]  # a row with many slots
-        pairs[: m // 4, 1:] = np.sort((pairs[0, 0] + 1 + rng.permuted(np.tile(np.arange(n - 1), (m // 4, 1)), axis=1)[:, :3]) % n)
+        k = m // 4 if same is None else same
+        pairs[:k, 0] = pairs[0, 0]  # a row with many slots
+        pairs[:k, 1:] = np.sort((pairs[0, 0] + 1 + rng.permuted(np.tile(np.arange(n - 1), (k, 1)), axis=1)[:, :3]) % n)
         w = np.zeros((m, 8), np.float32)
         w[:, 0] = 1.0
         w[:, 1:4] = -rng.dirichlet((1, 1, 1), m)
@@ -74,3 +75,15 @@ def test_warm_residual(side, mode):
     c = Contacts(side * side, 30, 5)
     a, b = (_run(sc, c, p, 10, 0.0, "previous", 2, mode) for p in (0, 2))
     assert np.abs(a.positions() - b.positions()).max() < 2e-6
+
+
+# more entries than a CTA keeps in shared memory (2048): the rest is read from the list; one CTA, eight, the grid barrier
+@pytest.mark.parametrize("side,m", [(20, 700), (64, 6000), (100, 14000)])
+def test_long_lists(side, m):
+    sc = scenes.config_large(side=side)
+    c = Contacts(side * side, m, side, 12)
+    a, b = (_run(sc, c, p, 10, 0.0) for p in (0, 2))
+    assert np.abs(a.positions() - b.positions()).max() < 5e-7
+    a, b = (_run(sc, c, p, 20000, 1e-8) for p in (0, 2))
+    assert a.stats()[2] == b.stats()[2] == capi.SOLVE_CONVERGED
+    assert np.abs(a.positions() - b.positions()).max() < 1e-5
