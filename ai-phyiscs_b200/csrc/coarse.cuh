@@ -341,27 +341,28 @@ __global__ void __launch_bounds__(kBatchInvThreads) coarse_invert_batched_kernel
 // and is given an identity row).  Per 32-column panel K, with T the inverse
 // of the diagonal tile:
 //     P1  W_KK <- T = W_KK^-1                      (one CTA, in shared memory)
-//     P2  W_KJ <- T W_KJ             (J != K)
-//     P3  W_IJ <- W_IJ - W_IK W_KJ   (I, J != K)
-//     P4  W_IK <- -W_IK T            (I != K; done beside the next panel's P1)
-// with a grid barrier between the phases (three per panel).  Cooperative
+//     P2  W_IJ <- W_IJ - W_IK (T W_KJ)  (I, J != K)
+//     P3  W_KJ <- T W_KJ, W_IK <- -W_IK T  (I, J != K; beside the next panel's P1)
+// with a grid barrier between the phases (two per panel).  In P2 a CTA takes
+// tiles of one column J and forms T W_KJ for them itself: a phase of its own
+// for that product cost a barrier and a round of loads per panel: the step of
+// 256 x 256 (768 unknowns) 2407 us with it, 2286 without.  Cooperative
 // launch (all CTAs co-resident), the barrier's counter zeroed before the
 // launch, every wait bounded; a failed wait or a non-positive pivot sets
 // ca.fail and the PCG kernel then runs without the coarse level.  Cross-CTA
 // data goes through L2 (__ldcg / __stcg).  Output: ca.ainv = S W S (FP32).
 constexpr int kInvTile = 32;
-static_assert(kInvTile * kInvTile % kCoarseInvertThreads == 0, "P3 gives every thread whole tile entries");
+static_assert(kInvTile * kInvTile % kCoarseInvertThreads == 0, "P2 gives every thread whole tile entries");
 
 // c = a * b for 32 x 32 tiles in shared memory (row stride 33); thread t
 // of the kCoarseInvertThreads computes the outputs (t / 32 + j * R, t % 32),
 // j < kTileOut, R = kCoarseInvertThreads / 32: one b entry serves its
 // kTileOut independent sums; sign -1 stores -a * b.
 constexpr int kTileOut = kInvTile * kInvTile / kCoarseInvertThreads;
-__device__ __forceinline__ void tile_mul(const double (*a)[kInvTile + 1], const double (*b)[kInvTile + 1],
-                                         double (*c)[kInvTile + 1], double sign) {
+__device__ __forceinline__ void tile_acc(const double (*a)[kInvTile + 1], const double (*b)[kInvTile + 1],
+                                         double (&acc)[kTileOut]) {
     constexpr int R = kCoarseInvertThreads / kInvTile;
     const int r0 = threadIdx.x / kInvTile, q = threadIdx.x % kInvTile;
-    double acc[kTileOut];
 #pragma unroll
     for (int j = 0; j < kTileOut; ++j) acc[j] = 0.0;
 #pragma unroll 8
@@ -370,6 +371,13 @@ __device__ __forceinline__ void tile_mul(const double (*a)[kInvTile + 1], const 
 #pragma unroll
         for (int j = 0; j < kTileOut; ++j) acc[j] = fma(a[r0 + j * R][k], bk, acc[j]);
     }
+}
+__device__ __forceinline__ void tile_mul(const double (*a)[kInvTile + 1], const double (*b)[kInvTile + 1],
+                                         double (*c)[kInvTile + 1], double sign) {
+    constexpr int R = kCoarseInvertThreads / kInvTile;
+    const int r0 = threadIdx.x / kInvTile, q = threadIdx.x % kInvTile;
+    double acc[kTileOut];
+    tile_acc(a, b, acc);
 #pragma unroll
     for (int j = 0; j < kTileOut; ++j) c[r0 + j * R][q] = sign * acc[j];
 }
@@ -402,6 +410,16 @@ __global__ void __launch_bounds__(kCoarseInvertThreads) coarse_invert_kernel(Coa
             __stcg(dst + (size_t)(o / kInvTile) * mp + o % kInvTile, t[o / kInvTile][o % kInvTile]);
     };
     auto tile_at = [&](int I, int J) { return W + (size_t)I * kInvTile * mp + (size_t)J * kInvTile; };
+    // P2's split of a column over CTAs: the least of rounds x (tiles + 1)
+    int chunks = 1, chunk = nt;
+    for (int c = 1, best = 0x7fffffff; c <= min(nt, 16); ++c) {
+        const int per = (nt + c - 1) / c, cost = (nt * c + (int)gridDim.x - 1) / (int)gridDim.x * (per + 1);
+        if (cost < best) {
+            best = cost;
+            chunks = c;
+            chunk = per;
+        }
+    }
     // dense A_c from its block rows
     for (size_t q = gt; q < (size_t)mp * mp; q += gn) __stcg(W + q, 0.0);
     if (!gsync()) goto fail;
@@ -431,18 +449,22 @@ __global__ void __launch_bounds__(kCoarseInvertThreads) coarse_invert_kernel(Coa
     }
     if (!gsync()) goto fail;
     for (int K = 0; K <= nt; ++K) {
-        // P4 of the previous panel: W_I,K-1 <- -W_I,K-1 T_{K-1}
+        // P3 of the previous panel
         if (K > 0) {
             const double* Tp = Tg + (size_t)((K - 1) & 1) * kInvTile * kInvTile;
-            for (int I = blockIdx.x; I < nt; I += gridDim.x) {
+            for (int x = blockIdx.x; x < 2 * nt; x += gridDim.x) {
+                const bool col = x < nt;  // W_I,K-1, or W_K-1,I
+                const int I = col ? x : x - nt;
                 if (I == K - 1) continue;
+                double* w = col ? tile_at(I, K - 1) : tile_at(K - 1, I);
                 for (int o = tid; o < kInvTile * kInvTile; o += blockDim.x)
                     sb[o / kInvTile][o % kInvTile] = __ldcg(Tp + o);
-                ld_tile(sa, tile_at(I, K - 1));
+                ld_tile(sa, w);
                 __syncthreads();
-                tile_mul(sa, sb, sc_, -1.0);
+                if (col) tile_mul(sa, sb, sc_, -1.0);
+                else tile_mul(sb, sa, sc_, 1.0);
                 __syncthreads();
-                st_tile(tile_at(I, K - 1), sc_);
+                st_tile(w, sc_);
                 __syncthreads();
             }
         }
@@ -451,7 +473,7 @@ __global__ void __launch_bounds__(kCoarseInvertThreads) coarse_invert_kernel(Coa
             break;
         }
         // P1: T = W_KK^-1 by Gauss-Jordan in shared memory (the last CTA,
-        // the others being busy with P4 above), two pivots a step: the chain
+        // the others being busy with P3 above), two pivots a step: the chain
         // of a step is its division, so a 2 x 2 pivot block (one division, by
         // its determinant) halves it.  Every step reads the tile of the
         // previous one and writes the other of two buffers, one CTA barrier
@@ -500,43 +522,50 @@ __global__ void __launch_bounds__(kCoarseInvertThreads) coarse_invert_kernel(Coa
             st_tile(tile_at(K, K), cur);
         }
         if (!gsync()) goto fail;
-        // P2: W_KJ <- T W_KJ
-        {
-            const double* Tk = Tg + (size_t)(K & 1) * kInvTile * kInvTile;
-            for (int J = blockIdx.x; J < nt; J += gridDim.x) {
-                if (J == K) continue;
-                for (int o = tid; o < kInvTile * kInvTile; o += blockDim.x)
-                    sa[o / kInvTile][o % kInvTile] = __ldcg(Tk + o);
-                ld_tile(sb, tile_at(K, J));
-                __syncthreads();
-                tile_mul(sa, sb, sc_, 1.0);
-                __syncthreads();
-                st_tile(tile_at(K, J), sc_);
-                __syncthreads();
-            }
-        }
-        if (!gsync()) goto fail;
-        // P3: W_IJ <- W_IJ - W_IK W_KJ
-        for (int x = blockIdx.x; x < nt * nt; x += gridDim.x) {
-            const int I = x / nt, J = x % nt;
-            if (I == K || J == K) continue;
-            // the tile to update is read with the two factors (one round trip)
-            double* dst = tile_at(I, J);
-            double cur[kInvTile * kInvTile / kCoarseInvertThreads];
+        // P2: chunk `x / nt` of column J = x % nt, the next tile of the column
+        // read while one is multiplied
+        const double* Tk = Tg + (size_t)(K & 1) * kInvTile * kInvTile;
+        for (int x = blockIdx.x; x < nt * chunks; x += gridDim.x) {
+            const int J = x % nt, end = min(nt, (x / nt + 1) * chunk);
+            auto next = [&](int I) { return I == K ? I + 1 : I; };
+            int I = next(x / nt * chunk);
+            if (J == K || I >= end) continue;
+            double ra[kTileOut], rc[kTileOut];  // W_IK, W_IJ: entries tid + j * threads
+            auto fetch = [&](int i) {
 #pragma unroll
-            for (int j = 0; j < kInvTile * kInvTile / kCoarseInvertThreads; ++j) {
-                const int o = tid + j * kCoarseInvertThreads;
-                cur[j] = __ldcg(dst + (size_t)(o / kInvTile) * mp + o % kInvTile);
-            }
-            ld_tile(sa, tile_at(I, K));
+                for (int j = 0; j < kTileOut; ++j) {
+                    const int o = tid + j * kCoarseInvertThreads;
+                    ra[j] = __ldcg(tile_at(i, K) + (size_t)(o / kInvTile) * mp + o % kInvTile);
+                    rc[j] = __ldcg(tile_at(i, J) + (size_t)(o / kInvTile) * mp + o % kInvTile);
+                }
+            };
+            for (int o = tid; o < kInvTile * kInvTile; o += blockDim.x)
+                sa[o / kInvTile][o % kInvTile] = __ldcg(Tk + o);
             ld_tile(sb, tile_at(K, J));
+            fetch(I);
             __syncthreads();
-            tile_mul(sa, sb, sc_, 1.0);
+            tile_mul(sa, sb, sc_, 1.0);  // the new W_KJ
             __syncthreads();
+            double(*buf)[kInvTile + 1] = sa;
+            while (I < end) {
+                double cur[kTileOut], acc[kTileOut];
 #pragma unroll
-            for (int j = 0; j < kInvTile * kInvTile / kCoarseInvertThreads; ++j) {
-                const int o = tid + j * kCoarseInvertThreads;
-                __stcg(dst + (size_t)(o / kInvTile) * mp + o % kInvTile, cur[j] - sc_[o / kInvTile][o % kInvTile]);
+                for (int j = 0; j < kTileOut; ++j) {
+                    const int o = tid + j * kCoarseInvertThreads;
+                    buf[o / kInvTile][o % kInvTile] = ra[j];
+                    cur[j] = rc[j];
+                }
+                const int In = next(I + 1);
+                if (In < end) fetch(In);
+                __syncthreads();  // and the other buffer's readers are past it
+                tile_acc(buf, sc_, acc);
+#pragma unroll
+                for (int j = 0; j < kTileOut; ++j) {
+                    const int o = tid + j * kCoarseInvertThreads;  // tile_acc's entry j
+                    __stcg(tile_at(I, J) + (size_t)(o / kInvTile) * mp + o % kInvTile, cur[j] - acc[j]);
+                }
+                buf = buf == sa ? sb : sa;
+                I = In;
             }
             __syncthreads();
         }
