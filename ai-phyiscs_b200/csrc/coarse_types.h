@@ -36,7 +36,7 @@ constexpr int kCoarseMaxSplits = 32;
 // 25.9 ms a step with these, 808 and 37.8 ms with a block per instance and CTA.
 constexpr int kTileBlockRows = 1024;
 constexpr int kTileBatchSlices = 9;
-// Relative diagonal shift of the streamed kernel's coarse matrix: A_c +
+// Relative diagonal shift of the streamed and tiled kernels' coarse matrix: A_c +
 // shift diag(A_c) is inverted instead of A_c (the resident kernel's coarse
 // matrix, on smaller blocks, is inverted unshifted).  The coarse matrix of a flat,
 // unstretched cloth (the first step from rest) has out-of-plane modes held
@@ -45,9 +45,9 @@ constexpr int kTileBatchSlices = 9;
 // usable preconditioner (the solve stalls).  The shift bounds the scaled
 // condition number near 3e5 and still leaves an SPD coarse correction.
 constexpr double kCoarseShift = 1.0e-5;
-// The streamed kernel's coarse level for batches: at most this many coarse
-// blocks per instance (each an instance's rows in one CTA, or a run of such
-// segments), so an instance's dense inverse has at most 144 unknowns.
+// The coarse level for batches: at most this many coarse blocks per instance
+// (streamed kernel: an instance's rows in one CTA, or a run of such segments;
+// tiled kernel: parts of them), so an instance's dense inverse has at most 144 unknowns.
 constexpr int kBatchMaxBlocks = 12;
 
 // Coarse space: coarse block B is the rows of CTAs [B G, (B + 1) G) of the

@@ -25,7 +25,7 @@
 // Per iteration a row costs its blocks and 16-bit columns (26 B each), D'
 // and M^-1 (48 B), and 32 B of coarse weights with the coarse level.
 // Measured on B200, streamed against tiled: 801 x 643 rows, 50 iterations,
-// 2.88 against 1.48 ms (53 against 25 us per iteration); 1024 x 1024 with the
+// 2.88 against 1.30 ms (53 against 21 us per iteration); 1024 x 1024 with the
 // coarse level 118 against 56 us per iteration; a batch of 128 grids of 16 to
 // 128 a side 105 against 47.
 //
@@ -40,7 +40,7 @@
 // (MODE 2): the grid is one thread-block cluster, whose barrier and shared
 // memory carry the reductions, as in the resident kernel's cluster build.
 // A 61 x 47 garment with bending (18 neighbours a row, 16 CTAs): 11.9 us per
-// iteration streamed, 5.0 as a cluster.
+// iteration streamed, 4.6 as a cluster.
 #pragma once
 
 #include "pcg_persistent.cuh"

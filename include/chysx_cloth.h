@@ -172,8 +172,8 @@ int chysx_cloth_get_static_contact(const chysx_cloth* h, float* thickness, float
  * and slips are given.  A contact whose stiffness is not finite and
  * positive is skipped; one with a weighted particle index outside the
  * particle range is dropped and counted (contact_stats).  Needs the
- * single-instance layout; the contact terms are streamed in every solver
- * iteration, whichever kernel holds the rows (chysx_cloth_solver_info). */
+ * single-instance layout; solver_info reports path 2 with one,
+ * whichever kernel holds the rows (chysx_cloth_solver_info). */
 typedef struct chysx_contact_op {
     uintptr_t pairs;       /* int32 x 4 per contact, 16-byte aligned */
     uintptr_t weights;     /* float x 8 per contact: w0..w3, nx, ny, nz, depth; 16-byte aligned */
@@ -272,8 +272,8 @@ int chysx_cloth_debug_dump(chysx_cloth* h, float* diag, int32_t* row_offsets,
  * blocks, CTAs per block, fields per block, unknowns m, 0};
  * with ac / ainv non-null (host, m * m floats each, cap >= m * m) the coarse
  * matrix A_c dense and the inverse the solver used (of A_c + shift
- * diag(A_c), shift 0 on the register-resident kernel, 1e-5 on the streamed
- * one; for the batched level the inverse is block-diagonal by instance),
+ * diag(A_c), shift 0 on the register-resident kernel, 1e-5 on the others;
+ * for the batched level the inverse is block-diagonal by instance),
  * unknown
  * index block * 3 * fields + 3 * field + component.  Synchronises. */
 int chysx_cloth_debug_coarse(chysx_cloth* h, int32_t* info, float* ac, float* ainv, int cap);
@@ -388,8 +388,8 @@ int chysx_cloth_set_sync_mode(chysx_cloth* h, int mode);
 
 /* Autotuner (no counterpart in the reference).  Times, on the current state,
  * every solver configuration that applies to the current system: the
- * planner's persistent kernel (register-resident rows when they fit, else
- * streamed), the streamed kernel at 128 / 256 / 512 threads per CTA (4 / 8 /
+ * planner's persistent kernel (register-resident rows or vectors on the SMs
+ * when they fit, else streamed), the streamed kernel at 128 / 256 / 512 threads per CTA (4 / 8 /
  * 16 32-row slices per CTA; one thread per row), both synchronisation modes,
  * and the graph-loop path; each `repetitions` times (best kept).  All run the
  * same PCG recurrence.  The caller's positions / velocities and the previous-step guess are
@@ -434,12 +434,12 @@ int chysx_cloth_row_of_particles(const chysx_cloth* h, int n, int32_t* rows);
  * most 2048 unknowns).  It applies to single-instance systems of at most
  * 160 CTAs and acts as kind 1 elsewhere.  Kinds 1 and 2 apply where the
  * register-resident kernel runs with synchronisation mode 0.  On systems too
- * large for that kernel (the streamed kernel), kinds 1 and 2 give
- * block-Jacobi plus the coarse level on blocks of about 5120 rows, A_c
- * shifted by 1e-5 diag(A_c) (single instance, synchronisation mode 0); on
+ * large for that kernel, kinds 1 and 2 give block-Jacobi plus the coarse
+ * level on blocks of whole CTAs (about 5120 rows on the streamed kernel, one
+ * or more SMs' rows where the vectors stay on the SMs), A_c shifted by 1e-5 diag(A_c) (single instance, synchronisation mode 0); on
  * batches of instances there (zero-guess solves, synchronisation mode 0),
  * block-Jacobi plus coarse blocks inside the instances (an instance's rows in
- * one CTA, or runs of such segments, at most 12 per instance; translation and
+ * one CTA, runs or parts of such segments, at most 12 per instance; translation and
  * linear fields; A_c block-diagonal by instance, each instance's dense
  * inverse formed on its own, same shift).
  * in_use reports what the last graph build uses (0 block-Jacobi, 1 local,
@@ -448,9 +448,9 @@ int chysx_cloth_row_of_particles(const chysx_cloth* h, int n, int32_t* rows);
 int chysx_cloth_set_preconditioner(chysx_cloth* h, int kind, int degree, float ratio);
 int chysx_cloth_preconditioner(const chysx_cloth* h, int* kind, int* degree, float* ratio, int* in_use);
 /* Kernel used at the last graph build: path 0 register-resident persistent,
- * 1 graph loop, 2 streamed persistent (every kernel that reads part of the
- * system again in each iteration: with a contact operator the register-
- * resident rows too); with its grid and block size. */
+ * 1 graph loop, 2 every other persistent kernel (vectors on the SMs, streamed,
+ * and the register-resident rows with a contact operator); with its grid and
+ * block size. */
 int chysx_cloth_solver_info(const chysx_cloth* h, int* path, int* grid, int* block);
 
 /* Measurement hooks (no counterpart in the reference): when enabled, the
