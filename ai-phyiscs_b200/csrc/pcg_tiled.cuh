@@ -335,8 +335,12 @@ pcg_tiled_kernel(DevTopo t, Vecs v, BatchPlan bp, SolverCfg cfg, int warm, const
     int staged = -1;
     uint32_t stage_par = 0;
     auto stage_blocks = [&](int k) { return min((s_off[k + 1] - s_off[k]) >> 5, n_stage); };
-    auto stage_slice = [&](int k) {  // the warp's reads of the stage are done (__syncwarp)
+    // every lane's reads of the stage come before the copy that overwrites it:
+    // plain reads and the copy engine's writes go through different proxies,
+    // which __syncwarp alone does not order
+    auto stage_slice = [&](int k) {
         const int c = stage_blocks(k);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (c == 0) return;
         staged = k;
