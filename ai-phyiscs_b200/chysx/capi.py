@@ -127,6 +127,7 @@ SIGNATURES = {
     "chysx_vbd_step_cloth": (ctypes.c_int, [H, u, u, u, ctypes.c_int, u, u, u, u, ctypes.c_int, u, u, u, u,
                                             ctypes.c_int, ctypes.c_float, ctypes.c_float, ctypes.c_float,
                                             ctypes.c_float, ctypes.c_int, u]),
+    "chysx_debug_tile_layout": (ctypes.c_int, [i32p, ctypes.POINTER(ctypes.c_uint64)]),
     "chysx_topology_pattern": (ctypes.c_int, [ctypes.c_int, i32p, ctypes.c_int, i32p, ctypes.c_int,
                                               i32p, i32p, ctypes.c_int, ip, ip, ip]),
 }
@@ -516,6 +517,16 @@ class Vbd:
         check(self._L.chysx_vbd_step_cloth(self.h, pos, vel, inv_mass, n, tris, poses, areas, mats, n_tris, edges,
                                            rest_angle, rest_length, props, n_edges, *[float(g) for g in gravity],
                                            float(dt), int(iterations), stream))
+
+
+def debug_tile_layout(parts, max_inst, coarse_bytes, max_blk, max_slices, max_halo, max_entries, ow, stage):
+    """Host-only: byte offsets of the tiled kernel's shared-memory regions by
+    name, and the total (see the header)."""
+    sizes = np.array([parts, max_inst, coarse_bytes, max_blk, max_slices, max_halo, max_entries, ow, stage], np.int32)
+    out = (ctypes.c_uint64 * 14)()
+    check(lib().chysx_debug_tile_layout(_p(sizes, i32p), out))
+    keys = ("li", "vbuf", "blk", "soff", "mask", "sli", "hrow", "hli", "p", "mat", "diag", "col", "stage", "bytes")
+    return dict(zip(keys, (int(v) for v in out)))
 
 
 def topology_pattern(n, tris, edges=None):

@@ -1929,7 +1929,7 @@ private:
             for (int c = 0; c < plan_.grid; ++c)
                 max_entries = std::max(max_entries, topo_.slice_off[plan_.cta_slice[c + 1]] -
                                                         topo_.slice_off[plan_.cta_slice[c]]);
-            max_entries = std::max(max_entries, 1);
+            max_entries = std::max(max_entries, 32);  // no entries at all: still MODE 2's layout
             // far above any SM's shared memory: no need to look for the halo
             if ((size_t)max_entries * off_width() * sizeof(float) > ((size_t)1 << 18)) return false;
         }
@@ -3054,6 +3054,17 @@ int chysx_cloth_enable_timing(chysx_cloth* h, int on) {
 int chysx_cloth_last_timing(chysx_cloth* h, float* assemble_ms, float* solve_ms, float* finalize_ms) {
     CHYSX_H(h);
     return guard([&] { h->sim.last_timing(assemble_ms, solve_ms, finalize_ms); });
+}
+
+int chysx_debug_tile_layout(const int32_t* in, uint64_t* out) {
+    return guard([&] {
+        if (!in || !out) throw std::invalid_argument("chysx_debug_tile_layout: null pointer");
+        for (int k = 0; k < 9; ++k)
+            if (in[k] < 0) throw std::invalid_argument("chysx_debug_tile_layout: negative size");
+        const chysx_b200::TileSmem t = chysx_b200::tile_smem(in[0], in[1], (size_t)in[2], in[3], in[4], in[5], in[6], in[7], in[8]);
+        const size_t o[14] = {t.li, t.vbuf, t.blk, t.soff, t.mask, t.sli, t.hrow, t.hli, t.p, t.mat, t.diag, t.col, t.stage, t.bytes};
+        std::copy(o, o + 14, out);
+    });
 }
 
 int chysx_topology_pattern(int n, const int32_t* tris, int n_tris, const int32_t* edges, int n_edges,

@@ -94,8 +94,9 @@ __host__ __device__ inline TileSmem tile_smem(int parts, int max_inst, size_t co
     s.hli = s.hrow + (size_t)max_halo * sizeof(int);
     s.p = tile_align(s.hli + (size_t)max_halo * sizeof(unsigned short));
     s.mat = tile_align(s.p + (size_t)3 * (32 * (size_t)max_slices + max_halo) * sizeof(float));
-    // MODE 2: blocks, D' and M^-1 (192 floats each per slice), columns
-    s.diag = s.mat + (size_t)max_entries * ow * sizeof(float);
+    // MODE 2: blocks, D' and M^-1 (192 floats each per slice; copied in 16-byte
+    // pieces, as the blocks), columns
+    s.diag = tile_align(s.mat + (size_t)max_entries * ow * sizeof(float));
     s.col = s.diag + (max_entries ? (size_t)384 * max_slices * sizeof(float) : 0);
     s.stage = (s.col + (size_t)max_entries * sizeof(unsigned short) + 127) & ~static_cast<size_t>(127);
     s.bytes = s.stage + (size_t)stage * (kTileThreads / 32) * 192 * sizeof(float);

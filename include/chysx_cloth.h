@@ -471,6 +471,15 @@ int chysx_topology_pattern(int n, const int32_t* tris, int n_tris, const int32_t
                            int32_t* row_offsets, int32_t* col_indices, int max_nnz, int* nnz_out,
                            int* ell_entries_out, int* max_width_out);
 
+/* Host-only: the shared-memory layout of the solver kernel that keeps the
+ * vectors on the SMs (test support, no counterpart in the reference).  in:
+ * slice partials, instances, coarse bytes, coarse blocks, slices, halo rows,
+ * matrix entries (0: matrix streamed), floats per entry, staged blocks per
+ * warp, each of a CTA; out: byte offsets of records, coarse values, blocks,
+ * slice offsets, masks, slice instances, halo rows, halo instances, p, matrix,
+ * diagonals, columns and stages, then the total.  Needs no GPU. */
+int chysx_debug_tile_layout(const int32_t* in, uint64_t* out);
+
 #ifdef __cplusplus
 }
 #endif

@@ -70,6 +70,19 @@ def test_warm_starts(w, h, block, warm, order):
     assert np.abs(a.positions() - b.positions()).max() < 1e-5
 
 
+@pytest.mark.parametrize("w,h", [(320, 320), (321, 317)])
+def test_particles_without_elements(w, h):
+    # inertia and pins alone, more rows than the register-resident kernel takes: a matrix without entries
+    sc = dict(_rect(w, h), k_spring=None, k_stretch=None)
+    a, b = _run(sc, 0, its=20, tol=1e-6, steps=2), _run(sc, 2, its=20, tol=1e-6, steps=2)
+    assert a.sim.num_off_diag_blocks() == 0 and a.sim.solver_info()[2] == 512
+    assert a.stats()[2] == capi.SOLVE_CONVERGED
+    assert np.abs(a.positions() - b.positions()).max() < 5e-7
+    # two steps of free fall from rest: 3 g dt^2 down
+    free = np.arange(w, w * h)
+    assert np.abs(a.positions()[free, 1] - sc["pos"][free, 1] + 3 * 9.81 / 3600.0).max() < 1e-6
+
+
 # Long solves with several slices per warp: the stage then holds another slice's blocks at every use (three and four
 # slices a warp at 801 x 643, seven at 1024 x 1024).  A block of another slice, or a halo value that is not its owner's,
 # costs conjugacy and shows in the count; over thousands of iterations the two kernels' roundings move it by less than

@@ -235,3 +235,18 @@ def test_bridge_device_addresses_and_host_arrays():
         device_address("x")
     a = host_array([[0, 1, 2], [2, 1, 3]], np.int32)
     assert a.dtype == np.int32 and a.shape == (2, 3)
+
+
+@pytest.mark.parametrize("entries", [0, 1, 31, 32, 96])
+@pytest.mark.parametrize("slices,halo,inst", [(1, 0, 1), (7, 3, 2), (17, 101, 13)])
+def test_tile_layout_alignment(slices, halo, inst, entries):
+    """16 bytes wherever the tiled kernel copies 16-byte pieces, whatever the sizes before it."""
+    for ow in (6, 9):
+        for stage in (0, 3):
+            d = capi.debug_tile_layout(16, inst, 100 * inst, inst, slices, halo, entries, ow, stage)
+            offs = list(d.values())
+            assert offs == sorted(offs)
+            assert [d[k] % 16 for k in ("vbuf", "blk", "p", "mat", "diag")] == [0] * 5
+            assert d["li"] % 8 == d["soff"] % 4 == d["hrow"] % 4 == d["col"] % 2 == d["stage"] % 128 == 0
+            assert d["diag"] - d["mat"] >= 4 * entries * ow
+            assert d["col"] - d["diag"] == (384 * 4 * slices if entries else 0)
