@@ -124,6 +124,8 @@ SIGNATURES = {
     "chysx_vbd_build_edge_adjacency": (ctypes.c_int, [H, i32p, ctypes.c_int, ctypes.c_int]),
     "chysx_vbd_num_colors": (ctypes.c_int, [H, ip]),
     "chysx_vbd_colors": (ctypes.c_int, [H, i32p, ctypes.c_int]),
+    "chysx_vbd_last_status": (ctypes.c_int, [H, ip]),
+    "chysx_vbd_debug_fail_barrier": (ctypes.c_int, [H, ctypes.c_int]),
     "chysx_vbd_step_cloth": (ctypes.c_int, [H, u, u, u, ctypes.c_int, u, u, u, u, ctypes.c_int, u, u, u, u,
                                             ctypes.c_int, ctypes.c_float, ctypes.c_float, ctypes.c_float,
                                             ctypes.c_float, ctypes.c_int, u]),
@@ -517,6 +519,16 @@ class Vbd:
         check(self._L.chysx_vbd_step_cloth(self.h, pos, vel, inv_mass, n, tris, poses, areas, mats, n_tris, edges,
                                            rest_angle, rest_length, props, n_edges, *[float(g) for g in gravity],
                                            float(dt), int(iterations), stream))
+
+    def last_status(self):
+        """Waits for the last step: SOLVE_KERNEL_ERROR when a step since the
+        last report was abandoned at a grid barrier, else SOLVE_CONVERGED."""
+        v = ctypes.c_int()
+        check(self._L.chysx_vbd_last_status(self.h, ctypes.byref(v)))
+        return v.value
+
+    def debug_fail_barrier(self, on):
+        check(self._L.chysx_vbd_debug_fail_barrier(self.h, int(on)))
 
 
 def debug_tile_layout(parts, max_inst, coarse_bytes, max_blk, max_slices, max_halo, max_entries, ow, stage):

@@ -3137,4 +3137,16 @@ int chysx_vbd_step_cloth(chysx_vbd* h, uintptr_t pos, uintptr_t vel, uintptr_t i
     });
 }
 
+int chysx_vbd_last_status(chysx_vbd* h, int* status) {
+    CHYSX_VBD(h);
+    return guard([&] {
+        const int st = h->solver.last_status();
+        if (status) *status = st;
+    });
+}
+int chysx_vbd_debug_fail_barrier(chysx_vbd* h, int on) {
+    CHYSX_VBD(h);
+    return guard([&] { h->solver.debug_fail_barrier(on != 0); });
+}
+
 }  // extern "C"

@@ -507,6 +507,13 @@ PYBIND11_MODULE(_chysx_native, m) {
              py::arg("edge_rest_angle_ptr"), py::arg("edge_rest_length_ptr"), py::arg("edge_bending_props_ptr"),
              py::arg("n_edges"), py::arg("gx"), py::arg("gy"), py::arg("gz"), py::arg("dt"), py::arg("iterations"),
              py::arg("cuda_stream") = 0, "Run one cloth VBD substep.")
+        .def("last_status",
+             [](PyVbd& s) {
+                 int st = 0;
+                 check(chysx_vbd_last_status(s.h(), &st));
+                 return st;
+             },
+             "0, or 3 when a step since the last report was abandoned at a grid barrier (waits for the last step).")
         .def("num_colors",
              [](const PyVbd& s) {
                  int c = 0;

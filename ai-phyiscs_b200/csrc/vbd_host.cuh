@@ -2,8 +2,8 @@
 // src/bindings.cpp:1868-1957, solver/vbd_solver.h:134-176): colouring,
 // per-vertex adjacency, and the step, which runs as one CUDA graph (one
 // cooperative kernel, or predictor, iterations x colours sweep kernels and
-// velocity update) rebuilt only when the step's arguments change.  Included by cloth_sim.cu (shares its error
-// handling and device buffers).
+// velocity update) rebuilt only when the step's arguments change.  Included by
+// cloth_sim.cu (shares its error handling and device buffers).
 #pragma once
 
 #include <numeric>
@@ -107,6 +107,7 @@ public:
             throw std::invalid_argument("step_cloth: edge arrays are required with n_edges > 0");
         if (n_tris > 0 && tri_n_ != n) throw std::invalid_argument("step_cloth: build_tri_adjacency first");
         if (n_edges > 0 && edge_n_ != n) throw std::invalid_argument("step_cloth: build_edge_adjacency first");
+        report_failure();
         if (dirty_) {
             d_ids_.upload(ids_.empty() ? std::vector<int>{0} : ids_);
             if (tri_n_ >= 0) {
@@ -127,6 +128,7 @@ public:
                 d_bar_.resize(1);
                 drop_graph();
             }
+            failed_.create();
         } else if (d_q_prev_.size() != 3 * (size_t)n) {
             d_q_prev_.resize(3 * (size_t)n);
             d_inertia_.resize(3 * (size_t)n);
@@ -164,10 +166,47 @@ public:
             if (one_launch_) build_graph_one(a, iterations);
             else build_graph(a, iterations);
         }
+        last_stream_ = stream;
         ck(cudaGraphLaunch(exec_, reinterpret_cast<cudaStream_t>(stream)), "cudaGraphLaunch(vbd step)");
     }
 
+    // CHYSX_SOLVE_KERNEL_ERROR when a step since the last report left the
+    // state as it was because a grid barrier timed out (waits for the last step).
+    int last_status() {
+        ck(cudaStreamSynchronize(reinterpret_cast<cudaStream_t>(last_stream_)), "cudaStreamSynchronize(vbd)");
+        return failed_.take() ? CHYSX_SOLVE_KERNEL_ERROR : CHYSX_SOLVE_CONVERGED;
+    }
+    // Test support: the one-kernel step's barriers fail at once.
+    void debug_fail_barrier(bool on) {
+        fail_barrier_ = on;
+        drop_graph();
+    }
+
 private:
+    // One word of pinned host memory that the device sets, read without waiting.
+    struct HostFlag {
+        int* p = nullptr;
+        void create() {
+            if (p) return;
+            ck(cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable),
+               "cudaHostAlloc(vbd)");
+            *p = 0;
+        }
+        bool take() {
+            const bool set = p && *(volatile int*)p != 0;
+            if (set) *(volatile int*)p = 0;
+            return set;
+        }
+        ~HostFlag() {
+            if (p) cudaFreeHost(p);
+        }
+    };
+    void report_failure() {
+        if (failed_.take())
+            throw std::runtime_error("step_cloth: a grid barrier of an earlier step timed out; that step left "
+                                     "positions and velocities as they were");
+    }
+
     void build_adjacency(const int32_t* el, int count, int arity, int n, std::vector<int>& off, std::vector<int>& adj,
                          const char* what) {
         if (n < 0 || count < 0) throw std::invalid_argument(std::string(what) + ": negative count");
@@ -286,7 +325,6 @@ private:
         cudaGraph_t g;
         ck(cudaGraphCreate(&g, 0), "cudaGraphCreate(vbd)");
         cudaGraphNode_t reset, node;
-        cudaMemsetParams mp{};
         vbd::StepPlan sp{};
         sp.state = d_state_.get();
         sp.own = d_own_.get();
@@ -302,12 +340,23 @@ private:
         sp.bar = d_bar_.get();
         sp.n_colors = num_colors();
         sp.iterations = iterations;
+        void* flag = nullptr;
+        cudaError_t e = cudaHostGetDevicePointer(&flag, failed_.p, 0);
+        sp.failed = static_cast<int*>(flag);
+        cudaMemsetParams mp{};
         mp.dst = sp.bar;
         mp.value = 0;
         mp.elementSize = 4;
         mp.width = sizeof(GridBarrier) / 4;
         mp.height = 1;
-        cudaError_t e = cudaGraphAddMemsetNode(&reset, g, nullptr, 0, &mp);
+        if (e == cudaSuccess) e = cudaGraphAddMemsetNode(&reset, g, nullptr, 0, &mp);
+        if (fail_barrier_ && e == cudaSuccess) {
+            const cudaGraphNode_t zeroed = reset;
+            mp.dst = &sp.bar->error;
+            mp.value = 1;
+            mp.width = 1;
+            e = cudaGraphAddMemsetNode(&reset, g, &zeroed, 1, &mp);
+        }
         vbd::ClothArgs args = a;
         void* prm[] = {&args, &sp};
         cudaKernelNodeParams p{};
@@ -378,6 +427,9 @@ private:
     std::vector<int> colors_, group_off_;
     std::vector<int> ids_, tri_off_, tri_adj_, edge_off_, edge_adj_;  // host copies, uploaded by step
     bool dirty_ = false;
+    HostFlag failed_;  // freed after the device buffers below, whose release waits for running steps
+    bool fail_barrier_ = false;
+    uintptr_t last_stream_ = 0;
     DevBuf<int> d_ids_, d_tri_off_, d_tri_adj_, d_edge_off_, d_edge_adj_;
     DevBuf<float> d_q_prev_, d_inertia_, d_disp_, d_mass_;
     // the one-kernel step

@@ -454,15 +454,36 @@ struct StepPlan {
     const int* hinge_rec;
     Records rec;
     GridBarrier* bar;
+    int* failed;           // host memory: a barrier timed out
     int n_colors, iterations;
 };
+
+// The barrier after which the result is written, with one outcome for the whole
+// grid: no CTA may leave because its wait ran out while another sees the count
+// complete and writes its share.  The CTAs count in gen, which a CTA that gives
+// up marks, unless the count is complete by then; all read that one word.
+__device__ __forceinline__ bool last_arrive_wait(GridBarrier* gb) {
+    constexpr unsigned kLeft = 0x80000000u;
+    red_release_add(&gb->gen, 1u);
+    const unsigned long long t0 = global_ns();
+    unsigned spins = 0;
+    for (;;) {
+        unsigned v = ld_acquire_gpu(&gb->gen);
+        if (v & kLeft) return false;
+        if (v == gridDim.x) return true;
+        if ((++spins & 255u) == 0 && (*(volatile int*)&gb->error || global_ns() - t0 > kBarrierTimeoutNs)) {
+            const unsigned was = atomicCAS(&gb->gen, v, v | kLeft);
+            if (was == v) return false;  // else look again: more have arrived, or another gave up
+        }
+    }
+}
 
 // Before the first barrier: the predictor (q_prev = x, m = 1/w, inertia y = x + dt v', x = y with v' = v +
 // dt g; a particle with w == 0 stays, vbd_solver.cu:64-92) and the packing of
 // every vertex's element records; then iterations x colours sweeps
 // (vbd_solver.cu:304-407) with a grid barrier each; then x and v = (x -
 // q_prev) / dt (vbd_solver.cu:284-293).  The caller's positions are q_prev
-// until the end.
+// until the end; where a barrier times out no CTA writes them.
 //
 // Records are read in lane order and fetched one round, one tile and one
 // barrier ahead, so a sweep waits for its neighbours' state and nothing else.
@@ -480,6 +501,15 @@ __global__ void __launch_bounds__(kVbdThreads, 2) vbd_step_kernel(ClothArgs a, S
         if (threadIdx.x == 0) s_ok = barrier_arrive_wait(s.bar, target) ? 1 : 0;
         __syncthreads();
         return s_ok != 0;
+    };
+    auto last_sync = [&]() -> bool {
+        __syncthreads();
+        if (threadIdx.x == 0) s_ok = last_arrive_wait(s.bar) ? 1 : 0;
+        __syncthreads();
+        return s_ok != 0;
+    };
+    auto give_up = [&]() {  // the caller's state stays as it was
+        if (threadIdx.x == 0) *(volatile int*)s.failed = 1;
     };
     const float dt = a.dt;
     for (int i = gt; i < a.n; i += gn) {
@@ -599,7 +629,7 @@ __global__ void __launch_bounds__(kVbdThreads, 2) vbd_step_kernel(ClothArgs a, S
         }
         return x;
     };
-    if (!grid_sync()) return;
+    if (!grid_sync()) return give_up();
     const long sweeps = (long)s.iterations * s.n_colors;
     ColorPlan cp = s.colors[0];
     Tile cur = fetch_tile(cp, gw);
@@ -686,10 +716,12 @@ __global__ void __launch_bounds__(kVbdThreads, 2) vbd_step_kernel(ClothArgs a, S
                 }
             }
         }
-        if (!grid_sync()) return;
+        if (sw + 1 == sweeps) break;
+        if (!grid_sync()) return give_up();
         cp = cn;
         c = c_next;
     }
+    if (!last_sync()) return give_up();
     for (int i = gt; i < a.n; i += gn) {
         const float4 p = s.state[i].xm;
         const V3 x = v3(p.x, p.y, p.z);

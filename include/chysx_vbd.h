@@ -46,12 +46,24 @@ int chysx_vbd_colors(const chysx_vbd* h, int32_t* out, int n_particles);
  * advanced in place; per triangle (int32 x3) Dm^-1 (float x4, row-major),
  * rest area, material (mu, lambda, damping); per bending edge (int32 x4) rest
  * angle, rest length, (stiffness, damping).  n_tris / n_edges = 0 leave that
- * energy out.  The step is one CUDA-graph launch on `stream`. */
+ * energy out.  The step is one CUDA-graph launch on `stream`.  Where it runs
+ * as one cooperative kernel, a grid barrier that times out (2 s) leaves pos and
+ * vel as they were; the next step_cloth reports that as CHYSX_ERR_RUNTIME
+ * without running, or chysx_vbd_last_status does. */
 int chysx_vbd_step_cloth(chysx_vbd* h, uintptr_t pos, uintptr_t vel, uintptr_t inv_mass, int n_particles,
                          uintptr_t tri_indices, uintptr_t tri_poses, uintptr_t tri_areas, uintptr_t tri_materials,
                          int n_tris, uintptr_t edge_indices, uintptr_t edge_rest_angle, uintptr_t edge_rest_length,
                          uintptr_t edge_bending_props, int n_edges, float gx, float gy, float gz, float dt,
                          int iterations, uintptr_t stream);
+
+/* Waits for the last step: CHYSX_SOLVE_KERNEL_ERROR when a step since the last
+ * report was abandoned at a grid barrier (the report clears it), else
+ * CHYSX_SOLVE_CONVERGED.  No counterpart in the reference, whose steps have no
+ * such wait. */
+int chysx_vbd_last_status(chysx_vbd* h, int* status);
+/* Test support: with on != 0 the cooperative step finds its first barrier
+ * failed. */
+int chysx_vbd_debug_fail_barrier(chysx_vbd* h, int on);
 
 #ifdef __cplusplus
 }

@@ -87,3 +87,36 @@ def test_single_color_of_loose_particles():
         vb[k] = vb[k][:0]
     vb["colors"][:] = 0
     _compare(vb, 6)
+
+
+@pytest.mark.parametrize("api", ["capi", "pybind"])
+def test_failed_barrier_is_reported_and_leaves_the_state(api):
+    vb = _problem(33, 20)
+    g = GpuVbd(vb, colors=vb["colors"], api=api)
+    g.step(3)
+    assert g.s.last_status() == capi.SOLVE_CONVERGED
+    p0, v0 = g.state()
+    if api == "pybind":  # the error flag of a barrier is set through the C ABI only
+        return
+    g.s.debug_fail_barrier(True)
+    g.step(3)
+    assert all(np.array_equal(a, b) for a, b in zip(g.state(), (p0, v0)))
+    g.s.debug_fail_barrier(False)
+    with pytest.raises(RuntimeError, match="barrier"):  # the next step, which does not run
+        g.step(3)
+    g.s.debug_fail_barrier(True)
+    g.step(3)
+    assert g.s.last_status() == capi.SOLVE_KERNEL_ERROR and g.s.last_status() == capi.SOLVE_CONVERGED
+    assert all(np.array_equal(a, b) for a, b in zip(g.state(), (p0, v0)))
+    # and from there as if nothing had been
+    g.s.debug_fail_barrier(False)
+    g.step(3)
+    h = GpuVbd(dict(vb, pos=p0.astype(np.float32), vel=v0.astype(np.float32)), colors=vb["colors"])
+    h.step(3)
+    assert all(np.array_equal(a, b) for a, b in zip(g.state(), h.state()))
+    # a launch per colour has no barrier to fail
+    vb = _problem(277, 276)
+    g = GpuVbd(vb, colors=vb["colors"])
+    g.s.debug_fail_barrier(True)
+    g.step(1)
+    assert g.s.last_status() == capi.SOLVE_CONVERGED and not np.array_equal(g.state()[0], vb["pos"])
