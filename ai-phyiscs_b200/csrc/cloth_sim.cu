@@ -155,6 +155,8 @@ void mlp_gradients(uintptr_t params, uintptr_t features, uintptr_t targets, int 
     if (rows <= 0) throw std::invalid_argument("mlp: rows must be positive");
     if (!params || !features || !workspace) throw std::invalid_argument("mlp: null device pointer");
     if (ws_bytes < mlp_workspace_bytes(rows)) throw std::invalid_argument("mlp: workspace too small");
+    // doubles; 16-byte pieces of the layers' rows in training
+    if (workspace % (targets ? 16 : 8)) throw std::invalid_argument("mlp: workspace not aligned");
     if (targets && !grad) throw std::invalid_argument("mlp: gradients need an output buffer");
     auto stream = reinterpret_cast<cudaStream_t>(stream_u);
     unsigned char* ws = reinterpret_cast<unsigned char*>(workspace);

@@ -566,10 +566,17 @@ mlp_train_tile_kernel(const MlpPacked* __restrict__ net, const float* __restrict
                                                      sizeof(__nv_bfloat16) * kTrainWarps * 16 * kT1);
     {
         static_assert(sizeof(MlpPacked) % 16 == 0, "copied in 16-byte pieces");
-        const uint4* __restrict__ src = reinterpret_cast<const uint4*>(net);
-        uint4* __restrict__ dst = reinterpret_cast<uint4*>(&Wp);
+        if ((reinterpret_cast<uintptr_t>(net) & 15u) == 0) {
+            const uint4* __restrict__ src = reinterpret_cast<const uint4*>(net);
+            uint4* __restrict__ dst = reinterpret_cast<uint4*>(&Wp);
 #pragma unroll 8
-        for (int q = threadIdx.x; q < (int)(sizeof(MlpPacked) / 16); q += kTrainWarps * 32) dst[q] = __ldg(src + q);
+            for (int q = threadIdx.x; q < (int)(sizeof(MlpPacked) / 16); q += kTrainWarps * 32)
+                dst[q] = __ldg(src + q);
+        } else {  // a prediction's workspace, 8-byte aligned
+            const uint2* __restrict__ src = reinterpret_cast<const uint2*>(net);
+            uint2* __restrict__ dst = reinterpret_cast<uint2*>(&Wp);
+            for (int q = threadIdx.x; q < (int)(sizeof(MlpPacked) / 8); q += kTrainWarps * 32) dst[q] = __ldg(src + q);
+        }
     }
     __syncthreads();
     const MlpFwd& W = Wp.f;

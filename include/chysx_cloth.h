@@ -303,7 +303,8 @@ int chysx_cloth_set_feature_output(chysx_cloth* h, uintptr_t features, uintptr_t
 int chysx_cloth_guess_kept(chysx_cloth* h, int* kept);
 int chysx_mlp_num_params(void);
 int chysx_mlp_num_features(void);
-/* Device workspace needed by the training / prediction calls for `rows`. */
+/* Device workspace needed by the training / prediction calls for `rows`
+ * (16-byte aligned for training, 8-byte for prediction). */
 uint64_t chysx_mlp_workspace_bytes(int rows);
 /* Loss (mean squared error of standardised dv) and its gradient in the flat
  * parameter layout, for `rows` feature / target rows (device pointers;

@@ -71,3 +71,23 @@ def test_adam_step(rows):
     assert np.abs(dp.cpu().numpy() - ep).max() < 3e-5 * step + 2.4e-7
     assert np.abs(d1.cpu().numpy() - e1).max() < 1e-6 * np.abs(e1).max()
     assert np.abs(d2.cpu().numpy() - e2).max() < 1e-6 * np.abs(e2).max() + 1e-4 * np.abs(e2 - m2).max()
+
+
+def test_workspace_alignment():
+    # prediction takes a workspace at 8 bytes as at 16; what a kernel could not use is refused before any launch
+    import torch
+
+    rows = 77
+    p, feat, targ, (dp, df, dt), ws = _problem(rows)
+    ws = torch.empty(ws.numel() + 16, dtype=torch.uint8, device="cuda")
+    n = ws.numel() - 16
+    out = [torch.zeros((rows, 3), device="cuda") for _ in range(2)]
+    for k, o in enumerate(out):
+        capi.check(capi.lib().chysx_mlp_predict(dp.data_ptr(), df.data_ptr(), rows, o.data_ptr(),
+                                                ws.data_ptr() + 8 * k, n, 0))
+    assert torch.equal(out[0], out[1]) and out[0].abs().max() > 0
+    grad = torch.zeros_like(dp)
+    assert capi.lib().chysx_mlp_predict(dp.data_ptr(), df.data_ptr(), rows, out[0].data_ptr(), ws.data_ptr() + 4, n,
+                                        0) == capi.ERR_INVALID_ARGUMENT
+    assert capi.lib().chysx_mlp_gradients(dp.data_ptr(), df.data_ptr(), dt.data_ptr(), rows, grad.data_ptr(), None,
+                                          ws.data_ptr() + 8, n, 0) == capi.ERR_INVALID_ARGUMENT
