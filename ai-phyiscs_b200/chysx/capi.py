@@ -15,6 +15,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libchysx_cloth.so")
 
 OK, ERR_INVALID_ARGUMENT, ERR_OUT_OF_RANGE, ERR_RUNTIME, ERR_CUDA = range(5)
+KERNELS = ("resident", "loop", "streamed", "tiled")  # as solver_info numbers them
 SOLVE_CONVERGED, SOLVE_MAX_ITER, SOLVE_NONFINITE, SOLVE_KERNEL_ERROR = range(4)
 WARM = {"zero": 0, "previous": 1, "learned": 2, "previous_scaled": 3}
 
@@ -361,10 +362,10 @@ class Cloth:
 
     def solver_info(self):
         """(kernel, grid, block) of the last graph build; kernel is
-        'resident', 'loop' or 'streamed'."""
+        'resident', 'loop', 'streamed' or 'tiled'."""
         p, g, b = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
         check(self._L.chysx_cloth_solver_info(self.h, ctypes.byref(p), ctypes.byref(g), ctypes.byref(b)))
-        return ("resident", "loop", "streamed")[p.value], g.value, b.value
+        return KERNELS[p.value], g.value, b.value
 
     def autotune(self, dt, repetitions=2, stream=0):
         """Times the applicable solver configurations on the current state
@@ -378,11 +379,10 @@ class Cloth:
         check(self._L.chysx_cloth_autotune_results(self.h, cnt.value, ctypes.byref(cnt),
                                                    cfg.ctypes.data_as(i32p), ms.ctypes.data_as(ctypes.POINTER(ctypes.c_float))))
         keys = ("path", "block", "sync", "kernel", "grid", "threads", "iters", "status")
-        kernels = ("resident", "loop", "streamed")
         out = []
         for k in range(cnt.value):
             d = dict(zip(keys, (int(x) for x in cfg[k])))
-            d["kernel"] = kernels[d["kernel"]]
+            d["kernel"] = KERNELS[d["kernel"]]
             d["solve_ms"] = float(ms[k])
             out.append(d)
         return out

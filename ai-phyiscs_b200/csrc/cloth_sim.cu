@@ -872,10 +872,10 @@ public:
     // is a single instance)
     bool pc_active() const { return pc_kind_ >= 1 && resident_ && graph_path_ == kPathPersistent && sync_mode_ == 0; }
 
-    // kernel actually used by the last graph build: 0 resident, 1 loop,
-    // 2 streamed (a contact operator's lists are, whichever kernel holds the rows)
+    // kernel actually used by the last graph build: 0 resident (with a contact
+    // operator too), 1 loop, 2 streamed, 3 tiled
     void solver_info(int* path, int* grid, int* block) const {
-        const int used = graph_path_ == kPathLoop ? 1 : (resident_ && !co_active_ ? 0 : 2);
+        const int used = graph_path_ == kPathLoop ? 1 : (resident_ ? 0 : (tiled_ ? 3 : 2));
         if (path) *path = used;
         if (grid) *grid = used == 1 ? 0 : plan_.grid;
         if (block) *block = used == 1 ? kVecBlock : solver_block();

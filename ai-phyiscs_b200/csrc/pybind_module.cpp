@@ -418,7 +418,7 @@ PYBIND11_MODULE(_chysx_native, m) {
              [](const PyClothSimulator& s) {
                  int p = 0, g = 0, b = 0;
                  check(chysx_cloth_solver_info(s.h(), &p, &g, &b));
-                 static const char* names[] = {"resident", "loop", "streamed"};
+                 static const char* names[] = {"resident", "loop", "streamed", "tiled"};
                  return py::make_tuple(names[p], g, b);
              })
         .def("set_sync_mode", [](PyClothSimulator& s, int mode) { check(chysx_cloth_set_sync_mode(s.h(), mode)); },
@@ -431,7 +431,7 @@ PYBIND11_MODULE(_chysx_native, m) {
                  std::vector<int32_t> cfg(8 * (size_t)std::max(count, 1));
                  std::vector<float> ms(std::max(count, 1));
                  check(chysx_cloth_autotune_results(s.h(), count, &count, cfg.data(), ms.data()));
-                 static const char* names[] = {"resident", "loop", "streamed"};
+                 static const char* names[] = {"resident", "loop", "streamed", "tiled"};
                  py::list out;
                  for (int k = 0; k < count; ++k) {
                      const int32_t* c = &cfg[8 * (size_t)k];

@@ -77,13 +77,18 @@ def workload(name):
 # ---------------------------------------------------------------------------
 # algorithmic bytes
 # ---------------------------------------------------------------------------
-def pcg_bytes_per_iteration(n, nnz):
+def pcg_bytes_per_iteration(n, nnz, kernel="streamed", coarse=False):
     """Bytes one PCG iteration of the persistent kernel must move in its own
     storage format: phase 1 reads z, p_old (16 B each), the diagonal block
     (24 B), nnz off-diagonal (col 4 B + symmetric block 24 B) and writes p,
     Ap (16 B each); phase 2 reads p, Ap, x, r (16 B each) and M^-1 (24 B) and
     writes x, r, z (16 B each).  Gathered neighbour vectors are counted once
-    (their owner's read)."""
+    (their owner's read).  The tiled kernel keeps the vectors on the SMs and
+    moves the matrix alone: nnz symmetric blocks with 16-bit columns (26 B),
+    the diagonal block and M^-1, and with the coarse level a row's weights
+    twice (16 B)."""
+    if kernel == "tiled":
+        return n * (24 + 24 + (32 if coarse else 0)) + nnz * 26
     return n * (16 + 16 + 24 + 16 + 16) + nnz * 28 + n * (4 * 16 + 24 + 3 * 16)
 
 
@@ -519,7 +524,8 @@ def run_ours(args, rank, world, local_rank):
         inst_of_edge = np.searchsorted(offs, e[:, 0], side="right") - 1
         nnz_b = 2 * np.bincount(inst_of_edge, minlength=len(offs) - 1)
         n_b = np.diff(offs)
-        inst_bytes = pcg_bytes_per_iteration(n_b, nnz_b).astype(np.float64)
+        inst_bytes = pcg_bytes_per_iteration(n_b, nnz_b, g.sim.solver_info()[0],
+                                             g.sim.preconditioner()[3] >= 2).astype(np.float64)
         inst_bytes_ref = reference_format_bytes_per_iteration(n_b, nnz_b).astype(np.float64)
     moved, moved_ref = [], []
     clocks = ClockSampler(local_rank)
@@ -587,7 +593,7 @@ def run_ours(args, rank, world, local_rank):
     nnz = g.sim.num_off_diag_blocks()
     iters = np.array(iters)
     solve_ms = np.array(solve_ms)
-    b_it = pcg_bytes_per_iteration(n, nnz)
+    b_it = pcg_bytes_per_iteration(n, nnz, g.sim.solver_info()[0], g.sim.preconditioner()[3] >= 2)
     b_ref = reference_format_bytes_per_iteration(n, nnz)
     if inst_bytes is None:
         moved, moved_ref = list(iters * b_it), list(iters * b_ref)
@@ -600,7 +606,7 @@ def run_ours(args, rank, world, local_rank):
     in_use = int(g.sim.preconditioner()[3])
     if kern == "resident":
         kern += {0: "", 1: "_chebyshev", 2: "_twolevel", 3: "_twolevel_linear"}[in_use]
-    elif kern == "streamed" and in_use >= 2:
+    elif kern in ("streamed", "tiled") and in_use >= 2:
         kern += "_twolevel"
     traffic_it = read_traffic(kern, args.workload)
     steps_total = args.steps * world
@@ -622,7 +628,7 @@ def run_ours(args, rank, world, local_rank):
 
     # the device's coarse blocks in rows (the CPU legs restate them)
     cinfo = g.sim.debug_coarse()[0] if int(g.sim.preconditioner()[3]) >= 2 else None
-    coarse_rows = int(cinfo["ctas_per_block"]) * int(g.sim.solver_info()[2]) if cinfo else 0
+    coarse_rows = int(np.diff(g.sim.debug_coarse_rows()).max()) if cinfo else 0
     if cinfo and offs is not None:
         coarse_rows = "blocks inside instances: one per CTA segment, at most 12 per instance"
     if cinfo and g.sim.solver_info()[0] == "resident" and coarse_rows != COARSE_ROWS:
@@ -669,6 +675,7 @@ def run_ours(args, rank, world, local_rank):
         "assembly_ms": float(np.mean(asm_ms)),
         "roofline": {"bound": "hbm", "kernel": {"resident": "pcg_resident_kernel",
                                                 "streamed": "pcg_persistent_kernel",
+                                                "tiled": "pcg_tiled_kernel",
                                                 "loop": "pcg_spmv_kernel+pcg_update_kernel"}[g.sim.solver_info()[0]],
                      "achieved": achieved,
                      "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind,

@@ -131,7 +131,7 @@ int chysx_cloth_build_fem_shear(chysx_cloth* h, float stiffness, const float* k_
  * current positions, stiffness k for all (constraint/cloth/
  * bending_constraint.h).  Its Hessian blocks are not symmetric, so a step
  * with bending stores full 3x3 off-diagonal blocks, and no kernel holds its
- * rows in registers (chysx_cloth_solver_info path 1 or 2). */
+ * rows in registers (chysx_cloth_solver_info path 1, 2 or 3). */
 int chysx_cloth_build_bending(chysx_cloth* h, float stiffness, uintptr_t stream);
 int chysx_cloth_num_dihedrals(const chysx_cloth* h, int* out);
 
@@ -172,8 +172,9 @@ int chysx_cloth_get_static_contact(const chysx_cloth* h, float* thickness, float
  * and slips are given.  A contact whose stiffness is not finite and
  * positive is skipped; one with a weighted particle index outside the
  * particle range is dropped and counted (contact_stats).  Needs the
- * single-instance layout; solver_info reports path 2 with one,
- * whichever kernel holds the rows (chysx_cloth_solver_info). */
+ * single-instance layout; a step with a contact operator uses the
+ * register-resident (block-Jacobi, synchronisation mode 0), the streamed or
+ * the graph-loop PCG kernel. */
 typedef struct chysx_contact_op {
     uintptr_t pairs;       /* int32 x 4 per contact, 16-byte aligned */
     uintptr_t weights;     /* float x 8 per contact: w0..w3, nx, ny, nz, depth; 16-byte aligned */
@@ -390,11 +391,11 @@ int chysx_cloth_set_sync_mode(chysx_cloth* h, int mode);
 /* Autotuner (no counterpart in the reference).  Times, on the current state,
  * every solver configuration that applies to the current system: the
  * planner's persistent kernel (register-resident rows or vectors on the SMs
- * when they fit, else streamed), the streamed kernel at 128 / 256 / 512 threads per CTA (4 / 8 /
- * 16 32-row slices per CTA; one thread per row), both synchronisation modes,
- * and the graph-loop path; each `repetitions` times (best kept).  All run the
- * same PCG recurrence.  The caller's positions / velocities and the previous-step guess are
- * restored after every trial, so the simulation does not advance; the
+ * when they fit, else streamed), the streamed kernel at 128 / 256 / 512
+ * threads per CTA (4 / 8 / 16 32-row slices per CTA; one thread per row), both
+ * synchronisation modes, and the graph-loop path; each `repetitions` times
+ * (best kept).  All run the same PCG recurrence.  The caller's positions /
+ * velocities and the previous-step guess are restored after every trial, so the simulation does not advance; the
  * fastest configuration stays selected.  Synchronises `stream`. */
 int chysx_cloth_autotune(chysx_cloth* h, float dt, int repetitions, uintptr_t stream);
 /* The autotuner's table: per candidate 8 ints (path, block, sync, kernel used
@@ -437,8 +438,8 @@ int chysx_cloth_row_of_particles(const chysx_cloth* h, int n, int32_t* rows);
  * register-resident kernel runs with synchronisation mode 0.  On systems too
  * large for that kernel, kinds 1 and 2 give block-Jacobi plus the coarse
  * level on blocks of whole CTAs (about 5120 rows on the streamed kernel, one
- * or more SMs' rows where the vectors stay on the SMs), A_c shifted by 1e-5 diag(A_c) (single instance, synchronisation mode 0); on
- * batches of instances there (zero-guess solves, synchronisation mode 0),
+ * or more SMs' rows where the vectors stay on the SMs), A_c shifted by
+ * 1e-5 diag(A_c) (single instance, synchronisation mode 0); on batches of instances there (zero-guess solves, synchronisation mode 0),
  * block-Jacobi plus coarse blocks inside the instances (an instance's rows in
  * one CTA, runs or parts of such segments, at most 12 per instance; translation and
  * linear fields; A_c block-diagonal by instance, each instance's dense
@@ -449,9 +450,8 @@ int chysx_cloth_row_of_particles(const chysx_cloth* h, int n, int32_t* rows);
 int chysx_cloth_set_preconditioner(chysx_cloth* h, int kind, int degree, float ratio);
 int chysx_cloth_preconditioner(const chysx_cloth* h, int* kind, int* degree, float* ratio, int* in_use);
 /* Kernel used at the last graph build: path 0 register-resident persistent,
- * 1 graph loop, 2 every other persistent kernel (vectors on the SMs, streamed,
- * and the register-resident rows with a contact operator); with its grid and
- * block size. */
+ * 1 graph loop, 2 streamed persistent, 3 tiled persistent (vectors on the SMs,
+ * matrix streamed or in shared memory); with its grid and block size. */
 int chysx_cloth_solver_info(const chysx_cloth* h, int* path, int* grid, int* block);
 
 /* Measurement hooks (no counterpart in the reference): when enabled, the

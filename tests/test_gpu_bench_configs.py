@@ -174,7 +174,7 @@ def test_grid1024_step_matches_fp64_oracle_system():
     g.step()
     it, rr, st = g.stats()
     assert st == capi.SOLVE_CONVERGED and rr <= 1e-6
-    assert g.sim.solver_info()[0] == "streamed" and g.sim.preconditioner()[3] == 3
+    assert g.sim.solver_info()[0] == "tiled" and g.sim.preconditioner()[3] == 3
     diag, rp, col, vals, rhs, dx = g.dump()
     o, im = oracle_sim(sc, tol=0.0, max_iter=0)
     o.set_state(p0, v0, im)

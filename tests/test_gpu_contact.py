@@ -208,7 +208,7 @@ def test_contact_operator_system_and_solve_match_oracle(path, per_contact, mu):
     assert (live, dropped) == (35, 1)
     assert slots == 4 * 34  # every weight of the generated contacts is non-zero
     info = g.sim.solver_info()
-    assert info[0] == ("loop" if path == 1 else "streamed")  # no register-resident kernel with contacts
+    assert info[0] == capi.KERNELS[path]
 
 
 @pytest.mark.parametrize("path", [0, 1])

@@ -59,7 +59,7 @@ def test_matches_streamed(side, grid):
     sc = scenes.config_large(side=side)
     c = Contacts(side * side, 40, side)
     a, b = (_run(sc, c, p, 10, 0.0) for p in (0, 2))
-    assert a.sim.solver_info() == ("streamed", grid, 512)  # the contact lists are streamed
+    assert a.sim.solver_info() == ("resident", grid, 512) and b.sim.solver_info()[0] == "streamed"
     assert np.abs(a.positions() - b.positions()).max() < 5e-7
     a, b = (_run(sc, c, p, 20000, 1e-8) for p in (0, 2))
     assert a.stats()[2] == b.stats()[2] == capi.SOLVE_CONVERGED
@@ -87,3 +87,12 @@ def test_long_lists(side, m):
     a, b = (_run(sc, c, p, 20000, 1e-8) for p in (0, 2))
     assert a.stats()[2] == b.stats()[2] == capi.SOLVE_CONVERGED
     assert np.abs(a.positions() - b.positions()).max() < 1e-5
+
+
+def test_autotune_tells_the_kernels_apart():
+    # 100 x 100: the resident and the streamed kernel both run 20 CTAs of 512 threads
+    sc = scenes.config_large(side=100)
+    g = _run(sc, Contacts(10000, 40, 3), 0, 50, 0.0)
+    table = g.sim.autotune(sc["dt"], 1)
+    kinds = {(t["kernel"], t["threads"], t["grid"]) for t in table if t["sync"] == 0}
+    assert ("resident", 512, 20) in kinds and ("streamed", 512, 20) in kinds

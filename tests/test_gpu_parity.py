@@ -150,7 +150,7 @@ def test_bending_system_and_trajectory_match_oracle(path):
             assert np.abs(vals - np.transpose(vals, (0, 2, 1))).max() > 0  # unsymmetric blocks stored
             assert np.abs(rhs - orhs).max() < 5e-4
     if path == 0:
-        assert g.sim.solver_info()[0] == "streamed"
+        assert g.sim.solver_info()[0] == "tiled"
     assert g.stats()[2] == capi.SOLVE_CONVERGED
     assert np.abs(g.positions() - o.state()[0]).max() < 1e-4
 

@@ -54,7 +54,8 @@ def _rect(w, h, seed=0):
 def test_size_limits(w, h, block):
     sc = _rect(w, h)
     a, b = _run(sc, 0), _run(sc, 2)
-    assert a.sim.solver_info()[2] == block and b.sim.solver_info()[2] == 256
+    assert a.sim.solver_info()[::2] == ("tiled" if block > 256 else "streamed", block)
+    assert b.sim.solver_info()[::2] == ("streamed", 256)
     assert a.stats()[0] == b.stats()[0] == 10
     assert np.abs(a.positions() - b.positions()).max() < 5e-7
 
@@ -65,7 +66,7 @@ def test_size_limits(w, h, block):
 def test_warm_starts(w, h, block, warm, order):
     sc = _rect(w, h)
     a, b = _second_step(sc, warm, order=order, its=20000, tol=1e-6)
-    assert a.sim.solver_info()[2] == block
+    assert a.sim.solver_info()[::2] == ("tiled", block)
     assert a.stats()[2] == capi.SOLVE_CONVERGED and a.stats()[1] <= 1e-6
     assert np.abs(a.positions() - b.positions()).max() < 1e-5
 
@@ -75,7 +76,7 @@ def test_particles_without_elements(w, h):
     # inertia and pins alone, more rows than the register-resident kernel takes: a matrix without entries
     sc = dict(_rect(w, h), k_spring=None, k_stretch=None)
     a, b = _run(sc, 0, its=20, tol=1e-6, steps=2), _run(sc, 2, its=20, tol=1e-6, steps=2)
-    assert a.sim.num_off_diag_blocks() == 0 and a.sim.solver_info()[2] == 512
+    assert a.sim.num_off_diag_blocks() == 0 and a.sim.solver_info()[::2] == ("tiled", 512)
     assert a.stats()[2] == capi.SOLVE_CONVERGED
     assert np.abs(a.positions() - b.positions()).max() < 5e-7
     # two steps of free fall from rest: 3 g dt^2 down
@@ -111,7 +112,7 @@ def test_wide_rows_on_one_cta():
     tris = np.array([[0, 1 + k, 1 + (k + 1) % 60] for k in range(60)], np.int32)
     sc = scenes._finish("fan", pos, tris, 1.0e3, 1.0e4, [1, 31], 1, 10, 0.0)
     a, b = _run(sc, 0), _run(sc, 2)
-    assert a.sim.solver_info()[2] == 512
+    assert a.sim.solver_info()[::2] == ("tiled", 512)
     assert np.abs(a.positions() - b.positions()).max() < 5e-7
 
 
@@ -125,7 +126,7 @@ def test_scattered_particles_keep_the_streamed_kernel():
         sh = scenes._finish("shuffled", pos.astype(np.float64), tris, 1.0e3, 1.0e4, inv[:side], 1, 10, 0.0,
                             det_eps=1.0e-12)
         a, b = _run(sh, 0), _run(sh, 2)
-        assert a.sim.solver_info()[2] == block
+        assert a.sim.solver_info()[::2] == ("tiled" if block > 256 else "streamed", block)
         assert np.abs(a.positions() - b.positions()).max() < 5e-7
 
 
@@ -135,7 +136,7 @@ def test_batches_stop_alone(lo, hi, count, coarse):
     # few large instances, and many small ones (a dozen per CTA)
     sc, offs = scenes.concat(scenes.batch_instances(count=count, seed=3, lo=lo, hi=hi, steps=1, max_iter=20000))
     a, b = (_run(sc, p, its=20000, tol=1e-6, offs=offs, order=1, coarse=coarse, steps=2) for p in (0, 2))
-    assert a.sim.solver_info()[2] == 1024 and a.sim.preconditioner()[3] == (3 if coarse else 0)
+    assert a.sim.solver_info()[::2] == ("tiled", 1024) and a.sim.preconditioner()[3] == (3 if coarse else 0)
     ia, ib = a.sim.instance_stats(), b.sim.instance_stats()
     assert (ia[2] == capi.SOLVE_CONVERGED).all() and (ia[1] <= 1e-6).all()
     assert len(set(ia[0].tolist())) > 1
@@ -147,7 +148,7 @@ def test_batches_stop_alone(lo, hi, count, coarse):
 def test_two_level_converges_to_the_streamed_solution():
     sc = scenes.config_large(side=300, steps=2, max_iter=20000)
     a, b = (_run(sc, p, its=20000, tol=1e-6, order=1, coarse=True) for p in (0, 2))
-    assert a.sim.solver_info()[2] == 1024 and a.sim.preconditioner()[3] == 3
+    assert a.sim.solver_info()[::2] == ("tiled", 1024) and a.sim.preconditioner()[3] == 3
     assert a.stats()[2] == capi.SOLVE_CONVERGED and a.stats()[1] <= 1e-6
     assert a.stats()[0] < 1.5 * b.stats()[0]
     assert np.abs(a.positions() - b.positions()).max() < 1e-5
@@ -160,7 +161,7 @@ def test_bending_systems(w, h):
     sc = _rect(w, h)
     sc["k_bend"], sc["k_shear"] = 5.0e-3, 5.0e3
     a, b = _run(sc, 0), _run(sc, 2)
-    assert a.sim.solver_info()[0] == b.sim.solver_info()[0] == "streamed"
+    assert a.sim.solver_info()[0] == "tiled" and b.sim.solver_info()[0] == "streamed"
     assert a.sim.solver_info()[2] == (1024 if w > 200 else 512)
     assert (a.sim.solver_info()[1] <= 16) == (w * h < 4000)
     assert np.abs(a.positions() - b.positions()).max() < 5e-7
