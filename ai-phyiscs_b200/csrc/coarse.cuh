@@ -172,6 +172,7 @@ __global__ void __launch_bounds__(288) coarse_assemble_kernel(DevTopo t, CoarseA
     for (int qb = 0; qb < nq; ++qb)
         for (int k = 0; k < mn; ++k) acc(qb, k) = 0.0f;
     const int pl = sym_plane(c);
+    const int ow = off_width(t), po = t.nsym ? c : pl;  // planes per off-diagonal block, this component's
     const int self = ca.self_idx[B];
     const int s0 = ca.cb_row0[B] >> 5, s1 = ca.cb_row0[B + 1] >> 5;
     auto weights = [&](int i) {  // (w_i0, w_i1, w_i2, w_i3) = (1, s_1, s_2, s_3)
@@ -202,7 +203,7 @@ __global__ void __launch_bounds__(288) coarse_assemble_kernel(DevTopo t, CoarseA
                 const int e = so + (k0 + k) * 32 + l;
                 const int cj = in ? t.col[e] : i;
                 nb8[k] = in ? ca.ell_nbr[e] : 0;
-                vv[k] = in ? wi * t.val[(size_t)so * 6 + (size_t)(k0 + k) * 192 + pl * 32 + l] : 0.0f;
+                vv[k] = in ? wi * t.val[(size_t)so * ow + (size_t)(k0 + k) * ow * 32 + po * 32 + l] : 0.0f;
                 wv[k] = weights(cj);
             }
             // difference form: entry (i, j) adds w_i A_ij w_j^C to (B, C)
