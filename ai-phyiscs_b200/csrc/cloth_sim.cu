@@ -1890,11 +1890,13 @@ private:
     }
 
     // The tiled kernel's plan: one CTA per SM, every solver vector of its rows
-    // on the SM.  Chosen for every system that is too large for the
-    // register-resident kernel and fits: at most kTileMaxSlices slices per CTA
-    // (tensor memory), own and halo rows of p in shared memory.  A caller's
-    // block or grid request, synchronisation mode 1, general 3x3 blocks
-    // (bending) and the contact operator keep the streamed kernel.
+    // on the SM.  Chosen for every system that the register-resident kernel
+    // does not take and that fits: at most kTileMaxSlices slices per CTA
+    // (tensor memory), own and halo rows of p in shared memory.  General 3x3
+    // blocks (bending) fit it as single block-Jacobi systems only.  A caller's
+    // block or grid request, synchronisation mode 1, the contact operator and
+    // bending in batches or with another preconditioner keep the streamed
+    // kernel.
     bool plan_tiled(int sms) {
         if (solver_path_ != kPathPersistent || pcg_block_req_ != 0 || pcg_grid_req_ != 0 || sync_mode_ != 0 ||
             co_active_)

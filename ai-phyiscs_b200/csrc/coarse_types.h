@@ -30,10 +30,14 @@ constexpr int kCoarseResidentCtas = 2;
 constexpr int kCoarseSplitSlices = 8;
 constexpr int kCoarseMaxSplits = 32;
 // The tiled kernel's coarse blocks.  Single instance: a block per CTA (of
-// g CTAs where they hold fewer than kTileBlockRows rows).  Batches: inside
-// instances, of at least kTileBatchSlices slices, at most kBatchMaxBlocks per
-// instance: a batch of 128 grids of 16 to 128 a side takes 539 iterations and
-// 25.9 ms a step with these, 808 and 37.8 ms with a block per instance and CTA.
+// g CTAs where they hold fewer than kTileBlockRows rows).  A CTA's rows are one
+// patch, so its block needs no exchange of its own; on 1024 x 1024 that is
+// 7,104 rows and 14% more iterations than the streamed kernel's 5,120-row
+// blocks (1,718 against 1,502 at one state), at half the time each.  Batches:
+// inside instances, of at least kTileBatchSlices slices, at most
+// kBatchMaxBlocks per instance: a batch of 128 grids of 16 to 128 a side takes
+// 539 iterations and 25.9 ms a step with these, 808 and 37.8 ms with a block
+// per instance and CTA.  Both numbers rest on these two systems alone.
 constexpr int kTileBlockRows = 1024;
 constexpr int kTileBatchSlices = 9;
 // Relative diagonal shift of the streamed and tiled kernels' coarse matrix: A_c +

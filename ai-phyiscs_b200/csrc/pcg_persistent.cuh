@@ -1579,12 +1579,12 @@ namespace chysx_b200 {
 // CT = 1 adds the contact operator: the particles' p of a row's contact slots
 // are formed from the exchanged (z, p), as a neighbour's is.  A CTA's rows are
 // consecutive in the step's list, so their entries are brought into shared
-// memory once per solve (as many as the dynamic allocation holds, the rest
-// // are read from L2): from the list, each entry was three dependent L2 reads
-// before its gathers, one entry after the other.  Two 160 x 160 sheets with
-// 8,500 contacts: 15.1 us per iteration streamed, 10.9 resident from the list,
-// 8.8 from shared memory (9.4 with the entries dealt out to all threads and
-// two at a time 9.7, for the registers).
+// memory once per solve (as many as the dynamic allocation holds, the rest are
+// read from L2): from the list, each entry was three dependent L2 reads before
+// its gathers, one entry after the other.  Two 160 x 160 sheets with 8,500
+// contacts, us per iteration: 15.1 streamed, 10.9 resident from the list, 8.8
+// from shared memory.  Dealing the entries out to all threads took 9.4, taking
+// two at a time 9.7 (both cost registers).
 // ---------------------------------------------------------------------------
 template <int W, int MAXW, int SYNC = 0, int PC = 0, int CT = 0>
 __global__ void __launch_bounds__(W * 32, 512 / (W * 32))  // 512 threads of rows per SM

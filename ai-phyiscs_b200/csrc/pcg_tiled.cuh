@@ -3,9 +3,9 @@
 //
 // The streamed kernel (pcg_persistent.cuh) re-reads z, p, x, r, A p of every
 // row each iteration and gathers each neighbour's z and old p from L2: 32 B
-// per entry on top of the entry's own 28, so its 96 us iteration at 1024 x
-// 1024 rows is bound by L2 traffic (~0.7 GB), not by the 0.4 GB that must come
-// from HBM.  Here
+// per entry on top of the entry's own 28, so its iteration at 1024 x 1024 rows
+// (96 us, block-Jacobi) is bound by L2 traffic (~0.7 GB), not by the 0.4 GB
+// that must come from HBM.  Here
 //   * p of the CTA's rows and of its halo (the other CTAs' rows that its
 //     entries reach) lies in shared memory, and entries carry 16-bit indices
 //     into it, so a gather is a shared-memory read;
@@ -25,9 +25,10 @@
 // Per iteration a row costs its blocks and 16-bit columns (26 B each), D'
 // and M^-1 (48 B), and 32 B of coarse weights with the coarse level.
 // Measured on B200, streamed against tiled: 801 x 643 rows, 50 iterations,
-// 2.88 against 1.30 ms (53 against 21 us per iteration); 1024 x 1024 with the
-// coarse level 118 against 56 us per iteration; a batch of 128 grids of 16 to
-// 128 a side 105 against 47.
+// 2.88 against 1.30 ms (53 against 21 us per iteration); 1024 x 1024 96
+// against 44 us per iteration, with the coarse level 118 against 56; a batch of
+// 128 grids of 16 to 128 a side 105 against 47.  Their arithmetic per row is
+// the same; only the FP64 sums run in another order.
 //
 // Phases, per-instance logic, preconditioner (block-Jacobi, or with a coarse
 // level: CO = 1 dense, CO = 2 batched) and stopping rules are those of

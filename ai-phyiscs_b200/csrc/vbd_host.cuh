@@ -241,11 +241,12 @@ private:
     // every colour fit the GPU at once (512 threads per SM: 18,944 vertices a
     // colour, e.g. a 275 x 275 grid in four): there a sweep is latency.  16
     // lanes take a regular mesh's 6 triangles and 12 hinges in one round each;
-    // colours that would not fit with 16 take 8 or 4.  Larger meshes keep a
-    // launch per colour: one kernel measured 2.16 against 2.86 ms on 701 x 513
-    // vertices, but steps at such resolutions can tear elements at a pinned
-    // corner (velocities of 1e4 m/s), and then any change of rounding shows in
-    // the result.
+    // colours that would not fit with 16 take 8 or 4.  The kernel also takes
+    // larger colours, several tiles to a warp, and faster (701 x 513 vertices:
+    // 2.16 against 2.86 ms); that those keep a launch per colour is a choice
+    // about rounding: some steps at such resolutions tear elements at a pinned
+    // corner (velocities of 1e4 m/s) and amplify the last bit of the state, so
+    // another order of sums gives another, equally wrong, result there.
     void plan_records() {
         int dev = 0, sms = 148;
         ck(cudaGetDevice(&dev), "cudaGetDevice");

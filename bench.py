@@ -798,7 +798,7 @@ def main():
     ap.add_argument("--workload", default="grid256")
     ap.add_argument("--warm", default="zero", choices=["zero", "previous", "learned", "previous_scaled"])
     ap.add_argument("--path", type=int, default=0,
-                    help="0 persistent PCG (resident when it fits), 1 graph loop, 2 streamed persistent")
+                    help="0 persistent PCG (resident, else tiled, else streamed, as fits), 1 graph loop, 2 streamed persistent")
     ap.add_argument("--block", type=int, default=0)
     ap.add_argument("--grid", type=int, default=0)
     ap.add_argument("--sync", type=int, default=0, help="persistent kernels: 0 grid counter barrier, 1 polled slots")

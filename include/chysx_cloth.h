@@ -435,8 +435,8 @@ int chysx_cloth_row_of_particles(const chysx_cloth* h, int n, int32_t* rows);
  * A_c^-1 is formed densely each step by an FP64 Gauss-Jordan kernel (at
  * most 2048 unknowns).  It applies to single-instance systems of at most
  * 160 CTAs and acts as kind 1 elsewhere.  Kinds 1 and 2 apply where the
- * register-resident kernel runs with synchronisation mode 0.  On systems too
- * large for that kernel, kinds 1 and 2 give block-Jacobi plus the coarse
+ * register-resident kernel runs with synchronisation mode 0.  On systems that
+ * kernel does not take, kind 1 is block-Jacobi, kind 2 that plus the coarse
  * level on blocks of whole CTAs (about 5120 rows on the streamed kernel, one
  * or more SMs' rows where the vectors stay on the SMs), A_c shifted by
  * 1e-5 diag(A_c) (single instance, synchronisation mode 0); on batches of instances there (zero-guess solves, synchronisation mode 0),

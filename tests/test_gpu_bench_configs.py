@@ -6,7 +6,7 @@ configuration (zero guess, rel-res 1e-6):
 * grid256: 256 x 256 plain-method configuration, two-level preconditioner
   (CTA-local Chebyshev of degree 7 on [lambda/60, lambda] plus the coarse
   level of translation and linear fields), spatially compact row order.
-* grid1024: 1024 x 1024 configuration, its second step (streamed kernel,
+* grid1024: 1024 x 1024 configuration, its second step (tiled kernel,
   block-Jacobi plus the coarse level, spatially compact row order).
 * batch: 16 instances of the batched configuration (sides U{16..128},
   seed 1) packed into one system and solved together.
@@ -160,7 +160,7 @@ TOL_GRID1024_RESIDUAL = 1.0e-3
 
 
 def test_grid1024_step_matches_fp64_oracle_system():
-    """The second step of grid1024 in the benchmarked configuration (streamed
+    """The second step of grid1024 in the benchmarked configuration (tiled
     kernel, block-Jacobi plus the coarse level, spatial order): the step's
     system against the FP64 oracle's assembly from the same FP32 state, and
     the returned dx in that FP64 system."""

@@ -125,7 +125,7 @@ def test_shear_system_and_trajectory_match_oracle(path, stretch):
 @pytest.mark.parametrize("path", PATHS)
 def test_bending_system_and_trajectory_match_oracle(path):
     """Discrete bending (k = 5e-3) beside springs and stretch: unsymmetric
-    off-diagonal blocks (stored as full 3x3), so path 0 runs the streamed
+    off-diagonal blocks (stored as full 3x3), so path 0 runs the tiled
     persistent kernel."""
     sc = scenes.config_small(steps=20)
     sc["k_bend"] = 5.0e-3
